@@ -307,6 +307,18 @@ int sg_rbsor_mixed_solve(int64_t H, int64_t W, void* p, int64_t ld_p, const void
                          int64_t workspace_bytes, int64_t* out_iterations, double* out_relres,
                          int64_t* out_refinements, void* stream);
 
+/* All `iterations` sweeps of sg_jacobi_solve (sor = 0) or sg_rbsor_solve (sor = 1) in one
+ * cooperative launch with the iterate held on the chip: the same iterates, bit for bit.
+ * workspace (16-byte aligned, sg_sweeps_workspace_bytes; cleared by the call): the cells that
+ * neighbouring blocks trade. sg_sweeps_workspace_bytes is 0, and the solve returns
+ * SG_ERR_CAPACITY, for grids that do not fit the current device at once. p and div may not
+ * overlap. A block whose neighbour never answers gives up after a bounded wait and writes NaN. */
+int64_t sg_sweeps_workspace_bytes(int dtype, int64_t H, int64_t W);
+int sg_sweeps_solve(int dtype, int sor, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div, int64_t ld_div,
+                    int mask_mode, const uint8_t* face_mask_u, int64_t ld_fmu, const uint8_t* face_mask_v,
+                    int64_t ld_fmv, double alpha, double reciprocal_beta, double omega, int iterations,
+                    void* workspace, int64_t workspace_bytes, void* stream);
+
 /* backends/numba/solvers/gauss_seidel.py:8-48 (lexicographic order), run as an
  * anti-diagonal wavefront in one thread block; intended for small grids. */
 int sg_gauss_seidel_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div,

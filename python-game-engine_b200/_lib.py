@@ -50,6 +50,8 @@ SIGNATURES = {
     "sg_jacobi_solve": [I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, I, P, P],
     "sg_jacobi_solve_noalloc": [I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, I, P],
     "sg_rbsor_solve": [I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, D, I, P],
+    "sg_sweeps_workspace_bytes": [I, I64, I64],
+    "sg_sweeps_solve": [I, I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, D, I, P, I64, P],
     "sg_gauss_seidel_solve": [I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, I, P],
     "sg_rbsor_split_workspace_bytes": [I, I64, I64],
     "sg_rbsor_split_pack": [I, I64, I64, P, I64, I, P, I64, P],
@@ -137,6 +139,7 @@ _RESTYPE = {
     "sg_batch_snapshot_bytes": ctypes.c_int64,
     "sg_field_stats_workspace_bytes": ctypes.c_int64,
     "sg_rbsor_split_workspace_bytes": ctypes.c_int64,
+    "sg_sweeps_workspace_bytes": ctypes.c_int64,
     "sg_rbsor_mixed_workspace_bytes": ctypes.c_int64,
 }
 

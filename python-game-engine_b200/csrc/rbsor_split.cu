@@ -24,6 +24,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "sweeps.cuh"
 
 namespace sg {
 
@@ -362,6 +363,9 @@ struct SplitWs {
   void* d[2];
   double* partials;
   double* result;  // [0] sum of squares of p, [1] of p = 0
+  void* xchg;      // the resident sweeps' trades (zeroed when the first launch uses it)
+  size_t xchg_bytes;
+  uint32_t tag;    // the next trade's tag; 0: not used yet
 };
 
 static int64_t split_pitch(int64_t W) { return ((((W + 1) >> 1) + 31) / 32) * 32; }
@@ -369,7 +373,9 @@ static int64_t split_pitch(int64_t W) { return ((((W + 1) >> 1) + 31) / 32) * 32
 static size_t split_bytes(int64_t elem, int64_t H, int64_t W, SplitWs* ws, void* base) {
   const int64_t ldh = split_pitch(W);
   const size_t plane = (size_t)(((H * ldh * elem) + 255) / 256 * 256);
-  const size_t total = 6 * plane + (size_t)kSumBlocks * 8 + 256;
+  const size_t fixed = 6 * plane + (size_t)kSumBlocks * 8 + 256;
+  const size_t xchg = ((size_t)resident_workspace_bytes(elem, H, W) + 255) / 256 * 256;
+  const size_t total = fixed + xchg;
   if (ws) {
     char* b = (char*)base;
     ws->ldh = ldh;
@@ -382,6 +388,9 @@ static size_t split_bytes(int64_t elem, int64_t H, int64_t W, SplitWs* ws, void*
     }
     ws->partials = (double*)(b + 6 * plane);
     ws->result = (double*)(b + 6 * plane + (size_t)kSumBlocks * 8);
+    ws->xchg = b + fixed;
+    ws->xchg_bytes = xchg;
+    ws->tag = 0;
   }
   return total;
 }
@@ -405,12 +414,14 @@ static int split_bind(int dtype, int64_t H, int64_t W, void* workspace, int64_t 
   return SG_OK;
 }
 
-// Variant -1 (automatic): the shared-memory tiles while the state and divergence planes fit
+// Variant -1 (automatic): the sweeps with the iterate resident on the chip (2) where the grid
+// fits there; else the shared-memory tiles while the state and divergence planes fit
 // well inside L2 (their launches are latency-bound there and the tiles do 4 sweeps per
 // launch), the streaming half sweeps above that (bandwidth-bound; the tiles' redundant halo
 // work then costs more than it saves).
 static int resolve_variant(int variant, int64_t H, int64_t W, int64_t elem) {
   if (variant >= 0) return variant;
+  if (resident_rows(H, W) > 0) return 2;
   return H * W * elem * 2 <= ((int64_t)8 << 20) ? 1 : 0;
 }
 
@@ -425,6 +436,7 @@ static void launch_half(int H, int W, const SplitWs& w, MasksT<MM> m, double alp
                                                              (const T*)w.d[color], w.ldh, m, alpha, rb, omega, color));
 }
 
+constexpr int kResidentSweeps = 1 << 14;  // sweeps of one resident launch (some tens of ms)
 constexpr int kTileHalo = 8;  // halo of the tile kernel: up to 4 sweeps per launch
 
 template <typename T, int MM>
@@ -448,9 +460,24 @@ static int launch_tiles(int H, int W, const SplitWs& w, bool a_to_b, MasksT<MM> 
 // launches per sweep; variant 1: tile launches of up to kTileHalo / 2 sweeps each, an even
 // number of them (a -> b -> a ...), or streaming launches for a single sweep.
 template <typename T, int MM>
-static int split_sweeps(int H, int W, const SplitWs& w, MasksT<MM> m, double alpha, double rb, double omega,
+static int split_sweeps(int H, int W, SplitWs& w, MasksT<MM> m, double alpha, double rb, double omega,
                         int64_t iterations, int variant, cudaStream_t s) {
   if (iterations <= 0) return SG_OK;
+  if (variant == 2) {
+    if (w.tag == 0) {
+      cudaError_t e = cudaMemsetAsync(w.xchg, 0, w.xchg_bytes, s);
+      if (e != cudaSuccess) return fail(SG_ERR_CUDA, "memset: %s", cudaGetErrorString(e));
+      w.tag = 1;
+    }
+    while (iterations > 0) {
+      const int n = (int)std::min<int64_t>(iterations, kResidentSweeps);
+      SG_CHECK(resident_sweeps<T>(1, 1, H, W, (T*)w.a[0], (T*)w.a[1], w.ldh, (const T*)w.d[0], (const T*)w.d[1], w.ldh,
+                                  m.template as<-1>(), alpha, rb, omega, n, w.xchg, w.tag, s));
+      w.tag += (uint32_t)resident_trades(1, n);
+      iterations -= n;
+    }
+    return SG_OK;
+  }
   if (variant == 0 || iterations == 1) {
     for (int64_t it = 0; it < iterations; ++it)
       for (int color = 0; color < 2; ++color) launch_half<T, MM>(H, W, w, m, alpha, rb, omega, color, s);

@@ -1,0 +1,474 @@
+// Fixed-count sweeps with the iterate held on the chip: Jacobi (jacobi.py:8-24) and red-black
+// SOR (red_black_sor_gauss_seidel.py:8-27), all sweeps of a call in one cooperative launch,
+// the cells in registers.
+//
+// Every update evaluates the reference's expression in the reference's order (masked
+// neighbour sum in T, l + r + d + up; the rest in double; one rounding to T), so the iterates
+// are those of the one-launch-per-sweep kernels bit for bit. Compiled with -fmad=false like
+// the other operator units.
+#include <algorithm>
+#include <type_traits>
+
+#include "sweeps.cuh"
+
+namespace sg {
+
+// ------------------------------------------------------------------ resident sweeps
+// A block of 16 warps holds a region of 16 RPT rows x 64 columns in registers: lane l of warp
+// w has columns i0 + 2l, i0 + 2l + 1 of rows j0 + w RPT .. + RPT - 1 (j0, i0 and RPT even, so
+// the colour of a register cell is known at compile time). Horizontal neighbours come by
+// shuffle, vertical ones from the thread's own registers or, at a warp's first and last row,
+// through shared memory with one barrier per half sweep (Jacobi: per sweep). The region
+// overlaps its neighbours' by kHalo cells on each side inside the grid: values grown wrong
+// from its edge move in one cell per half sweep, so after kHalo of them the block's own cells
+// still hold exactly the grid-wide iterates. Then the blocks trade the kHalo-wide frames of
+// their own cells and go on.
+//
+// What bounds it: a call is a chain of `sweeps` dependent sweeps of grids that sit on the
+// chip, so its time is the chain's latency: barrier, shuffle and the float64 part of the
+// update (for float32 fields the conversions, 16 lanes per clock) per half sweep, plus one
+// trade every kHalo of them (about 1.5 us). One launch per kHalo half sweeps pays the load,
+// store and launch of a whole tile at each trade instead. Measured, us a sweep (shared-memory
+// tiles of 8 Jacobi sweeps or 4 split-layout SOR sweeps a launch, one-colour launches before):
+//   Jacobi  128^2 float64 1.21 -> 0.54, 600 x 800 float32 3.9 -> 1.8
+//   SOR     389 x 514 float32 with obstacles 7.2 -> 1.1, 512^2 float64 to 1e-6 3.7 -> 1.3
+// 16 warps of few rows beat 8 warps of twice as many (512^2 float32 SOR 1.00 against 1.33).
+constexpr int kHalo = 8;
+constexpr int kResWarps = 16;
+constexpr int kResThreads = 32 * kResWarps;
+constexpr int kResCols = 64;
+constexpr int kResOwnCols = kResCols - 2 * kHalo;
+
+// Tile t of an axis of n cells covers [t own, t own + span) and owns what lies kHalo or more
+// inside, plus everything up to a grid edge.
+__host__ __device__ inline int res_tiles(int n, int span) {
+  const int own = span - 2 * kHalo;
+  return n <= span ? 1 : (n - 2 * kHalo + own - 1) / own;
+}
+
+template <typename T>
+struct ResArgs {
+  int H, W;
+  T* p;          // natural layout, or colour plane 0
+  T* p1;         // colour plane 1 (split layout)
+  int64_t ldp;   // row stride of p, or of the planes
+  const T* b;    // divergence (rhs), laid out likewise
+  const T* b1;
+  int64_t ldb;
+  Masks m;
+  double alpha, rb, omega;
+  int sweeps;
+  uint64_t* xchg;  // two parities of H x Wx cells, one or two tagged words each; null: one tile
+  int64_t ldx;     // cells per row of xchg (even)
+  uint32_t tag;    // tag of the launch's first trade; the words hold smaller tags or 0 before it
+};
+
+// A trade moves tagged words: 32 bits of a value beside the 32-bit number of the trade, so the
+// data say themselves when they are there and no flag, fence or second round trip is needed
+// (64-bit accesses are single). A reader of trade n has every neighbour's trade n - 1 behind
+// it, and each neighbour sent that after reading trade n - 2, so two parities suffice.
+constexpr int kTradeSpins = 1 << 21;  // polls of about a microsecond each
+
+__device__ __forceinline__ void st_words(uint64_t* p, uint64_t a, uint64_t b) {
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ void ld_words(const uint64_t* p, uint64_t& a, uint64_t& b) {
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+__device__ __forceinline__ uint64_t tagged(uint32_t v, uint32_t tag) { return ((uint64_t)tag << 32) | v; }
+
+// the two cells (columns i, i + 1; i even) of one row, at cell offset o (even) of the buffer
+__device__ __forceinline__ void trade_put(uint64_t* x, int64_t o, const float (&v)[2], uint32_t tag) {
+  st_words(x + o, tagged(__float_as_uint(v[0]), tag), tagged(__float_as_uint(v[1]), tag));
+}
+__device__ __forceinline__ void trade_put(uint64_t* x, int64_t o, const double (&v)[2], uint32_t tag) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q)
+    st_words(x + 2 * (o + q), tagged((uint32_t)__double2loint(v[q]), tag),
+             tagged((uint32_t)__double2hiint(v[q]), tag));
+}
+__device__ __forceinline__ bool trade_get(const uint64_t* x, int64_t o, float (&v)[2], uint32_t tag) {
+  uint64_t a, b;
+  ld_words(x + o, a, b);
+  v[0] = __uint_as_float((uint32_t)a);
+  v[1] = __uint_as_float((uint32_t)b);
+  return (uint32_t)(a >> 32) == tag && (uint32_t)(b >> 32) == tag;
+}
+__device__ __forceinline__ bool trade_get(const uint64_t* x, int64_t o, double (&v)[2], uint32_t tag) {
+  bool ok = true;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    uint64_t a, b;
+    ld_words(x + 2 * (o + q), a, b);
+    v[q] = __hiloint2double((int)(uint32_t)b, (int)(uint32_t)a);
+    ok = ok && (uint32_t)(a >> 32) == tag && (uint32_t)(b >> 32) == tag;
+  }
+  return ok;
+}
+
+template <typename T>
+struct ResEdges {  // first and last row of each warp, double-buffered; SOR uses one column of two
+  T top[2][kResWarps][2][32];
+  T bot[2][kResWarps][2][32];
+};
+
+// v where the bit is set, else c, without a branch around what v took to compute
+__device__ __forceinline__ float pick(uint32_t bit, float v, float c) {
+  float o;
+  asm("{.reg .pred p; setp.ne.u32 p, %1, 0; selp.f32 %0, %2, %3, p;}" : "=f"(o) : "r"(bit), "f"(v), "f"(c));
+  return o;
+}
+__device__ __forceinline__ double pick(uint32_t bit, double v, double c) {
+  double o;
+  asm("{.reg .pred p; setp.ne.u32 p, %1, 0; selp.f64 %0, %2, %3, p;}" : "=d"(o) : "r"(bit), "d"(v), "d"(c));
+  return o;
+}
+
+// One half sweep of colour COL (SOR), or one whole sweep (Jacobi), over the thread's cells,
+// with the trade of the warps' edge rows. CODED: faces by the cells' codes (five bits a cell,
+// four cells a word); otherwise every cell is updated and all its faces are open but those of
+// column 0 (edge0) and of the last column (edge1: the lane's second one).
+// Written stage by stage over the rows, so that the rows' chains overlap, with all that does
+// not need another warp's row ahead of the barrier: the shuffles, the sum's first term and the
+// old value's share. A half sweep reads one colour of its neighbours' rows, so that is all the
+// warps store. (float32 SOR at 128^2: 0.65 us a sweep, 0.73 row by row with whole rows stored.)
+//   res_ahead  stores the edge rows and does what comes ahead of the barrier
+//   res_after  the rest
+template <typename T, bool SOR, int COL, int RPT, bool CODED>
+__device__ __forceinline__ void res_ahead(ResEdges<T>& sh, int buf, int w, int lane, const T (&e)[RPT][2],
+                                          const uint32_t* code, bool edge0, bool edge1, double keep,
+                                          T (&s)[RPT][SOR ? 1 : 2], double (&x)[RPT][SOR ? 1 : 2]) {
+  constexpr int Q = SOR ? 1 : 2;  // updated cells per row
+  if (SOR) {
+    sh.bot[buf][w][0][lane] = e[RPT - 1][COL];  // for the next warp's first row
+    sh.top[buf][w][0][lane] = e[0][1 - COL];    // for the previous warp's last row
+  } else {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      sh.bot[buf][w][q][lane] = e[RPT - 1][q];
+      sh.top[buf][w][q][lane] = e[0][q];
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < RPT; ++r) {
+#pragma unroll
+    for (int n = 0; n < Q; ++n) {
+      const int q = SOR ? (COL + r) & 1 : n;
+      const T far = q == 0 ? __shfl_up_sync(0xffffffffu, e[r][1], 1) : __shfl_down_sync(0xffffffffu, e[r][0], 1);
+      const T c = e[r][q];
+      T l = q == 0 ? far : e[r][0];
+      T rt = q == 0 ? e[r][1] : far;
+      if (CODED) {
+        const uint32_t k = code[r >> 1] >> (10 * (r & 1) + 5 * q);
+        l = pick(k & K_L, l, c);
+        rt = pick(k & K_R, rt, c);
+      } else {
+        if (q == 0) l = edge0 ? c : l;
+        if (q == 1) rt = edge1 ? c : rt;
+      }
+      s[r][n] = l + rt;
+      if (SOR) x[r][n] = keep * (double)c;
+    }
+  }
+}
+
+template <typename T, bool SOR, int COL, int RPT, bool CODED>
+__device__ __forceinline__ void res_after(const ResEdges<T>& sh, int buf, int w, int lane, T (&e)[RPT][2],
+                                          const double (&ab)[RPT][2], const uint32_t* code, double rb, double omega,
+                                          T (&s)[RPT][SOR ? 1 : 2], double (&x)[RPT][SOR ? 1 : 2]) {
+  constexpr int Q = SOR ? 1 : 2;
+  const int wb = w > 0 ? w - 1 : w, wa = w < kResWarps - 1 ? w + 1 : w;
+  T below[Q], above[Q];
+#pragma unroll
+  for (int n = 0; n < Q; ++n) {
+    below[n] = sh.bot[buf][wb][n][lane];
+    above[n] = sh.top[buf][wa][n][lane];
+  }
+#pragma unroll
+  for (int r = 0; r < RPT; ++r) {
+#pragma unroll
+    for (int n = 0; n < Q; ++n) {
+      const int q = SOR ? (COL + r) & 1 : n;
+      T d = r > 0 ? e[r > 0 ? r - 1 : 0][q] : below[n];
+      T u = r < RPT - 1 ? e[r < RPT - 1 ? r + 1 : r][q] : above[n];
+      if (CODED) {
+        const uint32_t k = code[r >> 1] >> (10 * (r & 1) + 5 * q);
+        d = pick(k & K_D, d, e[r][q]);
+        u = pick(k & K_U, u, e[r][q]);
+      }
+      s[r][n] = s[r][n] + d;
+      s[r][n] = s[r][n] + u;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < RPT; ++r) {
+#pragma unroll
+    for (int n = 0; n < Q; ++n) {
+      const int q = SOR ? (COL + r) & 1 : n;
+      const double np_ = ((double)s[r][n] + ab[r][q]) * rb;
+      x[r][n] = SOR ? x[r][n] + omega * np_ : np_;
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < RPT; ++r) {
+#pragma unroll
+    for (int n = 0; n < Q; ++n) {
+      const int q = SOR ? (COL + r) & 1 : n;
+      const T v = (T)x[r][n];
+      e[r][q] = CODED ? pick((code[r >> 1] >> (10 * (r & 1) + 5 * q)) & K_FLUID, v, e[r][q]) : v;
+    }
+  }
+}
+
+template <typename T, bool SOR, bool SPLIT, int RPT>
+__global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid_constant__ ResArgs<T> a) {
+  constexpr int RR = kResWarps * RPT;
+  __shared__ ResEdges<T> sh;
+  __shared__ int s_lost;
+  const int H = a.H, W = a.W;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int r0 = blockIdx.y * (RR - 2 * kHalo), c0 = blockIdx.x * kResOwnCols;
+  const int j = r0 + w * RPT, i = c0 + 2 * lane;
+  // the block's own cells
+  const bool first_y = blockIdx.y == 0, last_y = blockIdx.y == gridDim.y - 1;
+  const bool first_x = blockIdx.x == 0, last_x = blockIdx.x == gridDim.x - 1;
+  const int oy0 = first_y ? 0 : r0 + kHalo, oy1 = last_y ? H : r0 + RR - kHalo;
+  const int ox0 = first_x ? 0 : c0 + kHalo, ox1 = last_x ? W : c0 + kResCols - kHalo;
+  const bool own_col = i >= ox0 && i < ox1;  // both of the lane's columns: the bounds are even or W
+  if (threadIdx.x == 0) s_lost = 0;
+  T e[RPT][2];
+  double ab[RPT][2];
+  uint32_t code[(RPT + 1) / 2];
+#pragma unroll
+  for (int r = 0; r < (RPT + 1) / 2; ++r) code[r] = 0;
+  bool plain = true;  // every cell inside the grid, fluid, with the edges as res_sweep has them
+#pragma unroll
+  for (int r = 0; r < RPT; ++r) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int jj = j + r, ii = i + q;
+      e[r][q] = (T)0;
+      ab[r][q] = 0.0;
+      uint32_t k = 0;
+      if (jj < H && ii < W) {
+        const int col = (jj + ii) & 1;
+        const int64_t o = SPLIT ? (int64_t)jj * a.ldp + (ii >> 1) : (int64_t)jj * a.ldp + ii;
+        const int64_t ob = SPLIT ? (int64_t)jj * a.ldb + (ii >> 1) : (int64_t)jj * a.ldb + ii;
+        e[r][q] = (SPLIT && col ? a.p1 : a.p)[o];
+        ab[r][q] = a.alpha * (double)(SPLIT && col ? a.b1 : a.b)[ob];
+        k = cell_code(a.m, H, W, jj, ii);
+      }
+      const uint32_t want = K_ALL & ~(ii == 0 ? K_L : 0u) & ~(ii == W - 1 ? K_R : 0u);
+      plain = plain && k == want;
+      code[r >> 1] |= k << (10 * (r & 1) + 5 * q);
+    }
+  }
+  // column 2l is never the last one of an all-fluid plain warp unless W is odd: keep those coded
+  plain = __all_sync(0xffffffffu, plain && i + 1 < W);
+  const bool edge0 = i == 0, edge1 = i + 1 == W - 1;
+  const double rb = a.rb, omega = a.omega, keep = 1.0 - a.omega;
+  const int64_t parity = (int64_t)H * a.ldx * (sizeof(T) / 4);  // words of one parity
+
+  const bool many = gridDim.x * gridDim.y > 1;
+  int left = SOR ? 2 * a.sweeps : a.sweeps;
+  int buf = 0;
+  uint32_t tag = a.tag;
+  bool traded = !many, lost = false;
+  while (true) {
+    const int n = left < kHalo ? left : kHalo;  // even for SOR
+    for (int h = 0; h < n; h += 2) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (!SOR && h + c >= n) break;
+        T sum[RPT][SOR ? 1 : 2];
+        double x[RPT][SOR ? 1 : 2];
+        if (plain) {
+          if (c == 0)
+            res_ahead<T, SOR, 0, RPT, false>(sh, buf, w, lane, e, code, edge0, edge1, keep, sum, x);
+          else
+            res_ahead<T, SOR, 1, RPT, false>(sh, buf, w, lane, e, code, edge0, edge1, keep, sum, x);
+        } else {
+          if (c == 0)
+            res_ahead<T, SOR, 0, RPT, true>(sh, buf, w, lane, e, code, edge0, edge1, keep, sum, x);
+          else
+            res_ahead<T, SOR, 1, RPT, true>(sh, buf, w, lane, e, code, edge0, edge1, keep, sum, x);
+        }
+        __syncthreads();
+        if (plain) {
+          if (c == 0)
+            res_after<T, SOR, 0, RPT, false>(sh, buf, w, lane, e, ab, code, rb, omega, sum, x);
+          else
+            res_after<T, SOR, 1, RPT, false>(sh, buf, w, lane, e, ab, code, rb, omega, sum, x);
+        } else {
+          if (c == 0)
+            res_after<T, SOR, 0, RPT, true>(sh, buf, w, lane, e, ab, code, rb, omega, sum, x);
+          else
+            res_after<T, SOR, 1, RPT, true>(sh, buf, w, lane, e, ab, code, rb, omega, sum, x);
+        }
+        buf ^= 1;
+      }
+    }
+    left -= n;
+    // one trade at least: no block may write p before its neighbours have read it
+    if (left <= 0 && traded) break;
+    if (many) {
+      if (!traded) __syncthreads();  // the whole block has read its region of p
+      uint64_t* x = a.xchg + (tag & 1) * parity;
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) {
+        const int jj = j + r;
+        if (!own_col || jj < oy0 || jj >= oy1) continue;
+        const bool frame = (!first_y && jj < oy0 + kHalo) || (!last_y && jj >= oy1 - kHalo) ||
+                           (!first_x && i < ox0 + kHalo) || (!last_x && i >= ox1 - kHalo);
+        if (frame && SG_IN_BOUNDS(jj < H && i + 1 < a.ldx)) trade_put(x, (int64_t)jj * a.ldx + i, e[r], tag);
+      }
+      // the halo: cells of the region inside the grid that other blocks own
+      const bool halo_col = !own_col && i < W;
+      bool wait = false;
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) wait |= j + r < H && i < W && (halo_col || j + r < oy0 || j + r >= oy1);
+      if (wait && !lost) {
+        int spins = 0;
+        bool all;
+        do {
+          all = true;
+#pragma unroll
+          for (int r = 0; r < RPT; ++r) {
+            const int jj = j + r;
+            if (jj < H && (halo_col || jj < oy0 || jj >= oy1)) {
+              if (!trade_get(x, (int64_t)jj * a.ldx + i, e[r], tag)) all = false;
+            }
+          }
+        } while (!all && ++spins < kTradeSpins);
+        if (!all) {
+          s_lost = 1;
+          lost = true;
+        }
+      }
+      // the lanes leave the polls at different times; the next barrier counts whole warps
+      __syncwarp();
+      traded = true;
+      ++tag;
+    }
+    if (left <= 0) break;
+  }
+  __syncthreads();
+  // a wait that gave up (its neighbour never arrived) leaves no usable iterate: say so in p
+  const bool bad = s_lost != 0;
+#pragma unroll
+  for (int r = 0; r < RPT; ++r) {
+    const int jj = j + r;
+    if (!own_col || jj < oy0 || jj >= oy1) continue;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int ii = i + q;
+      if (ii >= W) continue;
+      const int64_t o = SPLIT ? (int64_t)jj * a.ldp + (ii >> 1) : (int64_t)jj * a.ldp + ii;
+      (SPLIT && ((jj + ii) & 1) ? a.p1 : a.p)[o] = bad ? (T)__int_as_float(0x7fc00000) : e[r][q];
+    }
+  }
+}
+
+// ------------------------------------------------------------------ host side
+static int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 0;
+  return n;
+}
+
+// Rows per thread: the fewest whose tiles all fit on the chip at once, one block an SM (the
+// blocks wait for one another). 0: the grid does not fit. One row and one column have no
+// tile form worth the launch (and a single cell no fluid).
+int resident_rows(int64_t H, int64_t W) {
+  if (H < 2 || W < 2 || H > (1 << 15) || W > (1 << 15)) return 0;
+  const int sms = sm_count();
+  for (int rpt = 2; rpt <= 8; rpt *= 2)
+    if ((int64_t)res_tiles((int)H, kResWarps * rpt) * res_tiles((int)W, kResCols) <= sms) return rpt;
+  return 0;
+}
+
+int64_t resident_workspace_bytes(int64_t elem, int64_t H, int64_t W) {
+  const int rpt = resident_rows(H, W);
+  if (rpt == 0) return 0;
+  return 2 * H * ((W + 1) & ~(int64_t)1) * 2 * elem;
+}
+
+template <typename T, bool SOR, bool SPLIT, int RPT>
+static int launch_resident_rpt(ResArgs<T>& a, cudaStream_t s) {
+  dim3 grid((unsigned)res_tiles(a.W, kResCols), (unsigned)res_tiles(a.H, kResWarps * RPT));
+  void* args[] = {&a};
+  cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_sweeps_resident<T, SOR, SPLIT, RPT>, grid,
+                                              dim3(kResThreads), args, 0, s);
+  note_launch();
+  return e == cudaSuccess ? SG_OK : fail(SG_ERR_CUDA, "resident sweeps: %s", cudaGetErrorString(e));
+}
+
+int resident_trades(int sor, int sweeps) {
+  const int n = sor ? 2 * sweeps : sweeps;
+  return std::max(1, (n + kHalo - 1) / kHalo);
+}
+
+template <typename T>
+int resident_sweeps(int sor, int split, int H, int W, T* p, T* p1, int64_t ldp, const T* b, const T* b1, int64_t ldb,
+                    const Masks& m, double alpha, double rb, double omega, int sweeps, void* xchg, uint32_t tag,
+                    cudaStream_t s) {
+  const int rpt = resident_rows(H, W);
+  if (rpt == 0) return fail(SG_ERR_CAPACITY, "%d x %d cells do not fit the resident sweeps", H, W);
+  if (sweeps <= 0) return SG_OK;
+  ResArgs<T> a{H, W, p, p1, ldp, b, b1, ldb, m, alpha, rb, omega, sweeps, (uint64_t*)xchg, (W + 1) & ~1, tag};
+  auto go = [&](auto SOR_, auto SPLIT_) {
+    constexpr bool S = decltype(SOR_)::value, P = decltype(SPLIT_)::value;
+    if (rpt == 2) return launch_resident_rpt<T, S, P, 2>(a, s);
+    if (rpt == 4) return launch_resident_rpt<T, S, P, 4>(a, s);
+    return launch_resident_rpt<T, S, P, 8>(a, s);
+  };
+  if (!sor) return go(std::false_type{}, std::false_type{});
+  return split ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
+}
+template int resident_sweeps<float>(int, int, int, int, float*, float*, int64_t, const float*, const float*, int64_t,
+                                    const Masks&, double, double, double, int, void*, uint32_t, cudaStream_t);
+template int resident_sweeps<double>(int, int, int, int, double*, double*, int64_t, const double*, const double*,
+                                     int64_t, const Masks&, double, double, double, int, void*, uint32_t,
+                                     cudaStream_t);
+
+}  // namespace sg
+
+using namespace sg;
+
+extern "C" {
+
+int64_t sg_sweeps_workspace_bytes(int dtype, int64_t H, int64_t W) {
+  if ((dtype != SG_F32 && dtype != SG_F64) || H < 1 || W < 1) return -1;
+  return resident_workspace_bytes(dtype == SG_F32 ? 4 : 8, H, W);
+}
+
+int sg_sweeps_solve(int dtype, int sor, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div, int64_t ld_div,
+                    int mask_mode, const uint8_t* fmu, int64_t ld_fmu, const uint8_t* fmv, int64_t ld_fmv,
+                    double alpha, double reciprocal_beta, double omega, int iterations, void* workspace,
+                    int64_t workspace_bytes, void* stream) {
+  SG_REQUIRE(H >= 1 && W >= 1 && H <= (1 << 28) && W <= (1 << 28), "bad grid %lld x %lld", (long long)H, (long long)W);
+  SG_REQUIRE(p && div && ld_p >= W && ld_div >= W, "bad fields");
+  SG_REQUIRE(iterations >= 0, "iterations must be >= 0");
+  SG_REQUIRE(mask_mode == SG_MASK_OPEN || mask_mode == SG_MASK_RING || (mask_mode == SG_MASK_PLANES && fmu && fmv),
+             "bad mask mode %d or missing mask planes", mask_mode);
+  const int64_t need = sg_sweeps_workspace_bytes(dtype, H, W);
+  if (need < 0) return fail(SG_ERR_DTYPE, "unsupported dtype code %d", dtype);
+  if (need == 0)
+    return fail(SG_ERR_CAPACITY, "%lld x %lld cells do not fit the resident sweeps", (long long)H, (long long)W);
+  SG_REQUIRE(workspace && !((uintptr_t)workspace & 15) && workspace_bytes >= need,
+             "workspace must be 16-byte aligned and hold %lld bytes", (long long)need);
+  if (iterations == 0) return SG_OK;
+  Masks m = make_masks(mask_mode, H, W, fmu, ld_fmu, fmv, ld_fmv, nullptr, 0);
+  cudaStream_t s = as_stream(stream);
+  cudaError_t e = cudaMemsetAsync(workspace, 0, (size_t)need, s);
+  if (e != cudaSuccess) return fail(SG_ERR_CUDA, "sg_sweeps_solve: %s", cudaGetErrorString(e));
+  SG_DISPATCH(dtype, {
+    return resident_sweeps<T>(sor != 0, 0, (int)H, (int)W, (T*)p, nullptr, ld_p, (const T*)div, nullptr, ld_div, m,
+                              alpha, reciprocal_beta, omega, iterations, workspace, 1, s);
+  });
+}
+
+}  // extern "C"
+
+SG_BOUNDS_ACCESSOR(sweeps)

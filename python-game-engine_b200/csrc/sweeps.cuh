@@ -1,0 +1,40 @@
+// Sweeps with the iterate held on the chip (sweeps.cu), for the solver entry points.
+#pragma once
+
+#include "common.cuh"
+
+namespace sg {
+
+// Per-cell code: the open faces towards a neighbour inside the grid, and whether the cell is
+// fluid. A closed face, and an open one at the grid's edge (whose clamped neighbour is the
+// cell itself), both contribute the cell's own value.
+enum : uint32_t { K_L = 1, K_R = 2, K_D = 4, K_U = 8, K_FLUID = 16, K_ALL = 31 };
+
+__device__ __forceinline__ uint32_t cell_code(const Masks& m, int H, int W, int j, int i) {
+  const bool l = m.u(j, i), r = m.u(j, i + 1), d = m.v(j, i), u = m.v(j + 1, i);
+  uint32_t c = 0;
+  if (l && i > 0) c |= K_L;
+  if (r && i < W - 1) c |= K_R;
+  if (d && j > 0) c |= K_D;
+  if (u && j < H - 1) c |= K_U;
+  if (l || r || d || u) c |= K_FLUID;
+  return c;
+}
+
+// Rows per thread of the resident sweeps on an H x W grid, 0 when it does not fit the chip,
+// and the bytes of the buffer through which their blocks trade.
+int resident_rows(int64_t H, int64_t W);
+int64_t resident_workspace_bytes(int64_t elem, int64_t H, int64_t W);
+
+// Trades that a call of so many sweeps makes (each takes one tag).
+int resident_trades(int sor, int sweeps);
+
+// `sweeps` Jacobi (sor = 0) or red-black SOR sweeps of p in place. split: p, p1 and b, b1 are
+// colour planes. xchg: resident_workspace_bytes bytes, zeroed before the first call that uses
+// it; tag: 1 + the trades of the calls before on the same buffer.
+template <typename T>
+int resident_sweeps(int sor, int split, int H, int W, T* p, T* p1, int64_t ldp, const T* b, const T* b1, int64_t ldb,
+                    const Masks& m, double alpha, double rb, double omega, int sweeps, void* xchg, uint32_t tag,
+                    cudaStream_t s);
+
+}  // namespace sg

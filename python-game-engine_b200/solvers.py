@@ -57,16 +57,38 @@ def materialize_mask(m, H, W, which, device):
 
 
 # ---------------------------------------------------------------- reference methods
+# Sweep counts up to which the launches of the plain kernels cost less than one resident
+# launch with its cleared exchange buffer.
+RESIDENT_MIN_JACOBI = 8
+RESIDENT_MIN_SOR = 2
+
+
+def _resident_sweeps(sor, dtc, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv, alpha, omega, iterations, device):
+    """All sweeps in one launch with the iterate on the chip (``sg_sweeps_solve``: the same
+    iterates); False when the grid does not fit there."""
+    nbytes = L.load().sg_sweeps_workspace_bytes(dtc, H, W)
+    if nbytes <= 0:
+        return False
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    L.call("sg_sweeps_solve", dtc, sor, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv, alpha, calculate_reciprocal_beta(),
+           float(omega), int(iterations), ws.data_ptr(), nbytes, L.stream_ptr())
+    return True
+
+
 def jacobi_pressure_solver(pressure, divergence, face_mask_u, face_mask_v, fluid_density, cell_size, dt,
                            iterations, scratch=None, **_ignored):
     """jacobi.py:27-52: ``iterations`` ping-pong sweeps; the result ends in ``pressure``."""
     H, W = pressure.shape
     dtc = L.dtype_code(pressure)
     mode, pu, lu, pv, lv = _face_pair(face_mask_u, face_mask_v, H, W)
-    if scratch is None:
-        scratch = torch.empty((H, W), dtype=pressure.dtype, device=pressure.device)
     p, ldp = L.field(pressure, "pressure")
     d, ldd = L.field(divergence, "divergence", dtype=pressure.dtype)
+    if scratch is None and iterations > RESIDENT_MIN_JACOBI and _resident_sweeps(
+            0, dtc, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv, calculate_alpha(cell_size, fluid_density, dt), 0.0,
+            iterations, pressure.device):
+        return
+    if scratch is None:
+        scratch = torch.empty((H, W), dtype=pressure.dtype, device=pressure.device)
     L.call("sg_jacobi_solve", dtc, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv,
            calculate_alpha(cell_size, fluid_density, dt), calculate_reciprocal_beta(), int(iterations),
            scratch.data_ptr(), L.stream_ptr())
@@ -81,6 +103,10 @@ def red_black_sor_gauss_seidel_pressure_solver(pressure, divergence, face_mask_u
     mode, pu, lu, pv, lv = _face_pair(face_mask_u, face_mask_v, H, W)
     p, ldp = L.field(pressure, "pressure")
     d, ldd = L.field(divergence, "divergence", dtype=pressure.dtype)
+    if iterations > RESIDENT_MIN_SOR and _resident_sweeps(
+            1, L.dtype_code(pressure), H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv,
+            calculate_alpha(cell_size, fluid_density, dt), omega, iterations, pressure.device):
+        return
     L.call("sg_rbsor_solve", L.dtype_code(pressure), H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv,
            calculate_alpha(cell_size, fluid_density, dt), calculate_reciprocal_beta(), float(omega), int(iterations),
            L.stream_ptr())

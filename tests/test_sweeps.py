@@ -1,0 +1,86 @@
+"""Sweeps with the iterate held on the chip (csrc/sweeps.cu) against the one-launch-per-sweep
+kernels and the CPU oracle, bit for bit: grids at the edges of the blocks' regions (64 columns;
+32, 64 or 128 rows), odd extents, every mask kind, row strides, sweep counts that end between
+two trades of the blocks' frames."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import package
+
+pytestmark = pytest.mark.gpu
+
+if not torch.cuda.is_available():
+    pytest.skip("CUDA device required", allow_module_level=True)
+
+import oracle as O  # noqa: E402
+from cuda_adapter import dev  # noqa: E402
+
+sg = package()
+L = sg._lib
+
+
+def _case(H, W, npdt, kind, seed):
+    rng = np.random.default_rng(seed)
+    solid = np.zeros((H, W), bool)
+    if kind == "planes":
+        solid = O.box_solid(H, W)
+        solid[H // 3:H // 3 + max(H // 6, 1), W // 4:W // 2] = True
+    elif kind == "ring":
+        solid = O.box_solid(H, W)
+    fmu, fmv = O.face_masks_from_solid(solid)
+    return (rng.uniform(-1, 1, (H, W)).astype(npdt), rng.uniform(-1, 1, (H, W)).astype(npdt), fmu, fmv)
+
+
+def _mask_args(kind, fmu, fmv, W):
+    if kind == "planes":
+        t = [torch.from_numpy(x.astype(np.uint8)).cuda() for x in (fmu, fmv)]
+        return t, (L.SG_MASK_PLANES, t[0].data_ptr(), W + 1, t[1].data_ptr(), W)
+    return None, (L.SG_MASK_OPEN if kind == "open" else L.SG_MASK_RING, None, 0, None, 0)
+
+
+@pytest.mark.parametrize("sor", [0, 1])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("shape,kind", [
+    ((2, 2), "open"), ((5, 9), "ring"), ((32, 64), "open"), ((33, 65), "open"), ((17, 130), "planes"),
+    ((49, 112), "planes"), ((50, 113), "open"), ((131, 67), "ring"), ((300, 310), "planes"), ((421, 300), "open"),
+    ((600, 801), "planes"), ((1100, 90), "open")])
+def test_resident_sweeps_equal_plain_kernels(sor, dtype, shape, kind):
+    H, W = shape
+    lib = L.load()
+    s = L.stream_ptr()
+    npdt = np.float32 if dtype == torch.float32 else np.float64
+    p0, div, fmu, fmv = _case(H, W, npdt, kind, H + 3 * W)
+    code = L.dtype_code(torch.empty((), dtype=dtype))
+    keep, mask = _mask_args(kind, fmu, fmv, W)
+    n = int(lib.sg_sweeps_workspace_bytes(code, H, W))
+    assert n > 0
+    ws = torch.full((n,), 1, dtype=torch.uint8, device="cuda")
+    d = torch.zeros((H, W + 3), dtype=dtype, device="cuda")[:, :W]
+    d.copy_(dev(div))
+    for iters in (1, 2, 3, 4, 8, 9, 21):
+        got = torch.zeros((H, W + 5), dtype=dtype, device="cuda")[:, :W]
+        got.copy_(dev(p0))
+        rc = lib.sg_sweeps_solve(code, sor, H, W, got.data_ptr(), W + 5, d.data_ptr(), W + 3, *mask, -0.37, 0.25, 1.9,
+                                 iters, ws.data_ptr(), n, s)
+        assert rc == L.SG_OK, lib.sg_last_error()
+        ref = dev(p0)
+        if sor:
+            rc = lib.sg_rbsor_solve(code, H, W, ref.data_ptr(), W, d.data_ptr(), W + 3, *mask, -0.37, 0.25, 1.9, iters, s)
+        else:
+            scratch = torch.empty_like(ref)
+            rc = lib.sg_jacobi_solve(code, H, W, ref.data_ptr(), W, d.data_ptr(), W + 3, *mask, -0.37, 0.25, iters,
+                                     scratch.data_ptr(), s)
+        assert rc == L.SG_OK, lib.sg_last_error()
+        torch.cuda.synchronize()
+        assert torch.equal(got, ref), f"iterations {iters}: max {float((got - ref).abs().max()):.3e}"
+
+
+def test_resident_sweeps_refuse_what_does_not_fit():
+    lib = L.load()
+    p = torch.zeros((4000, 4000), device="cuda")
+    assert lib.sg_sweeps_workspace_bytes(L.SG_F32, 4000, 4000) == 0
+    rc = lib.sg_sweeps_solve(L.SG_F32, 1, 4000, 4000, p.data_ptr(), 4000, p.data_ptr(), 4000, L.SG_MASK_OPEN, None, 0,
+                             None, 0, -1.0, 0.25, 1.5, 3, p.data_ptr(), p.numel() * 4, L.stream_ptr())
+    assert rc == L.SG_ERR_CAPACITY
+    assert lib.sg_sweeps_workspace_bytes(7, 64, 64) == -1

@@ -319,8 +319,9 @@ int sg_sweeps_solve(int dtype, int sor, int64_t H, int64_t W, void* p, int64_t l
                     int64_t ld_fmv, double alpha, double reciprocal_beta, double omega, int iterations,
                     void* workspace, int64_t workspace_bytes, void* stream);
 
-/* backends/numba/solvers/gauss_seidel.py:8-48 (lexicographic order), run as an
- * anti-diagonal wavefront in one thread block; intended for small grids. */
+/* backends/numba/solvers/gauss_seidel.py:8-48 (lexicographic order), run as anti-diagonal
+ * wavefronts in one thread block with the sweeps following one another two diagonals apart
+ * (shorter side up to 1024 cells; one sweep after the other above). */
 int sg_gauss_seidel_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div,
                           int64_t ld_div, int mask_mode, const uint8_t* fmu, int64_t ld_fmu,
                           const uint8_t* fmv, int64_t ld_fmv, double alpha, double reciprocal_beta,

@@ -10,6 +10,7 @@
 #include <mutex>
 
 #include "cell_ops.cuh"
+#include "sweeps.cuh"
 
 namespace sg {
 
@@ -402,7 +403,8 @@ __global__ void k_rbsor_half(int H, int W, T* __restrict__ p, int64_t ldp, const
   p[(int64_t)j * ldp + i] = (T)((1.0 - omega) * (double)c + omega * np_);
 }
 
-// gauss_seidel.py:8-26 in lexicographic order, as anti-diagonal wavefronts of one block:
+// gauss_seidel.py:8-26 in lexicographic order, one sweep after the other, as anti-diagonal
+// wavefronts of one block (grids whose shorter side exceeds k_gauss_seidel_wave's 1024):
 // cell (j, i) reads its left/down neighbours from wavefront i+j-1 (already updated)
 // and its right/up neighbours from wavefront i+j+1 (not yet updated).
 template <typename T>
@@ -915,6 +917,10 @@ int sg_gauss_seidel_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p
   if (iterations == 0) return SG_OK;
   Masks m = make_masks(mask_mode, H, W, fmu, ld_fmu, fmv, ld_fmv, nullptr, 0);
   SG_DISPATCH(dtype, {
+    bool ran = false;
+    SG_CHECK(gauss_seidel_wave<T>((int)H, (int)W, (T*)p, ld_p, (const T*)div, ld_div, m, alpha, reciprocal_beta,
+                                  iterations, &ran, as_stream(stream)));
+    if (ran) return SG_OK;
     SG_LAUNCH(k_gauss_seidel<T><<<1, 1024, 0, as_stream(stream)>>>((int)H, (int)W, (T*)p, ld_p, (const T*)div, ld_div, m, alpha,
                                                          reciprocal_beta, iterations));
   });

@@ -37,4 +37,9 @@ int resident_sweeps(int sor, int split, int H, int W, T* p, T* p1, int64_t ldp, 
                     const Masks& m, double alpha, double rb, double omega, int sweeps, void* xchg, uint32_t tag,
                     cudaStream_t s);
 
+// Lexicographic Gauss-Seidel sweeps; *ran is false when the grid is too wide for it.
+template <typename T>
+int gauss_seidel_wave(int H, int W, T* p, int64_t ldp, const T* div, int64_t ldd, const Masks& m, double alpha,
+                      double rb, int iterations, bool* ran, cudaStream_t s);
+
 }  // namespace sg

@@ -1,7 +1,8 @@
 """Sweeps with the iterate held on the chip (csrc/sweeps.cu) against the one-launch-per-sweep
 kernels and the CPU oracle, bit for bit: grids at the edges of the blocks' regions (64 columns;
 32, 64 or 128 rows), odd extents, every mask kind, row strides, sweep counts that end between
-two trades of the blocks' frames."""
+two trades of the blocks' frames, and the pipelined Gauss-Seidel wavefront in one and in
+several passes."""
 import numpy as np
 import pytest
 import torch
@@ -84,3 +85,18 @@ def test_resident_sweeps_refuse_what_does_not_fit():
                              None, 0, -1.0, 0.25, 1.5, 3, p.data_ptr(), p.numel() * 4, L.stream_ptr())
     assert rc == L.SG_ERR_CAPACITY
     assert lib.sg_sweeps_workspace_bytes(7, 64, 64) == -1
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("shape,kind,iters", [((1, 7), "open", 3), ((2, 2), "open", 4), ((97, 161), "planes", 40),
+                                              ((161, 97), "ring", 5), ((33, 32), "open", 75), ((180, 180), "open", 41),
+                                              ((700, 260), "planes", 30), ((20, 1100), "planes", 2)])
+def test_gauss_seidel_wave_equals_oracle(dtype, shape, kind, iters):
+    H, W = shape
+    p0, div, fmu, fmv = _case(H, W, dtype, kind, 7 * H + W)
+    exp = p0.copy()
+    O.gauss_seidel_pressure_solver(exp, div, fmu, fmv, 1.0, 1.0 / W, 0.5 / W, iterations=iters)
+    got = dev(p0)
+    mu, mv = (sg.OPEN_BOX,) * 2 if kind == "open" else ((sg.RING_BOX,) * 2 if kind == "ring" else (dev(fmu), dev(fmv)))
+    sg.solvers.gauss_seidel_pressure_solver(got, dev(div), mu, mv, 1.0, 1.0 / W, 0.5 / W, iterations=iters)
+    assert np.array_equal(got.cpu().numpy(), exp)

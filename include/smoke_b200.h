@@ -342,6 +342,28 @@ int sg_mg_prolong(int dtype, int64_t Hc, int64_t Wc, const void* coarse, int64_t
                   int accumulate, void* stream);
 
 /* multigrid/masks.py:3-27 (any solid child makes the coarse cell solid). */
+/* The reference's V-cycles (multigrid/solver.py:94-176) on a hierarchy whose levels halve
+ * exactly: `cycles` cycles of p in place with `sweeps` smoothing sweeps a side and
+ * coarsest_sweeps on the last level, red-black SOR (sor = 1) or Jacobi, in two launches per
+ * level and cycle; every value equals the separate kernels'. Level k: extents, mask planes
+ * (H x (W + 1) and (H + 1) x W bytes, contiguous), their cell codes (sg_mg_codes, sg_mg_codes_bytes
+ * bytes, made once per mask), alpha(2^k h) and the SOR factor. Workspace
+ * 256-byte aligned; sg_mg_vcycles_workspace_bytes is 0, and the call returns SG_ERR_CAPACITY,
+ * for more than 4 SOR or 8 Jacobi sweeps a side or a coarsest level too large for the chip. */
+typedef struct {
+  int64_t H, W;
+  const void* face_mask_u;
+  const void* face_mask_v;
+  const void* code;
+  double alpha, omega;
+} sg_mg_level;
+int64_t sg_mg_codes_bytes(int64_t H, int64_t W);
+int sg_mg_codes(int64_t H, int64_t W, const uint8_t* face_mask_u, const uint8_t* face_mask_v, uint8_t* code,
+                void* stream);
+int64_t sg_mg_vcycles_workspace_bytes(int dtype, int n_levels, const sg_mg_level* levels, int sor, int sweeps);
+int sg_mg_vcycles(int dtype, int n_levels, const sg_mg_level* levels, void* p, int64_t ld_p, const void* div,
+                  int64_t ld_div, double reciprocal_beta, int sor, int cycles, int sweeps, int coarsest_sweeps,
+                  void* workspace, int64_t workspace_bytes, void* stream);
 int sg_mg_coarsen_solid(int64_t H, int64_t W, const uint8_t* solid, int64_t ld_s, uint8_t* coarse,
                         int64_t ld_c, void* stream);
 

@@ -66,6 +66,10 @@ SIGNATURES = {
     "sg_mg_restrict_average": [I, I64, I64, P, I64, I, P, I64, P, I64, I64, I64, D, P],
     "sg_mg_prolong": [I, I64, I64, P, I64, I64, I64, I, P, I64, P, I64, I, P],
     "sg_mg_coarsen_solid": [I64, I64, P, I64, P, I64, P],
+    "sg_mg_codes_bytes": [I64, I64],
+    "sg_mg_codes": [I64, I64, P, P, P, P],
+    "sg_mg_vcycles_workspace_bytes": [I, I, P, I, I],
+    "sg_mg_vcycles": [I, I, P, P, I64, P, I64, D, I, I, I, I, P, I64, P],
     "sg_gmg_plan_create": [ctypes.POINTER(P), I64, I64, I, P, P, P, I, D, I, I, I, I],
     "sg_gmg_plan_destroy": [P],
     "sg_gmg_workspace_bytes": [P],
@@ -140,8 +144,15 @@ _RESTYPE = {
     "sg_field_stats_workspace_bytes": ctypes.c_int64,
     "sg_rbsor_split_workspace_bytes": ctypes.c_int64,
     "sg_sweeps_workspace_bytes": ctypes.c_int64,
+    "sg_mg_codes_bytes": ctypes.c_int64,
+    "sg_mg_vcycles_workspace_bytes": ctypes.c_int64,
     "sg_rbsor_mixed_workspace_bytes": ctypes.c_int64,
 }
+
+class MgLevel(ctypes.Structure):
+    """sg_mg_level (include/smoke_b200.h)."""
+    _fields_ = [("H", I64), ("W", I64), ("face_mask_u", P), ("face_mask_v", P), ("code", P), ("alpha", D), ("omega", D)]
+
 
 _lib = None
 

@@ -28,7 +28,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
           "--expt-relaxed-constexpr", "-I" + INCLUDE, "-I" + CSRC]
 PER_FILE = {"operators.cu": ["-fmad=false"], "batch.cu": ["-fmad=false"], "rbsor_split.cu": ["-fmad=false"],
-            "sweeps.cu": ["-fmad=false"], "gauss_seidel.cu": ["-fmad=false"]}
+            "sweeps.cu": ["-fmad=false"], "gauss_seidel.cu": ["-fmad=false"],
+            "vcycle.cu": ["-fmad=false"]}
 
 
 def _nvcc():

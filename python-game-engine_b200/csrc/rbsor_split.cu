@@ -472,7 +472,7 @@ static int split_sweeps(int H, int W, SplitWs& w, MasksT<MM> m, double alpha, do
     while (iterations > 0) {
       const int n = (int)std::min<int64_t>(iterations, kResidentSweeps);
       SG_CHECK(resident_sweeps<T>(1, 1, H, W, (T*)w.a[0], (T*)w.a[1], w.ldh, (const T*)w.d[0], (const T*)w.d[1], w.ldh,
-                                  m.template as<-1>(), alpha, rb, omega, n, w.xchg, w.tag, s));
+                                  m.template as<-1>(), alpha, rb, omega, n, false, w.xchg, w.tag, s));
       w.tag += (uint32_t)resident_trades(1, n);
       iterations -= n;
     }

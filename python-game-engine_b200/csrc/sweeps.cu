@@ -10,6 +10,7 @@
 #include <type_traits>
 
 #include "sweeps.cuh"
+#include "sweep_region.cuh"
 
 namespace sg {
 
@@ -34,17 +35,7 @@ namespace sg {
 //   SOR     389 x 514 float32 with obstacles 7.2 -> 1.1, 512^2 float64 to 1e-6 3.7 -> 1.3
 // 16 warps of few rows beat 8 warps of twice as many (512^2 float32 SOR 1.00 against 1.33).
 constexpr int kHalo = 8;
-constexpr int kResWarps = 16;
-constexpr int kResThreads = 32 * kResWarps;
-constexpr int kResCols = 64;
 constexpr int kResOwnCols = kResCols - 2 * kHalo;
-
-// Tile t of an axis of n cells covers [t own, t own + span) and owns what lies kHalo or more
-// inside, plus everything up to a grid edge.
-__host__ __device__ inline int res_tiles(int n, int span) {
-  const int own = span - 2 * kHalo;
-  return n <= span ? 1 : (n - 2 * kHalo + own - 1) / own;
-}
 
 template <typename T>
 struct ResArgs {
@@ -58,6 +49,7 @@ struct ResArgs {
   Masks m;
   double alpha, rb, omega;
   int sweeps;
+  int from_zero;   // start from p = 0 without reading p
   uint64_t* xchg;  // two parities of H x Wx cells, one or two tagged words each; null: one tile
   int64_t ldx;     // cells per row of xchg (even)
   uint32_t tag;    // tag of the launch's first trade; the words hold smaller tags or 0 before it
@@ -106,120 +98,6 @@ __device__ __forceinline__ bool trade_get(const uint64_t* x, int64_t o, double (
   return ok;
 }
 
-template <typename T>
-struct ResEdges {  // first and last row of each warp, double-buffered; SOR uses one column of two
-  T top[2][kResWarps][2][32];
-  T bot[2][kResWarps][2][32];
-};
-
-// v where the bit is set, else c, without a branch around what v took to compute
-__device__ __forceinline__ float pick(uint32_t bit, float v, float c) {
-  float o;
-  asm("{.reg .pred p; setp.ne.u32 p, %1, 0; selp.f32 %0, %2, %3, p;}" : "=f"(o) : "r"(bit), "f"(v), "f"(c));
-  return o;
-}
-__device__ __forceinline__ double pick(uint32_t bit, double v, double c) {
-  double o;
-  asm("{.reg .pred p; setp.ne.u32 p, %1, 0; selp.f64 %0, %2, %3, p;}" : "=d"(o) : "r"(bit), "d"(v), "d"(c));
-  return o;
-}
-
-// One half sweep of colour COL (SOR), or one whole sweep (Jacobi), over the thread's cells,
-// with the trade of the warps' edge rows. CODED: faces by the cells' codes (five bits a cell,
-// four cells a word); otherwise every cell is updated and all its faces are open but those of
-// column 0 (edge0) and of the last column (edge1: the lane's second one).
-// Written stage by stage over the rows, so that the rows' chains overlap, with all that does
-// not need another warp's row ahead of the barrier: the shuffles, the sum's first term and the
-// old value's share. A half sweep reads one colour of its neighbours' rows, so that is all the
-// warps store. (float32 SOR at 128^2: 0.65 us a sweep, 0.73 row by row with whole rows stored.)
-//   res_ahead  stores the edge rows and does what comes ahead of the barrier
-//   res_after  the rest
-template <typename T, bool SOR, int COL, int RPT, bool CODED>
-__device__ __forceinline__ void res_ahead(ResEdges<T>& sh, int buf, int w, int lane, const T (&e)[RPT][2],
-                                          const uint32_t* code, bool edge0, bool edge1, double keep,
-                                          T (&s)[RPT][SOR ? 1 : 2], double (&x)[RPT][SOR ? 1 : 2]) {
-  constexpr int Q = SOR ? 1 : 2;  // updated cells per row
-  if (SOR) {
-    sh.bot[buf][w][0][lane] = e[RPT - 1][COL];  // for the next warp's first row
-    sh.top[buf][w][0][lane] = e[0][1 - COL];    // for the previous warp's last row
-  } else {
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      sh.bot[buf][w][q][lane] = e[RPT - 1][q];
-      sh.top[buf][w][q][lane] = e[0][q];
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < RPT; ++r) {
-#pragma unroll
-    for (int n = 0; n < Q; ++n) {
-      const int q = SOR ? (COL + r) & 1 : n;
-      const T far = q == 0 ? __shfl_up_sync(0xffffffffu, e[r][1], 1) : __shfl_down_sync(0xffffffffu, e[r][0], 1);
-      const T c = e[r][q];
-      T l = q == 0 ? far : e[r][0];
-      T rt = q == 0 ? e[r][1] : far;
-      if (CODED) {
-        const uint32_t k = code[r >> 1] >> (10 * (r & 1) + 5 * q);
-        l = pick(k & K_L, l, c);
-        rt = pick(k & K_R, rt, c);
-      } else {
-        if (q == 0) l = edge0 ? c : l;
-        if (q == 1) rt = edge1 ? c : rt;
-      }
-      s[r][n] = l + rt;
-      if (SOR) x[r][n] = keep * (double)c;
-    }
-  }
-}
-
-template <typename T, bool SOR, int COL, int RPT, bool CODED>
-__device__ __forceinline__ void res_after(const ResEdges<T>& sh, int buf, int w, int lane, T (&e)[RPT][2],
-                                          const double (&ab)[RPT][2], const uint32_t* code, double rb, double omega,
-                                          T (&s)[RPT][SOR ? 1 : 2], double (&x)[RPT][SOR ? 1 : 2]) {
-  constexpr int Q = SOR ? 1 : 2;
-  const int wb = w > 0 ? w - 1 : w, wa = w < kResWarps - 1 ? w + 1 : w;
-  T below[Q], above[Q];
-#pragma unroll
-  for (int n = 0; n < Q; ++n) {
-    below[n] = sh.bot[buf][wb][n][lane];
-    above[n] = sh.top[buf][wa][n][lane];
-  }
-#pragma unroll
-  for (int r = 0; r < RPT; ++r) {
-#pragma unroll
-    for (int n = 0; n < Q; ++n) {
-      const int q = SOR ? (COL + r) & 1 : n;
-      T d = r > 0 ? e[r > 0 ? r - 1 : 0][q] : below[n];
-      T u = r < RPT - 1 ? e[r < RPT - 1 ? r + 1 : r][q] : above[n];
-      if (CODED) {
-        const uint32_t k = code[r >> 1] >> (10 * (r & 1) + 5 * q);
-        d = pick(k & K_D, d, e[r][q]);
-        u = pick(k & K_U, u, e[r][q]);
-      }
-      s[r][n] = s[r][n] + d;
-      s[r][n] = s[r][n] + u;
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < RPT; ++r) {
-#pragma unroll
-    for (int n = 0; n < Q; ++n) {
-      const int q = SOR ? (COL + r) & 1 : n;
-      const double np_ = ((double)s[r][n] + ab[r][q]) * rb;
-      x[r][n] = SOR ? x[r][n] + omega * np_ : np_;
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < RPT; ++r) {
-#pragma unroll
-    for (int n = 0; n < Q; ++n) {
-      const int q = SOR ? (COL + r) & 1 : n;
-      const T v = (T)x[r][n];
-      e[r][q] = CODED ? pick((code[r >> 1] >> (10 * (r & 1) + 5 * q)) & K_FLUID, v, e[r][q]) : v;
-    }
-  }
-}
-
 template <typename T, bool SOR, bool SPLIT, int RPT>
 __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid_constant__ ResArgs<T> a) {
   constexpr int RR = kResWarps * RPT;
@@ -241,7 +119,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
   uint32_t code[(RPT + 1) / 2];
 #pragma unroll
   for (int r = 0; r < (RPT + 1) / 2; ++r) code[r] = 0;
-  bool plain = true;  // every cell inside the grid, fluid, with the edges as res_sweep has them
+  bool plain = true;
 #pragma unroll
   for (int r = 0; r < RPT; ++r) {
 #pragma unroll
@@ -254,16 +132,14 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
         const int col = (jj + ii) & 1;
         const int64_t o = SPLIT ? (int64_t)jj * a.ldp + (ii >> 1) : (int64_t)jj * a.ldp + ii;
         const int64_t ob = SPLIT ? (int64_t)jj * a.ldb + (ii >> 1) : (int64_t)jj * a.ldb + ii;
-        e[r][q] = (SPLIT && col ? a.p1 : a.p)[o];
+        if (!a.from_zero) e[r][q] = (SPLIT && col ? a.p1 : a.p)[o];
         ab[r][q] = a.alpha * (double)(SPLIT && col ? a.b1 : a.b)[ob];
         k = cell_code(a.m, H, W, jj, ii);
       }
-      const uint32_t want = K_ALL & ~(ii == 0 ? K_L : 0u) & ~(ii == W - 1 ? K_R : 0u);
-      plain = plain && k == want;
+      plain = plain && res_is_plain(k, ii, W);
       code[r >> 1] |= k << (10 * (r & 1) + 5 * q);
     }
   }
-  // column 2l is never the last one of an all-fluid plain warp unless W is odd: keep those coded
   plain = __all_sync(0xffffffffu, plain && i + 1 < W);
   const bool edge0 = i == 0, edge1 = i + 1 == W - 1;
   const double rb = a.rb, omega = a.omega, keep = 1.0 - a.omega;
@@ -276,38 +152,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
   bool traded = !many, lost = false;
   while (true) {
     const int n = left < kHalo ? left : kHalo;  // even for SOR
-    for (int h = 0; h < n; h += 2) {
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        if (!SOR && h + c >= n) break;
-        T sum[RPT][SOR ? 1 : 2];
-        double x[RPT][SOR ? 1 : 2];
-        if (plain) {
-          if (c == 0)
-            res_ahead<T, SOR, 0, RPT, false>(sh, buf, w, lane, e, code, edge0, edge1, keep, sum, x);
-          else
-            res_ahead<T, SOR, 1, RPT, false>(sh, buf, w, lane, e, code, edge0, edge1, keep, sum, x);
-        } else {
-          if (c == 0)
-            res_ahead<T, SOR, 0, RPT, true>(sh, buf, w, lane, e, code, edge0, edge1, keep, sum, x);
-          else
-            res_ahead<T, SOR, 1, RPT, true>(sh, buf, w, lane, e, code, edge0, edge1, keep, sum, x);
-        }
-        __syncthreads();
-        if (plain) {
-          if (c == 0)
-            res_after<T, SOR, 0, RPT, false>(sh, buf, w, lane, e, ab, code, rb, omega, sum, x);
-          else
-            res_after<T, SOR, 1, RPT, false>(sh, buf, w, lane, e, ab, code, rb, omega, sum, x);
-        } else {
-          if (c == 0)
-            res_after<T, SOR, 0, RPT, true>(sh, buf, w, lane, e, ab, code, rb, omega, sum, x);
-          else
-            res_after<T, SOR, 1, RPT, true>(sh, buf, w, lane, e, ab, code, rb, omega, sum, x);
-        }
-        buf ^= 1;
-      }
-    }
+    res_sweeps<T, SOR, RPT>(sh, buf, w, lane, e, ab, code, plain, edge0, edge1, rb, omega, keep, n);
     left -= n;
     // one trade at least: no block may write p before its neighbours have read it
     if (left <= 0 && traded) break;
@@ -384,7 +229,7 @@ int resident_rows(int64_t H, int64_t W) {
   if (H < 2 || W < 2 || H > (1 << 15) || W > (1 << 15)) return 0;
   const int sms = sm_count();
   for (int rpt = 2; rpt <= 8; rpt *= 2)
-    if ((int64_t)res_tiles((int)H, kResWarps * rpt) * res_tiles((int)W, kResCols) <= sms) return rpt;
+    if ((int64_t)res_tiles((int)H, kResWarps * rpt, kHalo) * res_tiles((int)W, kResCols, kHalo) <= sms) return rpt;
   return 0;
 }
 
@@ -396,7 +241,7 @@ int64_t resident_workspace_bytes(int64_t elem, int64_t H, int64_t W) {
 
 template <typename T, bool SOR, bool SPLIT, int RPT>
 static int launch_resident_rpt(ResArgs<T>& a, cudaStream_t s) {
-  dim3 grid((unsigned)res_tiles(a.W, kResCols), (unsigned)res_tiles(a.H, kResWarps * RPT));
+  dim3 grid((unsigned)res_tiles(a.W, kResCols, kHalo), (unsigned)res_tiles(a.H, kResWarps * RPT, kHalo));
   void* args[] = {&a};
   cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_sweeps_resident<T, SOR, SPLIT, RPT>, grid,
                                               dim3(kResThreads), args, 0, s);
@@ -411,12 +256,12 @@ int resident_trades(int sor, int sweeps) {
 
 template <typename T>
 int resident_sweeps(int sor, int split, int H, int W, T* p, T* p1, int64_t ldp, const T* b, const T* b1, int64_t ldb,
-                    const Masks& m, double alpha, double rb, double omega, int sweeps, void* xchg, uint32_t tag,
-                    cudaStream_t s) {
+                    const Masks& m, double alpha, double rb, double omega, int sweeps, bool from_zero, void* xchg,
+                    uint32_t tag, cudaStream_t s) {
   const int rpt = resident_rows(H, W);
   if (rpt == 0) return fail(SG_ERR_CAPACITY, "%d x %d cells do not fit the resident sweeps", H, W);
   if (sweeps <= 0) return SG_OK;
-  ResArgs<T> a{H, W, p, p1, ldp, b, b1, ldb, m, alpha, rb, omega, sweeps, (uint64_t*)xchg, (W + 1) & ~1, tag};
+  ResArgs<T> a{H, W, p, p1, ldp, b, b1, ldb, m, alpha, rb, omega, sweeps, from_zero, (uint64_t*)xchg, (W + 1) & ~1, tag};
   auto go = [&](auto SOR_, auto SPLIT_) {
     constexpr bool S = decltype(SOR_)::value, P = decltype(SPLIT_)::value;
     if (rpt == 2) return launch_resident_rpt<T, S, P, 2>(a, s);
@@ -427,9 +272,9 @@ int resident_sweeps(int sor, int split, int H, int W, T* p, T* p1, int64_t ldp, 
   return split ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
 }
 template int resident_sweeps<float>(int, int, int, int, float*, float*, int64_t, const float*, const float*, int64_t,
-                                    const Masks&, double, double, double, int, void*, uint32_t, cudaStream_t);
+                                    const Masks&, double, double, double, int, bool, void*, uint32_t, cudaStream_t);
 template int resident_sweeps<double>(int, int, int, int, double*, double*, int64_t, const double*, const double*,
-                                     int64_t, const Masks&, double, double, double, int, void*, uint32_t,
+                                     int64_t, const Masks&, double, double, double, int, bool, void*, uint32_t,
                                      cudaStream_t);
 
 }  // namespace sg
@@ -465,7 +310,7 @@ int sg_sweeps_solve(int dtype, int sor, int64_t H, int64_t W, void* p, int64_t l
   if (e != cudaSuccess) return fail(SG_ERR_CUDA, "sg_sweeps_solve: %s", cudaGetErrorString(e));
   SG_DISPATCH(dtype, {
     return resident_sweeps<T>(sor != 0, 0, (int)H, (int)W, (T*)p, nullptr, ld_p, (const T*)div, nullptr, ld_div, m,
-                              alpha, reciprocal_beta, omega, iterations, workspace, 1, s);
+                              alpha, reciprocal_beta, omega, iterations, false, workspace, 1, s);
   });
 }
 

@@ -31,11 +31,11 @@ int resident_trades(int sor, int sweeps);
 
 // `sweeps` Jacobi (sor = 0) or red-black SOR sweeps of p in place. split: p, p1 and b, b1 are
 // colour planes. xchg: resident_workspace_bytes bytes, zeroed before the first call that uses
-// it; tag: 1 + the trades of the calls before on the same buffer.
+// it; tag: 1 + the trades of the calls before on the same buffer. from_zero: p is 0 and not read.
 template <typename T>
 int resident_sweeps(int sor, int split, int H, int W, T* p, T* p1, int64_t ldp, const T* b, const T* b1, int64_t ldb,
-                    const Masks& m, double alpha, double rb, double omega, int sweeps, void* xchg, uint32_t tag,
-                    cudaStream_t s);
+                    const Masks& m, double alpha, double rb, double omega, int sweeps, bool from_zero, void* xchg,
+                    uint32_t tag, cudaStream_t s);
 
 // Lexicographic Gauss-Seidel sweeps; *ran is false when the grid is too wide for it.
 template <typename T>

@@ -139,6 +139,7 @@ class MultigridSolver:
         self._key = None
         self.levels = []
         self.buffers = []
+        self._workspace = None
 
     def _ensure(self, H, W, fmu, fmv, num_levels, dtype, device, rebuild):
         kind = fmu.name if isinstance(fmu, AnalyticMask) else "planes"
@@ -160,6 +161,11 @@ class MultigridSolver:
             cu, cv, cf = build_masks(sc.bool())
             levels.append(dict(is_fluid=cf, fmu=cu, fmv=cv, solid=sc.bool()))
             solid = sc.bool()
+        for lv in levels:
+            h, w = lv["is_fluid"].shape
+            lv["code"] = torch.empty(L.load().sg_mg_codes_bytes(h, w), dtype=torch.uint8, device=device)
+            L.call("sg_mg_codes", h, w, lv["fmu"].data_ptr(), lv["fmv"].data_ptr(), lv["code"].data_ptr(),
+                   L.stream_ptr())
         self.levels = levels
         self.buffers = [{k: torch.zeros(lv["is_fluid"].shape, dtype=dtype, device=device)
                          for k in ("pressure", "residual", "rhs")} for lv in levels]
@@ -189,6 +195,40 @@ class MultigridSolver:
         smoother(p, rhs, lv["fmu"], lv["fmv"], rho, h, dt, nu)
         return p
 
+    def _fused(self, smoother, pressure, divergence, rho, h, dt, cycles, nu, nu_c):
+        """The cycles in two launches per level (``sg_mg_vcycles``: the same values); False for
+        what that does not take: another smoother, fields it cannot read in place, more sweeps
+        a side than a tile's halo, a coarsest level too large for the chip."""
+        if smoother is jacobi_pressure_solver:
+            sor = 0
+        elif smoother is red_black_sor_gauss_seidel_pressure_solver:
+            sor = 1
+        else:
+            return False
+        if (divergence.dtype != pressure.dtype or divergence.shape != pressure.shape or pressure.stride(1) != 1
+                or divergence.stride(1) != 1 or divergence.device != pressure.device):
+            return False
+        n = len(self.levels)
+        table = (L.MgLevel * n)()
+        for k, lv in enumerate(self.levels):
+            H, W = lv["is_fluid"].shape
+            e = table[k]
+            e.H, e.W = H, W
+            e.face_mask_u, e.face_mask_v, e.code = (lv[m].data_ptr() for m in ("fmu", "fmv", "code"))
+            e.alpha, e.omega = calculate_alpha(h, rho, dt), calculate_optimal_omega(max(H, W))
+            h *= 2.0
+        code = L.dtype_code(pressure)
+        nbytes = L.load().sg_mg_vcycles_workspace_bytes(code, n, ctypes.addressof(table), sor, int(nu))
+        if nbytes <= 0:
+            return False
+        if self._workspace is None or self._workspace.numel() < nbytes or self._workspace.device != pressure.device:
+            self._workspace = torch.empty(nbytes, dtype=torch.uint8, device=pressure.device)
+        p, ldp = L.field(pressure, "pressure")
+        d, ldd = L.field(divergence, "divergence")
+        L.call("sg_mg_vcycles", code, n, ctypes.addressof(table), p, ldp, d, ldd, calculate_reciprocal_beta(), sor,
+               int(cycles), int(nu), int(nu_c), self._workspace.data_ptr(), nbytes, L.stream_ptr())
+        return True
+
     def __call__(self, pressure, divergence, face_mask_u, face_mask_v, fluid_density, cell_size, dt, v_cycles=2,
                  smoother_type="jacobi", smoother_backend="cuda", num_levels=4, smoother_iterations=2,
                  coarsest_iterations=50, rebuild_masks=False, profiler=None, **_ignored):
@@ -196,6 +236,9 @@ class MultigridSolver:
         self._ensure(H, W, face_mask_u, face_mask_v, num_levels, pressure.dtype, pressure.device, rebuild_masks)
         backend = smoother_backend if smoother_backend == "cuda" else "cuda"
         smoother = get_solver(smoother_type, backend)
+        if self._fused(smoother, pressure, divergence, fluid_density, cell_size, dt, v_cycles, smoother_iterations,
+                       coarsest_iterations):
+            return
         fb = self.buffers[0]
         fb["pressure"].copy_(pressure)
         fb["rhs"].copy_(divergence)

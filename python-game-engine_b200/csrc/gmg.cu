@@ -70,6 +70,12 @@ struct GmgState {
   long long failures;      // solves that ended at the cycle cap or on a non-finite residual
   double history[kHist];
   double bmean;  // mean of alpha div over the fluid cells (when the plan removes it)
+  // the solve's fields: the kernels take them from here, so that one instantiated graph serves
+  // every pressure and divergence the plan is called with
+  void* p;
+  int64_t ldp;
+  const void* div;
+  int64_t ldd;
 };
 
 // ---------------------------------------------------------------- point operations
@@ -233,9 +239,11 @@ inline dim3 grid_wide(int64_t W, int64_t H) {
 }
 
 template <typename T, typename TO>
-__global__ void k_gmg_fine_residual(int H, int W, const T* __restrict__ p, int64_t ldp, const T* __restrict__ bf,
+__global__ void k_gmg_fine_residual(int H, int W, const GmgState* __restrict__ st, const T* __restrict__ bf,
                                     int64_t ldb, LevelMask m, TO* __restrict__ r, int64_t ldr, T* __restrict__ rfull,
                                     double* __restrict__ partial) {
+  const T* p = (const T*)st->p;
+  const int64_t ldp = st->ldp;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int ib = blockIdx.x * kWX + threadIdx.x;
   double sq = 0.0;
@@ -257,13 +265,15 @@ __global__ void k_gmg_fine_residual(int H, int W, const T* __restrict__ p, int64
 
 // bf = alpha * div on fluid cells (alpha from the solve state; b may be null when only the
 // outputs below are needed) plus per-block sums of bf^2.
-// For a zero initial guess (pz non-null) it also writes p = 0 and, bf being the residual,
+// For a zero initial guess it also writes p = 0 and, bf being the residual,
 // the first cycle's rhs b0 (cycle precision) and the carried residual r64 (when kept).
 template <typename TD, typename TB, typename TC>
-__global__ void k_gmg_rhs(int H, int W, const TD* __restrict__ div, int64_t ldd, const GmgState* __restrict__ st,
-                          LevelMask m, TB* __restrict__ b, int64_t ldb, double* __restrict__ partial,
-                          TB* __restrict__ pz, int64_t ldpz, TC* __restrict__ b0, int64_t ld0, TB* __restrict__ r64,
-                          int sub_mean) {
+__global__ void k_gmg_rhs(int H, int W, const GmgState* __restrict__ st, LevelMask m, TB* __restrict__ b, int64_t ldb,
+                          double* __restrict__ partial, int zero_guess, TC* __restrict__ b0, int64_t ld0,
+                          TB* __restrict__ r64, int sub_mean) {
+  const TD* div = (const TD*)st->div;
+  const int64_t ldd = st->ldd, ldpz = st->ldp;
+  TB* pz = zero_guess ? (TB*)st->p : nullptr;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int ib = blockIdx.x * kWX + threadIdx.x;
   const double alpha = st->alpha;
@@ -296,7 +306,9 @@ __global__ void k_gmg_rhs(int H, int W, const TD* __restrict__ div, int64_t ldd,
 
 // p += e (fine precision += cycle precision).
 template <typename TP, typename TE>
-__global__ void k_gmg_correct(int H, int W, TP* __restrict__ p, int64_t ldp, const TE* __restrict__ e, int64_t lde) {
+__global__ void k_gmg_correct(int H, int W, const GmgState* __restrict__ st, const TE* __restrict__ e, int64_t lde) {
+  TP* p = (TP*)st->p;
+  const int64_t ldp = st->ldp;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int ib = blockIdx.x * kWX + threadIdx.x;
   if (j >= H) return;
@@ -323,7 +335,12 @@ __device__ __forceinline__ double sum_partials(const double* __restrict__ partia
   return t;
 }
 
-__global__ void k_gmg_set_params(GmgState* st, double alpha, double tol, int max_cycles) {
+__global__ void k_gmg_set_params(GmgState* st, double alpha, double tol, int max_cycles, void* p, int64_t ldp,
+                                 const void* div, int64_t ldd) {
+  st->p = p;
+  st->ldp = ldp;
+  st->div = div;
+  st->ldd = ldd;
   st->alpha = alpha;
   st->tol = tol;
   st->max_cycles = max_cycles;
@@ -334,8 +351,10 @@ __global__ void k_gmg_set_params(GmgState* st, double alpha, double tol, int max
 
 // Per-block sums of div over the fluid cells (for the mean the plan removes from the rhs).
 template <typename TD>
-__global__ void k_gmg_rhs_sum(int H, int W, const TD* __restrict__ div, int64_t ldd, LevelMask m,
+__global__ void k_gmg_rhs_sum(int H, int W, const GmgState* __restrict__ st, LevelMask m,
                               double* __restrict__ partial) {
+  const TD* div = (const TD*)st->div;
+  const int64_t ldd = st->ldd;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int ib = blockIdx.x * kWX + threadIdx.x;
   double acc = 0.0;
@@ -1345,11 +1364,8 @@ struct sg_gmg_plan {
   // cached solve graph
   cudaStream_t capture_stream = nullptr;
   cudaGraphExec_t exec = nullptr;
-  const void* g_p = nullptr;
-  const void* g_div = nullptr;
-  int64_t g_ldp = 0, g_ldd = 0;
-  int g_div_dtype = -1;
-  int g_zero = 0;
+  int g_form = -1;  // what the graph was built for (solve_form)
+  bool fields_staged = false;  // the pressure rows of the solve being recorded are 16-byte units
   int prologue_nodes = 0, body_nodes = 0;
 };
 
@@ -1680,16 +1696,17 @@ static dim3 post_final_grid(const sg_gmg_plan* p) {
   return dim3((L.W + txo - 1) / txo, (L.H + tyo - 1) / tyo);
 }
 
+// pp: the pressure when the kernel is launched outside a solve, null to take the solve's own;
+// aligned: its rows start on 16-byte boundaries.
 template <typename TC, typename TP, int SW>
-static void launch_post_final(const sg_gmg_plan* p, TP* pp, int64_t ldp, cudaStream_t s) {
+static void launch_post_final(const sg_gmg_plan* p, TP* pp, int64_t ldp, bool aligned, cudaStream_t s) {
   constexpr int RPT = RegShape<TC>::RPT_FINAL, NW = RegShape<TC>::NWARP_FINAL, MB = RegShape<TC>::MINB_FINAL;
   const Level& L = p->levels[0];
   const Level& C = p->levels[1];
   TP* r64 = p->off_r64 ? (TP*)(p->ws + p->off_r64) : nullptr;
   // p and r64 staged in shared memory by bulk copies when every owned row of theirs starts on
   // a 16-byte boundary (the workspace rows always do; the caller's p must)
-  const bool staged = ((uintptr_t)pp % 16) == 0 && ((size_t)ldp * sizeof(TP)) % 16 == 0 &&
-                      ((uintptr_t)p->ws % 16) == 0 && ((size_t)L.ld * sizeof(TP)) % 16 == 0;
+  const bool staged = aligned && ((uintptr_t)p->ws % 16) == 0 && ((size_t)L.ld * sizeof(TP)) % 16 == 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   if (p->post_ev_next + 1 < p->post_ev.size()) {  // timing events, outside stream capture only
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusActive;
@@ -1919,8 +1936,8 @@ static void cycle(const sg_gmg_plan* p, int k, bool zero_init, cudaStream_t s) {
 // Prologue: bf = alpha div, ||bf||, r0 = bf - A p -> cycle rhs, relres0 and the loop condition.
 // zero_guess: p is not read; it starts at 0 (written here), so the first residual is bf.
 template <typename TP, typename TD, typename TC>
-static void prologue(const sg_gmg_plan* p, TP* pp, int64_t ldp, const TD* div, int64_t ldd,
-                     cudaGraphConditionalHandle h, int use_handle, cudaStream_t s, bool zero_guess = false) {
+static void prologue(const sg_gmg_plan* p, cudaGraphConditionalHandle h, int use_handle, cudaStream_t s,
+                     bool zero_guess = false) {
   const Level& L = p->levels[0];
   LevelMask m = level_mask(p, 0);
   double* part = (double*)(p->ws + p->off_partial);
@@ -1929,7 +1946,7 @@ static void prologue(const sg_gmg_plan* p, TP* pp, int64_t ldp, const TD* div, i
   TP* bf = (TP*)(p->ws + p->off_bfine);
   TP* r64 = p->off_r64 ? (TP*)(p->ws + p->off_r64) : nullptr;
   if (p->remove_mean) {
-    SG_LAUNCH(k_gmg_rhs_sum<TD><<<g, block2d(), 0, s>>>(L.H, L.W, div, ldd, m, part));
+    SG_LAUNCH(k_gmg_rhs_sum<TD><<<g, block2d(), 0, s>>>(L.H, L.W, st, m, part));
     SG_LAUNCH(k_gmg_finalize_mean<<<1, 1024, 0, s>>>(part, (int)(g.x * g.y), st, p->inv_fluid));
   }
   // from a zero guess the fused fine level carries the residual from here on (b0 / r64), so
@@ -1937,8 +1954,8 @@ static void prologue(const sg_gmg_plan* p, TP* pp, int64_t ldp, const TD* div, i
   TP* bkeep = (zero_guess && p->fused_ir && p->inner <= 1) ? nullptr : bf;
   // the first cycle of such a solve forms r64 from the divergence itself (FirstCycle), so the
   // prologue does not write it
-  SG_LAUNCH(k_gmg_rhs<TD, TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, div, ldd, st, m, bkeep, p->ld_bfine, part,
-                                                          zero_guess ? pp : nullptr, ldp, ws_ptr<TC>(p, L.off_b), L.ld,
+  SG_LAUNCH(k_gmg_rhs<TD, TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, st, m, bkeep, p->ld_bfine, part,
+                                                          zero_guess ? 1 : 0, ws_ptr<TC>(p, L.off_b), L.ld,
                                                           (zero_guess && p->fc.active) ? nullptr : r64,
                                                           p->remove_mean));
   SG_LAUNCH(k_gmg_finalize_norm<<<1, 1024, 0, s>>>(part, (int)(g.x * g.y), st));
@@ -1946,7 +1963,7 @@ static void prologue(const sg_gmg_plan* p, TP* pp, int64_t ldp, const TD* div, i
     SG_LAUNCH(k_gmg_finalize_rel<<<1, 1024, 0, s>>>(part, (int)(g.x * g.y), st, h, use_handle, 0));
     return;
   }
-  SG_LAUNCH(k_gmg_fine_residual<TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, pp, ldp, bf, p->ld_bfine, m,
+  SG_LAUNCH(k_gmg_fine_residual<TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, st, bf, p->ld_bfine, m,
                                                                    ws_ptr<TC>(p, L.off_b), L.ld,
                                                                    r64, part));
   SG_LAUNCH(k_gmg_finalize_rel<<<1, 1024, 0, s>>>(part, (int)(g.x * g.y), st, h, use_handle, 0));
@@ -1954,8 +1971,7 @@ static void prologue(const sg_gmg_plan* p, TP* pp, int64_t ldp, const TD* div, i
 
 // Body: one cycle, p += e, new residual, relres and the loop condition.
 template <typename TP, typename TC>
-static void body(const sg_gmg_plan* p, TP* pp, int64_t ldp, cudaGraphConditionalHandle h, int use_handle,
-                 cudaStream_t s) {
+static void body(const sg_gmg_plan* p, cudaGraphConditionalHandle h, int use_handle, cudaStream_t s) {
   const Level& L = p->levels[0];
   LevelMask m = level_mask(p, 0);
   double* part = (double*)(p->ws + p->off_partial);
@@ -1972,9 +1988,9 @@ static void body(const sg_gmg_plan* p, TP* pp, int64_t ldp, cudaGraphConditional
     int reps = (p->cycle == 1 && 1 < nl - 1) ? 2 : 1;
     for (int q = 0; q < reps; ++q) cycle<TC>(p, 1, q == 0, s);
     switch (p->post) {
-      case 1: launch_post_final<TC, TP, 1>(p, pp, ldp, s); break;
-      case 2: launch_post_final<TC, TP, 2>(p, pp, ldp, s); break;
-      default: launch_post_final<TC, TP, 3>(p, pp, ldp, s); break;
+      case 1: launch_post_final<TC, TP, 1>(p, nullptr, 0, p->fields_staged, s); break;
+      case 2: launch_post_final<TC, TP, 2>(p, nullptr, 0, p->fields_staged, s); break;
+      default: launch_post_final<TC, TP, 3>(p, nullptr, 0, p->fields_staged, s); break;
     }
     dim3 gf = post_final_grid<TC>(p);
     SG_LAUNCH(k_gmg_finalize_rel<<<1, 1024, 0, s>>>(part, (int)(gf.x * gf.y), st, h, use_handle, 1));
@@ -1983,8 +1999,8 @@ static void body(const sg_gmg_plan* p, TP* pp, int64_t ldp, cudaGraphConditional
   dim3 g = grid_wide(L.W, L.H);
   const int inner = p->inner < 1 ? 1 : p->inner;
   for (int q = 0; q < inner; ++q) cycle<TC>(p, 0, q == 0, s);
-  SG_LAUNCH(k_gmg_correct<TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, pp, ldp, ws_ptr<TC>(p, L.off_e), L.ld));
-  SG_LAUNCH(k_gmg_fine_residual<TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, pp, ldp, (const TP*)(p->ws + p->off_bfine),
+  SG_LAUNCH(k_gmg_correct<TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, st, ws_ptr<TC>(p, L.off_e), L.ld));
+  SG_LAUNCH(k_gmg_fine_residual<TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, st, (const TP*)(p->ws + p->off_bfine),
                                                                    p->ld_bfine, m, ws_ptr<TC>(p, L.off_b), L.ld,
                                                                    (TP*)nullptr, part));
   SG_LAUNCH(k_gmg_finalize_rel<<<1, 1024, 0, s>>>(part, (int)(g.x * g.y), st, h, use_handle, inner));
@@ -1998,9 +2014,24 @@ static unsigned long long counter() { return launch_count(); }
     if (_e != cudaSuccess) return fail(SG_ERR_CUDA, "%s: %s", what, cudaGetErrorString(_e)); \
   } while (0)
 
-// Capture prologue + WHILE(body) into one executable graph for these pointers.
+// What the recorded launches depend on beyond the plan: the divergence's type, the zero guess,
+// and which rows can be staged by bulk copies. Not the fields' addresses, which the kernels
+// take from the solve state: a graph built per address cost 140 us of instantiation on every
+// call whose tensors differed from the last one's (several simulations, fresh outputs).
+template <typename TP, typename TD>
+static int solve_form(const sg_gmg_plan* p, const TP* pp, int64_t ldp, const TD* div, int64_t ldd, bool zero_guess) {
+  const bool p16 = ((uintptr_t)pp % 16) == 0 && ((size_t)ldp * sizeof(TP)) % 16 == 0;
+  // a zero-guess solve on the fused fine level starts from p = 0 and r64 = alpha div: its first
+  // post kernel forms both itself when the divergence rows can be staged (16-byte units)
+  const bool fc = zero_guess && p->fused_ir && p->inner <= 1 && ((uintptr_t)div % 16) == 0 &&
+                  ((size_t)ldd * sizeof(TD)) % 16 == 0;
+  return (sizeof(TD) == 8 ? 1 : 0) | (zero_guess ? 2 : 0) | (p16 ? 4 : 0) | (fc ? 8 : 0);
+}
+
+// Capture prologue + WHILE(body) into one executable graph of the given form.
 template <typename TP, typename TD, typename TC>
-static int build_graph(sg_gmg_plan* p, TP* pp, int64_t ldp, const TD* div, int64_t ldd, bool zero_guess) {
+static int build_graph(sg_gmg_plan* p, int form) {
+  const bool zero_guess = (form & 2) != 0;
   if (p->exec) {
     cudaGraphExecDestroy(p->exec);
     p->exec = nullptr;
@@ -2011,20 +2042,16 @@ static int build_graph(sg_gmg_plan* p, TP* pp, int64_t ldp, const TD* div, int64
   SG_CUDA_TRY(cudaGraphCreate(&g, 0), "cudaGraphCreate");
   cudaGraphConditionalHandle h;
   SG_CUDA_TRY(cudaGraphConditionalHandleCreate(&h, g, 0, 0), "cudaGraphConditionalHandleCreate");
-  // a zero-guess solve on the fused fine level starts from p = 0 and r64 = alpha div: its first
-  // post kernel forms both itself when the divergence rows can be staged (16-byte units)
   struct FcGuard {
     const sg_gmg_plan* p;
     ~FcGuard() { p->fc = FirstCycle{nullptr, 0, 0, 0, 0, 0.0, 0.0}; }
   } fc_guard{p};
-  const bool fc_ok = zero_guess && p->fused_ir && p->inner <= 1 && ((uintptr_t)div % 16) == 0 &&
-                     ((size_t)ldd * sizeof(TD)) % 16 == 0;
-  p->fc = FirstCycle{fc_ok ? (const void*)div : nullptr, ldd, sizeof(TD) == 8 ? 1 : 0, p->remove_mean ? 1 : 0,
-                     fc_ok ? 1 : 0, 0.0, 0.0};
+  p->fc = FirstCycle{nullptr, 0, sizeof(TD) == 8 ? 1 : 0, p->remove_mean ? 1 : 0, (form & 8) ? 1 : 0, 0.0, 0.0};
+  p->fields_staged = (form & 4) != 0;
   SG_CUDA_TRY(cudaStreamBeginCaptureToGraph(cs, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
               "begin capture");
   unsigned long long c0 = counter();
-  prologue<TP, TD, TC>(p, pp, ldp, div, ldd, h, 1, cs, zero_guess);
+  prologue<TP, TD, TC>(p, h, 1, cs, zero_guess);
   unsigned long long c1 = counter();
   cudaStreamCaptureStatus cst;
   cudaGraph_t cg = nullptr;
@@ -2045,7 +2072,7 @@ static int build_graph(sg_gmg_plan* p, TP* pp, int64_t ldp, const TD* div, int64
   SG_CUDA_TRY(cudaStreamEndCapture(cs, &g), "end capture");
   SG_CUDA_TRY(cudaStreamBeginCaptureToGraph(cs, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
               "begin body capture");
-  body<TP, TC>(p, pp, ldp, h, 1, cs);
+  body<TP, TC>(p, h, 1, cs);
   unsigned long long c2 = counter();
   SG_CUDA_TRY(cudaStreamEndCapture(cs, &bodyg), "end body capture");
   cudaError_t e = cudaGraphInstantiate(&p->exec, g, 0);
@@ -2053,25 +2080,19 @@ static int build_graph(sg_gmg_plan* p, TP* pp, int64_t ldp, const TD* div, int64
   if (e != cudaSuccess) return fail(SG_ERR_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e));
   p->prologue_nodes = (int)(c1 - c0);
   p->body_nodes = (int)(c2 - c1);
-  p->g_p = pp;
-  p->g_ldp = ldp;
-  p->g_div = div;
-  p->g_ldd = ldd;
-  p->g_div_dtype = sizeof(TD) == 4 ? SG_F32 : SG_F64;
-  p->g_zero = zero_guess ? 1 : 0;
+  p->g_form = form;
   return SG_OK;
 }
 
 template <typename TP, typename TD, typename TC>
 static int solve_async_impl(sg_gmg_plan* p, TP* pp, int64_t ldp, const TD* div, int64_t ldd, double alpha, double tol,
                             int max_cycles, cudaStream_t s, bool zero_guess) {
-  int dd = sizeof(TD) == 4 ? SG_F32 : SG_F64;
-  if (!p->exec || p->g_p != pp || p->g_ldp != ldp || p->g_div != div || p->g_ldd != ldd || p->g_div_dtype != dd ||
-      p->g_zero != (zero_guess ? 1 : 0)) {
-    int rc = build_graph<TP, TD, TC>(p, pp, ldp, div, ldd, zero_guess);
+  const int form = solve_form<TP, TD>(p, pp, ldp, div, ldd, zero_guess);
+  if (!p->exec || p->g_form != form) {
+    int rc = build_graph<TP, TD, TC>(p, form);
     if (rc != SG_OK) return rc;
   }
-  SG_LAUNCH(k_gmg_set_params<<<1, 1, 0, s>>>(state_ptr(p), alpha, tol, max_cycles));
+  SG_LAUNCH(k_gmg_set_params<<<1, 1, 0, s>>>(state_ptr(p), alpha, tol, max_cycles, pp, ldp, div, ldd));
   SG_CUDA_TRY(cudaGraphLaunch(p->exec, s), "cudaGraphLaunch");
   return check_launch("sg_gmg_solve_async");
 }
@@ -2080,10 +2101,11 @@ static int solve_async_impl(sg_gmg_plan* p, TP* pp, int64_t ldp, const TD* div, 
 template <typename TP, typename TD, typename TC>
 static int cycles_eager_impl(sg_gmg_plan* p, TP* pp, int64_t ldp, const TD* div, int64_t ldd, double alpha, int n,
                              double* relres_dev, cudaStream_t s) {
-  SG_LAUNCH(k_gmg_set_params<<<1, 1, 0, s>>>(state_ptr(p), alpha, -1.0, n));
+  SG_LAUNCH(k_gmg_set_params<<<1, 1, 0, s>>>(state_ptr(p), alpha, -1.0, n, pp, ldp, div, ldd));
+  p->fields_staged = (solve_form<TP, TD>(p, pp, ldp, div, ldd, false) & 4) != 0;
   cudaGraphConditionalHandle none = 0;
-  prologue<TP, TD, TC>(p, pp, ldp, div, ldd, none, 0, s);
-  for (int c = 0; c < n; ++c) body<TP, TC>(p, pp, ldp, none, 0, s);
+  prologue<TP, TD, TC>(p, none, 0, s);
+  for (int c = 0; c < n; ++c) body<TP, TC>(p, none, 0, s);
   int m = std::min(n + 1, kHist);
   SG_CUDA_TRY(cudaMemcpyAsync(relres_dev, state_ptr(p)->history, sizeof(double) * m, cudaMemcpyDeviceToDevice, s),
               "history copy");
@@ -2605,10 +2627,11 @@ int sg_gmg_fine_kernel_async(sg_gmg_plan* plan, int which, void* p, int64_t ld_p
   auto post = [&](auto tc, auto tp) {
     using TC = decltype(tc);
     using TP = decltype(tp);
+    const bool aligned = ((uintptr_t)p % 16) == 0 && ((size_t)ld_p * sizeof(TP)) % 16 == 0;
     switch (plan->post) {
-      case 1: launch_post_final<TC, TP, 1>(plan, (TP*)p, ld_p, s); break;
-      case 2: launch_post_final<TC, TP, 2>(plan, (TP*)p, ld_p, s); break;
-      default: launch_post_final<TC, TP, 3>(plan, (TP*)p, ld_p, s); break;
+      case 1: launch_post_final<TC, TP, 1>(plan, (TP*)p, ld_p, aligned, s); break;
+      case 2: launch_post_final<TC, TP, 2>(plan, (TP*)p, ld_p, aligned, s); break;
+      default: launch_post_final<TC, TP, 3>(plan, (TP*)p, ld_p, aligned, s); break;
     }
   };
   if (plan->precision == SG_GMG_FP64) {

@@ -26,8 +26,8 @@ constexpr int kRW = 64;  // tile columns: 32 lanes x 2
 // on entry (not read), and when div is set the carried float64 residual r64 starts as
 // alpha div (- the fluid mean with sub_mean), formed here from the divergence instead of being
 // written by the prologue and read back. div: float32 (f64 = 0) or float64 values, row stride
-// ldd. active = 0: an ordinary cycle. alpha and mean are filled in on the device from the
-// solve state by the kernel that takes the struct.
+// ldd. active = 0: an ordinary cycle. div, ldd, alpha and mean are filled in on the device
+// from the solve state by the kernel that takes the struct.
 struct FirstCycle {
   const void* div;
   int64_t ldd;
@@ -614,6 +614,12 @@ __global__ void __launch_bounds__(32 * NWARP, MINB)
   fc.active = sizeof(TC) != sizeof(TP) && fc.active && st->cycles == 0;
   fc.alpha = st->alpha;
   fc.mean = st->bmean;
+  fc.div = st->div;
+  fc.ldd = st->ldd;
+  if (!p) {  // the solve's own pressure
+    p = (TP*)st->p;
+    ldp = st->ldp;
+  }
   if (inside)
     reg_post_final_body<TC, TP, SW, RPT, NWARP, false>(x, e_in, bsrc, bdst, ld, H, W, ec, ldc, Hc, Wc, omega, p, ldp,
                                                       r64, i0, j0, sq, fc);

@@ -140,6 +140,12 @@ __global__ void __launch_bounds__(32 * NWARP, MINB)
   fc.active = sizeof(TC) != sizeof(TP) && fc.active && st->cycles == 0;
   fc.alpha = st->alpha;
   fc.mean = st->bmean;
+  fc.div = st->div;
+  fc.ldd = st->ldd;
+  if (!p) {  // the solve's own pressure
+    p = (TP*)st->p;
+    ldp = st->ldp;
+  }
   if (inside) {
     const int t = threadIdx.x;
     // rows to stage: p and r64 (or p alone); on the first cycle only the divergence rows that

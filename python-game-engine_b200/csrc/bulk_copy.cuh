@@ -42,6 +42,20 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
       : "memory");
 }
 
+// One bulk copy of `bytes` (multiple of 16) from shared src to global dst, in the thread's
+// current bulk group; the generic writes to src are made visible to it by bulk_fence_shared
+// before a block barrier that precedes the copy.
+__device__ __forceinline__ void bulk_s2g(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_addr(src)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_fence_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// Close the thread's bulk group and wait until its copies have read shared memory.
+__device__ __forceinline__ void bulk_commit_wait_read() {
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+
 // Wait until the barrier's phase with the given parity has completed; false after the limit.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   const uint32_t a = smem_addr(bar);

@@ -12,10 +12,11 @@
 // Outer loop: residual-correction form r = b - A p (precision of p), e = cycle(r) in the
 // cycle precision, p += e; SG_GMG_MIXED runs FP32 cycles inside FP64 refinement.
 //
-// Execution: levels up to 1024 x 1024 cells in total shared-memory footprint run as one
-// thread block (the "tail": every level <= 128^2 in FP32, <= 64^2 in FP64, down to the
-// exact coarsest solve) so the launch-latency-bound coarse levels cost one launch per
-// visit. Larger levels use grid-wide kernels (zero-initial-guess first sweep and the
+// Execution: two launches per level and cycle, on register tiles (large open levels,
+// gmg_regtile.cuh) or register regions (the others, gmg_region.cuh), down to levels of 64 x 64
+// cells, which run as one thread block with the exact coarsest solve. Sweep counts beyond
+// three a side and fine levels with a closed face between fluid cells use grid-wide kernels
+// (zero-initial-guess first sweep and the
 // residual fused into the restriction). The tolerance loop is one CUDA graph whose
 // cycles sit in a conditional WHILE node; the convergence test runs on the device, so
 // a solve needs no host synchronisation.
@@ -53,6 +54,8 @@ struct LevelMask {
   }
 };
 
+#include "gmg_weights.cuh"
+
 constexpr int kHist = 128;  // relative residuals kept per solve (history[0] = initial)
 
 // Solve state in device memory (written by the graph, read by the host on demand).
@@ -60,7 +63,6 @@ struct GmgState {
   double bnorm;
   double relres;
   double tol;
-  double alpha;
   int cycles;
   int max_cycles;
   int status;  // 0 running, 1 converged, 2 cycle cap reached, 3 non-finite residual, 4 device error
@@ -69,13 +71,7 @@ struct GmgState {
   long long solves;
   long long failures;      // solves that ended at the cycle cap or on a non-finite residual
   double history[kHist];
-  double bmean;  // mean of alpha div over the fluid cells (when the plan removes it)
-  // the solve's fields: the kernels take them from here, so that one instantiated graph serves
-  // every pressure and divergence the plan is called with
-  void* p;
-  int64_t ldp;
-  const void* div;
-  int64_t ldd;
+  SolveFields f;
 };
 
 // ---------------------------------------------------------------- point operations
@@ -128,8 +124,6 @@ __device__ __forceinline__ void pcand(int j, int i, int Hc, int Wc, const LevelM
   for (int q = 1; q < 4; ++q)
     if (!cm.fluid(cj[q], ci[q])) { cj[q] = J; ci[q] = I; }
 }
-
-#include "gmg_weights.cuh"
 
 // (P^T r)(J, I) with r evaluated on the fly from e and b of the fine level.
 template <typename T>
@@ -239,11 +233,10 @@ inline dim3 grid_wide(int64_t W, int64_t H) {
 }
 
 template <typename T, typename TO>
-__global__ void k_gmg_fine_residual(int H, int W, const GmgState* __restrict__ st, const T* __restrict__ bf,
-                                    int64_t ldb, LevelMask m, TO* __restrict__ r, int64_t ldr, T* __restrict__ rfull,
-                                    double* __restrict__ partial) {
-  const T* p = (const T*)st->p;
-  const int64_t ldp = st->ldp;
+__device__ __forceinline__ void fine_residual_body(int H, int W, const T* __restrict__ p, int64_t ldp,
+                                                   const T* __restrict__ bf, int64_t ldb, const LevelMask& m,
+                                                   TO* __restrict__ r, int64_t ldr, T* __restrict__ rfull,
+                                                   double* __restrict__ partial) {
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int ib = blockIdx.x * kWX + threadIdx.x;
   double sq = 0.0;
@@ -262,22 +255,27 @@ __global__ void k_gmg_fine_residual(int H, int W, const GmgState* __restrict__ s
   double s = block_sum(sq);
   if (threadIdx.x == 0 && threadIdx.y == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = s;
 }
+// The pointers from the solve state go through a function's restrict parameters: as plain
+// pointers the loads of a thread's later cells waited for the stores of its earlier ones
+// (256^2 float32 4.3 instead of 3.3 us; the rhs kernel at 2048^2 15.7 instead of 12.1).
+template <typename T, typename TO>
+__global__ void k_gmg_fine_residual(int H, int W, const GmgState* __restrict__ st, const T* __restrict__ bf,
+                                    int64_t ldb, LevelMask m, TO* __restrict__ r, int64_t ldr, T* __restrict__ rfull,
+                                    double* __restrict__ partial) {
+  fine_residual_body<T, TO>(H, W, (const T*)st->f.p, st->f.ldp, bf, ldb, m, r, ldr, rfull, partial);
+}
 
 // bf = alpha * div on fluid cells (alpha from the solve state; b may be null when only the
 // outputs below are needed) plus per-block sums of bf^2.
 // For a zero initial guess it also writes p = 0 and, bf being the residual,
 // the first cycle's rhs b0 (cycle precision) and the carried residual r64 (when kept).
 template <typename TD, typename TB, typename TC>
-__global__ void k_gmg_rhs(int H, int W, const GmgState* __restrict__ st, LevelMask m, TB* __restrict__ b, int64_t ldb,
-                          double* __restrict__ partial, int zero_guess, TC* __restrict__ b0, int64_t ld0,
-                          TB* __restrict__ r64, int sub_mean) {
-  const TD* div = (const TD*)st->div;
-  const int64_t ldd = st->ldd, ldpz = st->ldp;
-  TB* pz = zero_guess ? (TB*)st->p : nullptr;
+__device__ __forceinline__ void rhs_body(int H, int W, const TD* __restrict__ div, int64_t ldd, double alpha,
+                                         double mean, const LevelMask& m, TB* __restrict__ b, int64_t ldb,
+                                         double* __restrict__ partial, TB* __restrict__ pz, int64_t ldpz,
+                                         TC* __restrict__ b0, int64_t ld0, TB* __restrict__ r64, int sub_mean) {
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int ib = blockIdx.x * kWX + threadIdx.x;
-  const double alpha = st->alpha;
-  const double mean = sub_mean ? st->bmean : 0.0;
   double sq = 0.0;
   if (j < H) {
 #pragma unroll
@@ -286,8 +284,8 @@ __global__ void k_gmg_rhs(int H, int W, const GmgState* __restrict__ st, LevelMa
       if (i < W) {
         TB v = (TB)0;
         if (m.fluid(j, i)) {
-          double x = alpha * (double)div[(int64_t)j * ldd + i];
-          if (sub_mean) x -= mean;
+          double x = __dmul_rn(alpha, (double)div[(int64_t)j * ldd + i]);
+          if (sub_mean) x = __dsub_rn(x, mean);
           v = (TB)x;
           sq += (double)v * (double)v;
         }
@@ -303,12 +301,18 @@ __global__ void k_gmg_rhs(int H, int W, const GmgState* __restrict__ st, LevelMa
   double s = block_sum(sq);
   if (threadIdx.x == 0 && threadIdx.y == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = s;
 }
+template <typename TD, typename TB, typename TC>
+__global__ void k_gmg_rhs(int H, int W, const GmgState* __restrict__ st, LevelMask m, TB* __restrict__ b, int64_t ldb,
+                          double* __restrict__ partial, int zero_guess, TC* __restrict__ b0, int64_t ld0,
+                          TB* __restrict__ r64, int sub_mean) {
+  rhs_body<TD, TB, TC>(H, W, (const TD*)st->f.div, st->f.ldd, st->f.alpha, sub_mean ? st->f.bmean : 0.0, m, b, ldb,
+                       partial, zero_guess ? (TB*)st->f.p : nullptr, st->f.ldp, b0, ld0, r64, sub_mean);
+}
 
 // p += e (fine precision += cycle precision).
 template <typename TP, typename TE>
-__global__ void k_gmg_correct(int H, int W, const GmgState* __restrict__ st, const TE* __restrict__ e, int64_t lde) {
-  TP* p = (TP*)st->p;
-  const int64_t ldp = st->ldp;
+__device__ __forceinline__ void correct_body(int H, int W, TP* __restrict__ p, int64_t ldp, const TE* __restrict__ e,
+                                             int64_t lde) {
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int ib = blockIdx.x * kWX + threadIdx.x;
   if (j >= H) return;
@@ -317,6 +321,10 @@ __global__ void k_gmg_correct(int H, int W, const GmgState* __restrict__ st, con
     const int i = ib + 32 * q;
     if (i < W) p[(int64_t)j * ldp + i] += (TP)e[(int64_t)j * lde + i];
   }
+}
+template <typename TP, typename TE>
+__global__ void k_gmg_correct(int H, int W, const GmgState* __restrict__ st, const TE* __restrict__ e, int64_t lde) {
+  correct_body<TP, TE>(H, W, (TP*)st->f.p, st->f.ldp, e, lde);
 }
 
 // Sum of partial[0 .. n) over one block (1-D, a multiple of 32 threads): strided sums, then
@@ -337,11 +345,11 @@ __device__ __forceinline__ double sum_partials(const double* __restrict__ partia
 
 __global__ void k_gmg_set_params(GmgState* st, double alpha, double tol, int max_cycles, void* p, int64_t ldp,
                                  const void* div, int64_t ldd) {
-  st->p = p;
-  st->ldp = ldp;
-  st->div = div;
-  st->ldd = ldd;
-  st->alpha = alpha;
+  st->f.p = p;
+  st->f.ldp = ldp;
+  st->f.div = div;
+  st->f.ldd = ldd;
+  st->f.alpha = alpha;
   st->tol = tol;
   st->max_cycles = max_cycles;
   st->cycles = 0;
@@ -353,8 +361,8 @@ __global__ void k_gmg_set_params(GmgState* st, double alpha, double tol, int max
 template <typename TD>
 __global__ void k_gmg_rhs_sum(int H, int W, const GmgState* __restrict__ st, LevelMask m,
                               double* __restrict__ partial) {
-  const TD* div = (const TD*)st->div;
-  const int64_t ldd = st->ldd;
+  const TD* div = (const TD*)st->f.div;
+  const int64_t ldd = st->f.ldd;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int ib = blockIdx.x * kWX + threadIdx.x;
   double acc = 0.0;
@@ -371,7 +379,7 @@ __global__ void k_gmg_rhs_sum(int H, int W, const GmgState* __restrict__ st, Lev
 
 __global__ void k_gmg_finalize_mean(const double* __restrict__ partial, int n, GmgState* st, double inv_fluid) {
   double s = sum_partials(partial, n);
-  if (threadIdx.x == 0) st->bmean = st->alpha * (s * inv_fluid);
+  if (threadIdx.x == 0) st->f.bmean = st->f.alpha * (s * inv_fluid);
 }
 
 __global__ void k_gmg_finalize_norm(const double* __restrict__ partial, int n, GmgState* st) {
@@ -1054,183 +1062,6 @@ static void coarse_dct_tables_split(int H, int W, int nc, std::vector<double>& t
       for (int kl = 0; kl < wc; ++kl)
         sp[(size_t)c * W * wc + (size_t)i * wc + kl] = cxt[(size_t)i * W + c * wc + kl];
 }
-// Levels up to this many cells a side run inside the single-block tail kernel; larger
-// open-box levels use the fused tiled kernels (two launches per level and cycle).
-constexpr int kTailMaxSide = 16;
-constexpr int kTailThreads = 1024;
-
-template <typename T>
-struct TailArgs {
-  int n;                    // tail levels; the last one is the coarsest (exact solve)
-  LevelMask m[kMaxLevels];  // masks (codes in global memory)
-  int off_e[kMaxLevels];    // shared-memory offsets (elements of T), row stride = W
-  int off_b[kMaxLevels];
-  int off_x;                // restriction scratch: rows x coarse columns of the first level
-  T* ge;                    // first tail level in global memory (e in/out, b in)
-  const T* gb;
-  int64_t gld;
-  const double* pinv;       // coarsest pseudo-inverse
-  T omega;
-  int pre, post, wcycle, zero_init;
-};
-
-
-// Open-face bits of (j, i): analytic levels from the bounds, others from their codes.
-__device__ __forceinline__ uint8_t tail_code(const LevelMask& m, int j, int i) {
-  if (!m.analytic) return m.code[j * m.W + i];
-  return (uint8_t)(C_FLUID | (i > 0 ? C_L : 0) | (i < m.W - 1 ? C_R : 0) | (j > 0 ? C_D : 0) | (j < m.H - 1 ? C_U : 0));
-}
-
-// Half sweep over shared-memory arrays (row stride W); threads laid out 32 x 32.
-template <typename T>
-__device__ void tail_relax(const LevelMask& m, T* e, const T* b, T omega, int color) {
-  const int H = m.H, W = m.W, Wh = (W + 1) >> 1;
-  for (int j = threadIdx.y; j < H; j += blockDim.y) {
-    const int par = (j + color) & 1;
-    for (int k = threadIdx.x; k < Wh; k += blockDim.x) {
-      const int i = 2 * k + par;
-      if (i >= W) continue;
-      const uint8_t c = tail_code(m, j, i);
-      if (!(c & C_FLUID)) continue;
-      const int o = j * W + i;
-      T acc = b[o];
-      int n = 0;
-      if (c & C_L) { acc += e[o - 1]; ++n; }
-      if (c & C_R) { acc += e[o + 1]; ++n; }
-      if (c & C_D) { acc += e[o - W]; ++n; }
-      if (c & C_U) { acc += e[o + W]; ++n; }
-      if (n == 0) continue;
-      const T x = e[o];
-      e[o] = x + omega * (acc * rcp_open<T>(n) - x);
-    }
-  }
-  __syncthreads();
-}
-
-// Residual b - A e at (j, i) of a shared-memory level.
-template <typename T>
-__device__ __forceinline__ T tail_res(const LevelMask& m, const T* e, const T* b, int j, int i) {
-  const uint8_t c = tail_code(m, j, i);
-  if (!(c & C_FLUID)) return (T)0;
-  const int W = m.W, o = j * W + i;
-  const T x = e[o];
-  T acc = b[o];
-  if (c & C_L) acc += e[o - 1] - x;
-  if (c & C_R) acc += e[o + 1] - x;
-  if (c & C_D) acc += e[o - W] - x;
-  if (c & C_U) acc += e[o + W] - x;
-  return acc;
-}
-
-// bc = P^T (b - A e), ec = 0. Analytic level pairs use the separable form: rows of the
-// fine level are first restricted along x into the scratch X (H x Wc), then along y.
-template <typename T>
-__device__ void tail_restrict(const LevelMask& m, const T* e, const T* b, const LevelMask& cm, T* bc, T* ec, T* X) {
-  const int H = m.H, W = m.W, Hc = cm.H, Wc = cm.W;
-  if (m.analytic && cm.analytic) {
-    for (int j = threadIdx.y; j < H; j += blockDim.y)
-      for (int I = threadIdx.x; I < Wc; I += blockDim.x) {
-        T acc = (T)0;
-#pragma unroll
-        for (int d = 0; d < 4; ++d) {
-          const int i = 2 * I - 1 + d;
-          if (i < 0 || i >= W) continue;
-          const T w = (T)w1(i, I, Wc);
-          if (w != (T)0) acc += w * tail_res(m, e, b, j, i);
-        }
-        X[j * Wc + I] = acc;
-      }
-    __syncthreads();
-    for (int J = threadIdx.y; J < Hc; J += blockDim.y)
-      for (int I = threadIdx.x; I < Wc; I += blockDim.x) {
-        T acc = (T)0;
-#pragma unroll
-        for (int d = 0; d < 4; ++d) {
-          const int j = 2 * J - 1 + d;
-          if (j < 0 || j >= H) continue;
-          const T w = (T)w1(j, J, Hc);
-          if (w != (T)0) acc += w * X[j * Wc + I];
-        }
-        bc[J * Wc + I] = acc;
-        ec[J * Wc + I] = (T)0;
-      }
-  } else {
-    for (int J = threadIdx.y; J < Hc; J += blockDim.y)
-      for (int I = threadIdx.x; I < Wc; I += blockDim.x) {
-        bc[J * Wc + I] = restrict_at(J, I, e, (int64_t)W, b, (int64_t)W, m, cm);
-        ec[J * Wc + I] = (T)0;
-      }
-  }
-  __syncthreads();
-}
-
-// e += P ec on the fluid cells of a shared-memory level.
-template <typename T>
-__device__ void tail_prolong(const LevelMask& m, T* e, const LevelMask& cm, const T* ec) {
-  for (int j = threadIdx.y; j < m.H; j += blockDim.y)
-    for (int i = threadIdx.x; i < m.W; i += blockDim.x)
-      if (m.fluid(j, i)) e[j * m.W + i] += prolong_at(j, i, ec, (int64_t)cm.W, cm);
-  __syncthreads();
-}
-
-template <typename T>
-__device__ void tail_coarse_solve(const LevelMask& m, T* e, const T* b, const double* __restrict__ pinv) {
-  int n = m.H * m.W;
-  int tid = threadIdx.y * blockDim.x + threadIdx.x;
-  int lane = tid & 31, warp = tid >> 5, nw = (blockDim.x * blockDim.y) >> 5;
-  for (int row = warp; row < n; row += nw) {
-    double acc = 0.0;
-    for (int q = lane; q < n; q += 32) acc += pinv[(int64_t)row * n + q] * (double)b[q];
-    acc = warp_sum(acc);
-    if (lane == 0) e[row] = (T)acc;
-  }
-  __syncthreads();
-}
-
-template <typename T>
-__device__ __noinline__ void tail_cycle(const TailArgs<T>& a, T* sm, int k) {
-  const LevelMask& m = a.m[k];
-  T* e = sm + a.off_e[k];
-  T* b = sm + a.off_b[k];
-  if (k == a.n - 1) {
-    tail_coarse_solve(m, e, b, a.pinv);
-    return;
-  }
-  for (int s = 0; s < a.pre; ++s) {
-    tail_relax(m, e, b, a.omega, 0);
-    tail_relax(m, e, b, a.omega, 1);
-  }
-  const LevelMask& cm = a.m[k + 1];
-  T* ec = sm + a.off_e[k + 1];
-  T* bc = sm + a.off_b[k + 1];
-  tail_restrict(m, (const T*)e, (const T*)b, cm, bc, ec, sm + a.off_x);
-  int reps = (a.wcycle && k + 1 < a.n - 1) ? 2 : 1;
-  for (int q = 0; q < reps; ++q) tail_cycle(a, sm, k + 1);
-  tail_prolong(m, e, cm, (const T*)ec);
-  for (int s = 0; s < a.post; ++s) {
-    tail_relax(m, e, b, a.omega, 0);
-    tail_relax(m, e, b, a.omega, 1);
-  }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kTailThreads) k_gmg_tail(const __grid_constant__ TailArgs<T> a) {
-  extern __shared__ __align__(16) unsigned char tail_smem[];
-  T* sm = reinterpret_cast<T*>(tail_smem);
-  const LevelMask& m0 = a.m[0];
-  T* e0 = sm + a.off_e[0];
-  T* b0 = sm + a.off_b[0];
-  for (int j = threadIdx.y; j < m0.H; j += blockDim.y)
-    for (int i = threadIdx.x; i < m0.W; i += blockDim.x) {
-      b0[j * m0.W + i] = a.gb[(int64_t)j * a.gld + i];
-      e0[j * m0.W + i] = a.zero_init ? (T)0 : a.ge[(int64_t)j * a.gld + i];
-    }
-  __syncthreads();
-  tail_cycle(a, sm, 0);
-  for (int j = threadIdx.y; j < m0.H; j += blockDim.y)
-    for (int i = threadIdx.x; i < m0.W; i += blockDim.x) a.ge[(int64_t)j * a.gld + i] = e0[j * m0.W + i];
-}
-
 // Tiled bc = P^T (b - A e) for analytic (open-box) level pairs: a 32 x 8 block restricts
 // a 32 x 8 tile of coarse cells; the fine residual of the tile (18 x 66 cells including
 // the window overlap) is computed once into shared memory from e (20 x 68) and b, then
@@ -1300,10 +1131,9 @@ __global__ void __launch_bounds__(kRX * kRY) k_gmg_residual_restrict_tiled(const
 }
 
 // ---------------------------------------------------------------- fused tiled level kernels
-#include "gmg_tiled.cuh"
-#include "gmg_tail_open.cuh"
 #include "gmg_regtile.cuh"
 #include "gmg_regtile_stage.cuh"
+#include "gmg_region.cuh"
 
 // ---------------------------------------------------------------- plan
 struct Level {
@@ -1311,8 +1141,10 @@ struct Level {
   int64_t ld = 0;              // row stride of the real arrays
   int analytic = 0;            // every cell fluid and every interior face open
   std::vector<uint8_t> code;   // H * W codes (host), empty when analytic
-  int fused = 0;               // this level and the next run the fused tiled kernels
-  int64_t off_e = 0, off_e2 = 0, off_b = 0, off_code = 0;  // e2: second e buffer (fused levels)
+  int fused = 0;               // an open box above another one: register tiles where large
+  int simple = 1;              // every face between two fluid cells is open
+  int region = 0;              // runs the region kernels (gmg_region.cuh)
+  int64_t off_e = 0, off_e2 = 0, off_b = 0, off_code = 0;  // e2: second e buffer (fused and region levels)
 };
 
 }  // namespace sg
@@ -1331,7 +1163,7 @@ struct sg_gmg_plan {
   int64_t dct_cluster_smem[2] = {0, 0};  // forward, inverse
   int dct_fp64 = 0;           // the transform's arithmetic and tables in float64 (FP64 and mixed precision)
   // the first cycle of a graph solve from a zero guess (set while its graph is captured)
-  mutable sg::FirstCycle fc{nullptr, 0, 0, 0, 0, 0.0, 0.0};
+  mutable sg::FirstCycle fc{nullptr, 0, 0, 0};
   // events recorded around the fused fine-level post launches of kernel-by-kernel solves
   // (pairs, consumed in order; sg_gmg_set_post_events)
   mutable std::vector<cudaEvent_t> post_ev;
@@ -1341,8 +1173,7 @@ struct sg_gmg_plan {
   std::vector<double> dct;
   std::vector<float> dct_f;  // the same in float, for FP32 cycles
   int64_t off_dct = 0, dct_smem = 0;
-  int tail_start = 0;        // first level handled by the single-block tail kernel
-  int tail_open = 0;         // every tail level is an open box (k_gmg_tail_open)
+  int tail_start = 0;        // first level of the single-block tail (k_gmg_tail_region)
   int64_t tail_smem = 0;     // its dynamic shared memory (bytes)
   int64_t off_pinv = 0, off_bfine = 0, off_partial = 0, off_state = 0, bytes = 0;
   int64_t ld_bfine = 0;
@@ -1352,6 +1183,9 @@ struct sg_gmg_plan {
   // the residual in the precision of p when that differs from the cycle precision
   int fused_ir = 0;
   int64_t off_b2 = 0, off_r64 = 0;
+  // the same on a region fine level: 1 carries the residual likewise; 2 (float32 solves) only
+  // adds the correction to p, and the residual is formed from p afresh
+  int region_ir = 0;
   // cycles per refinement step (classical iterative refinement): with inner >= 2 the body
   // runs `inner` cycles on the cycle-precision correction from zero, then one p += e and one
   // fine-precision residual, instead of the fused fine level's per-cycle correction
@@ -1405,6 +1239,34 @@ static std::vector<uint8_t> pack_codes(const std::vector<uint8_t>& fl, const std
       c[(size_t)j * W + i] = x;
     }
   return c;
+}
+
+// Whether every face between two fluid cells is open (the region kernels rely on it).
+static bool faces_follow_cells(const std::vector<uint8_t>& c, int H, int W) {
+  for (int j = 0; j < H; ++j)
+    for (int i = 0; i < W; ++i) {
+      const uint8_t k = c[(size_t)j * W + i];
+      if (!(k & C_FLUID)) continue;
+      if (i + 1 < W && (c[(size_t)j * W + i + 1] & C_FLUID) && !(k & C_R)) return false;
+      if (j + 1 < H && (c[(size_t)(j + 1) * W + i] & C_FLUID) && !(k & C_U)) return false;
+    }
+  return true;
+}
+
+// Adds the transfer bits (C_XHOME ..) to a level's codes (pcand's rule).
+static void add_transfer_codes(Level& L, const Level& C) {
+  if (L.analytic || C.analytic) return;
+  auto fluid = [&](int J, int I) { return (C.code[(size_t)J * C.W + I] & C_FLUID) != 0; };
+  for (int j = 0; j < L.H; ++j)
+    for (int i = 0; i < L.W; ++i) {
+      const int J = j >> 1, I = i >> 1;
+      const int X = std::min(std::max(I + ((i & 1) ? 1 : -1), 0), C.W - 1);
+      const int Y = std::min(std::max(J + ((j & 1) ? 1 : -1), 0), C.H - 1);
+      uint8_t& k = L.code[(size_t)j * L.W + i];
+      if (X != I && !fluid(J, X)) k |= C_XHOME;
+      if (Y != J && !fluid(Y, I)) k |= C_YHOME;
+      if ((X != I || Y != J) && !fluid(Y, X)) k |= C_DHOME;
+    }
 }
 
 // Pseudo-inverse of the graph Laplacian A of one level: A+ = (A + Pi)^-1 - Pi, with Pi
@@ -1518,53 +1380,28 @@ static T* ws_ptr(const sg_gmg_plan* p, int64_t off) {
 
 static GmgState* state_ptr(const sg_gmg_plan* p) { return (GmgState*)(p->ws + p->off_state); }
 
-// Shared-memory layout of the open-box tail (elements of T): every level's e planes first
-// (zeroed at start), then the b planes, then the restriction and residual scratch.
-struct OpenTailLayout {
-  int off_e[kMaxLevels], off_b[kMaxLevels], e_total, off_x, off_r, total;
-};
+// Cells of the tail's levels, and each level's first one.
+static int tail_cells(const std::vector<Level>& levels, int start, int* off) {
+  int cells = 0;
+  for (size_t q = start; q < levels.size(); ++q) {
+    if (off) off[q - start] = cells;
+    cells += levels[q].H * levels[q].W;
+  }
+  return cells;
+}
 
-static OpenTailLayout open_tail_layout(const std::vector<Level>& levels, int start) {
-  OpenTailLayout t;
-  std::memset(&t, 0, sizeof(t));
-  int n = (int)levels.size() - start;
-  int off = 0;
-  for (int q = 0; q < n; ++q) {
-    const Level& L = levels[start + q];
-    const int wh = (L.W + 1) / 2;
-    t.off_e[q] = off;
-    off += 2 * (L.H + 2) * (wh + 2);
-  }
-  t.e_total = off;
-  for (int q = 0; q < n; ++q) {
-    const Level& L = levels[start + q];
-    t.off_b[q] = off;
-    off += 2 * L.H * ((L.W + 1) / 2);
-  }
-  t.off_x = off;
-  off += levels[start].H * ((levels[start].W + 1) / 2);
-  t.off_r = off;
-  off += levels[start].H * levels[start].W;
-  t.total = off;
-  return t;
+static RegionLevel region_level(const sg_gmg_plan* p, int k) {
+  const Level& L = p->levels[k];
+  return RegionLevel{L.analytic ? nullptr : (const uint8_t*)(p->ws + L.off_code), L.H, L.W};
 }
 
 template <typename T>
-static int tail_open_launch(const sg_gmg_plan* p, bool zero_init, cudaStream_t s) {
-  OpenTailArgs<T> a;
+static void tail_launch(const sg_gmg_plan* p, bool zero_init, cudaStream_t s) {
+  RegionTailArgs<T> a;
   std::memset(&a, 0, sizeof(a));
-  int nl = (int)p->levels.size();
-  a.n = nl - p->tail_start;
-  OpenTailLayout t = open_tail_layout(p->levels, p->tail_start);
-  for (int q = 0; q < a.n; ++q) {
-    a.H[q] = p->levels[p->tail_start + q].H;
-    a.W[q] = p->levels[p->tail_start + q].W;
-    a.off_e[q] = t.off_e[q];
-    a.off_b[q] = t.off_b[q];
-  }
-  a.e_total = t.e_total;
-  a.off_x = t.off_x;
-  a.off_r = t.off_r;
+  a.n = (int)p->levels.size() - p->tail_start;
+  a.cells = tail_cells(p->levels, p->tail_start, a.off);
+  for (int q = 0; q < a.n; ++q) a.m[q] = region_level(p, p->tail_start + q);
   const Level& L0 = p->levels[p->tail_start];
   a.ge = ws_ptr<T>(p, L0.off_e);
   a.gb = ws_ptr<T>(p, L0.off_b);
@@ -1575,91 +1412,75 @@ static int tail_open_launch(const sg_gmg_plan* p, bool zero_init, cudaStream_t s
   a.post = p->post;
   a.wcycle = p->cycle;
   a.zero_init = zero_init ? 1 : 0;
-  SG_LAUNCH(k_gmg_tail_open<T><<<1, dim3(32, kOpenTailThreads / 32), p->tail_smem, s>>>(a));
-  return SG_OK;
+  SG_LAUNCH(k_gmg_tail_region<T><<<1, kRgThreads, p->tail_smem, s>>>(a));
 }
 
-template <typename T>
-static int tail_launch(const sg_gmg_plan* p, bool zero_init, cudaStream_t s) {
-  if (p->tail_open) return tail_open_launch<T>(p, zero_init, s);
-  TailArgs<T> a;
-  std::memset(&a, 0, sizeof(a));
-  int nl = (int)p->levels.size();
-  a.n = nl - p->tail_start;
-  int64_t off = 0;
-  for (int q = 0; q < a.n; ++q) {
-    const Level& L = p->levels[p->tail_start + q];
-    a.m[q] = level_mask(p, p->tail_start + q);
-    a.off_e[q] = (int)off;
-    off += (int64_t)L.H * L.W;
-    a.off_b[q] = (int)off;
-    off += (int64_t)L.H * L.W;
-    off = (off + 3) & ~(int64_t)3;
-  }
-  a.off_x = (int)off;
-  const Level& L0 = p->levels[p->tail_start];
-  a.ge = ws_ptr<T>(p, L0.off_e);
-  a.gb = ws_ptr<T>(p, L0.off_b);
-  a.gld = L0.ld;
-  a.pinv = (const double*)(p->ws + p->off_pinv);
-  a.omega = (T)p->omega;
-  a.pre = p->pre;
-  a.post = p->post;
-  a.wcycle = p->cycle;
-  a.zero_init = zero_init ? 1 : 0;
-  SG_LAUNCH(k_gmg_tail<T><<<1, dim3(32, kTailThreads / 32), p->tail_smem, s>>>(a));
-  return SG_OK;
-}
-
-// The fused tiled kernels serve open-box level pairs with 1..3 sweeps per side.
-static bool fused_level(const sg_gmg_plan* p, int k) { return p->levels[k].fused != 0; }
-
-// Register tiles on levels of at least SG_GMG_REG_MIN_TILES 64 x 32 blocks, 16 x 16 shared-
-// memory tiles below: a small level is latency-bound, and more blocks with less serial work
-// each finish sooner. Per V-cycle at 2048^2 (32^2 exact coarsest; mixed / float64 / float32):
-// threshold 296 (512^2 on small tiles) 139 / 165 / 125 us, 100 (512^2 on register tiles)
-// 137 / 159 / 123, 30 (256^2 too) 141 / 160 / 127, every level 150 / 163 / 136.
+// Register tiles on open levels of at least SG_GMG_REG_MIN_TILES 64 x 32 blocks, regions of
+// 32 x 64 cells below: a small level is latency-bound, and two rows a thread finish sooner than
+// six (256^2 float32: pre 11.7 on register tiles, 5.6 on 16 x 16 shared-memory tiles, 3.6 us on
+// regions; post 7.8 / 4.3 / 3.4).
 #ifndef SG_GMG_REG_MIN_TILES
 #define SG_GMG_REG_MIN_TILES 100
 #endif
 static bool small_tiles(const Level& L) {
-  const int64_t large_blocks = (int64_t)((L.W + kTX - 1) / kTX) * ((L.H + kTY - 1) / kTY);
+  const int64_t large_blocks = (int64_t)((L.W + 63) / 64) * ((L.H + 31) / 32);
   return large_blocks < SG_GMG_REG_MIN_TILES;
 }
 
-// Rows of 32 threads of a shared-memory tile block: kTBY, or SG_TILE_FEW_ROWS on levels of
-// at most SG_TILE_FEW_TILES tiles (a wave or less of blocks: more threads per block
-// shorten each phase of the block, which is all the level costs).
-#ifndef SG_TILE_FEW_TILES
-#define SG_TILE_FEW_TILES 256
-#endif
-#ifndef SG_TILE_FEW_ROWS
-#define SG_TILE_FEW_ROWS 16
-#endif
-static dim3 tile_block(dim3 g) {
-  return dim3(kTBX, (int64_t)g.x * g.y <= SG_TILE_FEW_TILES ? SG_TILE_FEW_ROWS : kTBY);
-}
-
-template <typename T, int SW, int TX, int TY>
-static void launch_pre_t(const sg_gmg_plan* p, int k, bool zero_init, cudaStream_t s) {
+template <typename T>
+static RegionArgs<T> region_args(const sg_gmg_plan* p, int k) {
   const Level& L = p->levels[k];
   const Level& C = p->levels[k + 1];
-  dim3 g((L.W + TX - 1) / TX, (L.H + TY - 1) / TY);
-  // reads E0 (nothing for a zero initial guess), writes E1
-  SG_LAUNCH(k_gmg_pre_tiled<T, SW, TX, TY><<<g, tile_block(g), PreShape<SW, TX, TY>::template bytes<T>(), s>>>(
-      zero_init ? nullptr : ws_ptr<T>(p, L.off_e), ws_ptr<T>(p, L.off_e2), ws_ptr<T>(p, L.off_b), L.ld, L.H, L.W,
-      ws_ptr<T>(p, C.off_b), C.ld, C.H, C.W, (T)p->omega));
+  RegionArgs<T> a;
+  std::memset(&a, 0, sizeof(a));
+  a.m = region_level(p, k);
+  a.Hc = C.H;
+  a.Wc = C.W;
+  a.ld = L.ld;
+  a.ldc = C.ld;
+  a.b = ws_ptr<T>(p, L.off_b);
+  a.omega = (T)p->omega;
+  a.st = state_ptr(p);
+  return a;
 }
 
-template <typename T, int SW, int TX, int TY>
-static void launch_post_t(const sg_gmg_plan* p, int k, cudaStream_t s) {
+static dim3 region_grid(const Level& L, int halo) {
+  return dim3((unsigned)region_tiles(L.W, kRgCols, halo), (unsigned)region_tiles(L.H, kRgWarps * kRgRows, halo));
+}
+// The values that a tile's edge has spoilt after its half sweeps, and the residual's and the
+// restriction's reach, rounded up to even.
+static int region_halo(int sweeps, bool residual) { return 2 * sweeps + (residual ? 2 : 0); }
+
+// E0 (nothing for a zero initial guess) -> E1 and the coarse rhs; b_alt: see k_gmg_pre_region
+template <typename T>
+static void launch_pre_region(const sg_gmg_plan* p, int k, bool zero_init, T* b_alt, cudaStream_t s) {
   const Level& L = p->levels[k];
-  const Level& C = p->levels[k + 1];
-  dim3 g((L.W + TX - 1) / TX, (L.H + TY - 1) / TY);
-  // reads E1 and the coarse correction (the coarse level's E0), writes E0
-  SG_LAUNCH(k_gmg_post_tiled<T, SW, TX, TY><<<g, tile_block(g), PostShape<SW, TX, TY>::template bytes<T>(), s>>>(
-      ws_ptr<T>(p, L.off_e2), ws_ptr<T>(p, L.off_e), ws_ptr<T>(p, L.off_b), L.ld, L.H, L.W, ws_ptr<T>(p, C.off_e),
-      C.ld, C.H, C.W, (T)p->omega));
+  RegionArgs<T> a = region_args<T>(p, k);
+  a.e_in = zero_init ? nullptr : ws_ptr<T>(p, L.off_e);
+  a.e_out = ws_ptr<T>(p, L.off_e2);
+  a.b_alt = b_alt;
+  a.bc = ws_ptr<T>(p, p->levels[k + 1].off_b);
+  a.sweeps = p->pre;
+  a.halo = region_halo(p->pre, true);
+  SG_LAUNCH(k_gmg_pre_region<T><<<region_grid(L, a.halo), kRgThreads, 0, s>>>(a));
+}
+
+// E1 and the coarse correction (the coarse level's E0) -> E0, or the end of a solve's cycle
+template <typename T, typename TP, int FINAL>
+static dim3 launch_post_region(const sg_gmg_plan* p, int k, T* b_alt, cudaStream_t s) {
+  const Level& L = p->levels[k];
+  RegionArgs<T> a = region_args<T>(p, k);
+  a.e_in = ws_ptr<T>(p, L.off_e2);
+  a.e_out = ws_ptr<T>(p, L.off_e);
+  a.b_alt = b_alt;
+  a.ec = ws_ptr<T>(p, p->levels[k + 1].off_e);
+  a.sweeps = p->post;
+  a.halo = region_halo(p->post, FINAL == 1);
+  a.r64 = FINAL == 1 && p->off_r64 ? (void*)(p->ws + p->off_r64) : nullptr;
+  a.partial = (double*)(p->ws + p->off_partial);
+  const dim3 g = region_grid(L, a.halo);
+  SG_LAUNCH((k_gmg_post_region<T, TP, FINAL><<<g, kRgThreads, 0, s>>>(a)));
+  return g;
 }
 
 template <typename T, int SW>
@@ -1729,43 +1550,6 @@ static void launch_post_final(const sg_gmg_plan* p, TP* pp, int64_t ldp, bool al
         p->fc));
   }
   if (ev1) cudaEventRecord(ev1, s);
-}
-
-// Large levels: register tiles; small levels: 16 x 16 shared-memory tiles.
-template <typename T, int SW>
-static void launch_pre(const sg_gmg_plan* p, int k, bool zero_init, cudaStream_t s) {
-  if (small_tiles(p->levels[k]))
-    launch_pre_t<T, SW, kSX, kSY>(p, k, zero_init, s);
-  else
-    launch_pre_reg<T, SW>(p, k, zero_init, s);
-}
-
-template <typename T, int SW>
-static void launch_post(const sg_gmg_plan* p, int k, cudaStream_t s) {
-  if (small_tiles(p->levels[k]))
-    launch_post_t<T, SW, kSX, kSY>(p, k, s);
-  else
-    launch_post_reg<T, SW>(p, k, s);
-}
-
-template <typename T>
-static int set_tiled_smem_limits() {
-  cudaError_t e = cudaSuccess;
-#define SG_TILED_ATTR(SW, TX, TY)                                                                                  \
-  e = cudaFuncSetAttribute(k_gmg_pre_tiled<T, SW, TX, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
-                           (int)PreShape<SW, TX, TY>::template bytes<T>());                                        \
-  if (e != cudaSuccess) return fail(SG_ERR_CUDA, "smem attr: %s", cudaGetErrorString(e));                          \
-  e = cudaFuncSetAttribute(k_gmg_post_tiled<T, SW, TX, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize,           \
-                           (int)PostShape<SW, TX, TY>::template bytes<T>());                                       \
-  if (e != cudaSuccess) return fail(SG_ERR_CUDA, "smem attr: %s", cudaGetErrorString(e));
-  SG_TILED_ATTR(1, kTX, kTY)
-  SG_TILED_ATTR(2, kTX, kTY)
-  SG_TILED_ATTR(3, kTX, kTY)
-  SG_TILED_ATTR(1, kSX, kSY)
-  SG_TILED_ATTR(2, kSX, kSY)
-  SG_TILED_ATTR(3, kSX, kSY)
-#undef SG_TILED_ATTR
-  return SG_OK;
 }
 
 // Thread groups of k_dct_stream for a level W cells wide (at most 256 threads a block).
@@ -1892,18 +1676,24 @@ static void cycle(const sg_gmg_plan* p, int k, bool zero_init, cudaStream_t s) {
     return;
   }
   const int nl = (int)p->levels.size();
-  if (fused_level(p, k)) {
+  const int reps = (p->cycle == 1 && k + 1 < nl - 1) ? 2 : 1;
+  if (p->levels[k].region) {
+    launch_pre_region<T>(p, k, zero_init, nullptr, s);
+    for (int q = 0; q < reps; ++q) cycle<T>(p, k + 1, q == 0, s);
+    launch_post_region<T, T, 0>(p, k, nullptr, s);
+    return;
+  }
+  if (p->levels[k].fused) {
     switch (p->pre) {
-      case 1: launch_pre<T, 1>(p, k, zero_init, s); break;
-      case 2: launch_pre<T, 2>(p, k, zero_init, s); break;
-      default: launch_pre<T, 3>(p, k, zero_init, s); break;
+      case 1: launch_pre_reg<T, 1>(p, k, zero_init, s); break;
+      case 2: launch_pre_reg<T, 2>(p, k, zero_init, s); break;
+      default: launch_pre_reg<T, 3>(p, k, zero_init, s); break;
     }
-    int reps = (p->cycle == 1 && k + 1 < nl - 1) ? 2 : 1;
     for (int q = 0; q < reps; ++q) cycle<T>(p, k + 1, q == 0, s);
     switch (p->post) {
-      case 1: launch_post<T, 1>(p, k, s); break;
-      case 2: launch_post<T, 2>(p, k, s); break;
-      default: launch_post<T, 3>(p, k, s); break;
+      case 1: launch_post_reg<T, 1>(p, k, s); break;
+      case 2: launch_post_reg<T, 2>(p, k, s); break;
+      default: launch_post_reg<T, 3>(p, k, s); break;
     }
     return;
   }
@@ -1925,7 +1715,6 @@ static void cycle(const sg_gmg_plan* p, int k, bool zero_init, cudaStream_t s) {
   else
     SG_LAUNCH(k_gmg_residual_restrict<T><<<grid2d(C.W, C.H), block2d(), 0, s>>>(e, b, L.ld, m, ws_ptr<T>(p, C.off_b),
                                                                                  C.ld, cm));
-  int reps = (p->cycle == 1 && k + 1 < nl - 1) ? 2 : 1;
   for (int q = 0; q < reps; ++q) cycle<T>(p, k + 1, q == 0, s);
   SG_LAUNCH(k_gmg_prolong_add<T><<<grid2d(L.W, L.H), block2d(), 0, s>>>(ws_ptr<T>(p, C.off_e), C.ld, cm, e, L.ld, m));
   for (int sw = 0; sw < p->post; ++sw)
@@ -1951,7 +1740,7 @@ static void prologue(const sg_gmg_plan* p, cudaGraphConditionalHandle h, int use
   }
   // from a zero guess the fused fine level carries the residual from here on (b0 / r64), so
   // the FP64 rhs itself is not kept
-  TP* bkeep = (zero_guess && p->fused_ir && p->inner <= 1) ? nullptr : bf;
+  TP* bkeep = (zero_guess && (p->fused_ir || p->region_ir == 1) && p->inner <= 1) ? nullptr : bf;
   // the first cycle of such a solve forms r64 from the divergence itself (FirstCycle), so the
   // prologue does not write it
   SG_LAUNCH(k_gmg_rhs<TD, TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, st, m, bkeep, p->ld_bfine, part,
@@ -1998,8 +1787,24 @@ static void body(const sg_gmg_plan* p, cudaGraphConditionalHandle h, int use_han
   }
   dim3 g = grid_wide(L.W, L.H);
   const int inner = p->inner < 1 ? 1 : p->inner;
-  for (int q = 0; q < inner; ++q) cycle<TC>(p, 0, q == 0, s);
-  SG_LAUNCH(k_gmg_correct<TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, st, ws_ptr<TC>(p, L.off_e), L.ld));
+  if (p->region_ir && inner == 1) {
+    constexpr bool kCarried = !std::is_same<TP, float>::value;  // region_ir 1
+    TC* b_alt = kCarried ? ws_ptr<TC>(p, p->off_b2) : nullptr;
+    const int nl = (int)p->levels.size();
+    launch_pre_region<TC>(p, 0, true, b_alt, s);
+    const int reps = (p->cycle == 1 && 1 < nl - 1) ? 2 : 1;
+    for (int q = 0; q < reps; ++q) cycle<TC>(p, 1, q == 0, s);
+    if constexpr (kCarried) {
+      const dim3 gr = launch_post_region<TC, TP, 1>(p, 0, b_alt, s);
+      SG_LAUNCH(k_gmg_finalize_rel<<<1, 1024, 0, s>>>(part, (int)(gr.x * gr.y), st, h, use_handle, 1));
+      return;
+    } else {
+      launch_post_region<TC, TP, 2>(p, 0, nullptr, s);
+    }
+  } else {
+    for (int q = 0; q < inner; ++q) cycle<TC>(p, 0, q == 0, s);
+    SG_LAUNCH(k_gmg_correct<TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, st, ws_ptr<TC>(p, L.off_e), L.ld));
+  }
   SG_LAUNCH(k_gmg_fine_residual<TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, st, (const TP*)(p->ws + p->off_bfine),
                                                                    p->ld_bfine, m, ws_ptr<TC>(p, L.off_b), L.ld,
                                                                    (TP*)nullptr, part));
@@ -2044,9 +1849,9 @@ static int build_graph(sg_gmg_plan* p, int form) {
   SG_CUDA_TRY(cudaGraphConditionalHandleCreate(&h, g, 0, 0), "cudaGraphConditionalHandleCreate");
   struct FcGuard {
     const sg_gmg_plan* p;
-    ~FcGuard() { p->fc = FirstCycle{nullptr, 0, 0, 0, 0, 0.0, 0.0}; }
+    ~FcGuard() { p->fc = FirstCycle{nullptr, 0, 0, 0}; }
   } fc_guard{p};
-  p->fc = FirstCycle{nullptr, 0, sizeof(TD) == 8 ? 1 : 0, p->remove_mean ? 1 : 0, (form & 8) ? 1 : 0, 0.0, 0.0};
+  p->fc = FirstCycle{&state_ptr(p)->f, sizeof(TD) == 8 ? 1 : 0, p->remove_mean ? 1 : 0, (form & 8) ? 1 : 0};
   p->fields_staged = (form & 4) != 0;
   SG_CUDA_TRY(cudaStreamBeginCaptureToGraph(cs, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
               "begin capture");
@@ -2184,7 +1989,10 @@ int sg_gmg_plan_create(sg_gmg_plan** out, int64_t H, int64_t W, int mask_mode, c
     L.H = h;
     L.W = w;
     L.analytic = level_is_open(fl, fu, fv, h, w) ? 1 : 0;
-    if (!L.analytic) L.code = pack_codes(fl, fu, fv, h, w);
+    if (!L.analytic) {
+      L.code = pack_codes(fl, fu, fv, h, w);
+      L.simple = faces_follow_cells(L.code, h, w) ? 1 : 0;
+    }
     p->levels.push_back(L);
     if (std::max(h, w) <= coarsest || (int)p->levels.size() == kMaxLevels) break;
     int hc = (h + 1) / 2, wc = (w + 1) / 2;
@@ -2234,30 +2042,16 @@ int sg_gmg_plan_create(sg_gmg_plan** out, int64_t H, int64_t W, int mask_mode, c
       return fail(SG_ERR_ARG, "coarsest operator could not be factorised");
     }
   }
-  // tail: the largest suffix of levels that fits one block's shared memory: open boxes up
-  // to kOpenTailMaxSide cells a side (k_gmg_tail_open), otherwise up to kTailMaxSide
-  // (k_gmg_tail, codes from global memory); e and b of every level plus the scratch of
-  // the first one
+  for (size_t k = 0; k + 1 < p->levels.size(); ++k) add_transfer_codes(p->levels[k], p->levels[k + 1]);
+  // tail: the levels of at most kRgTailSide cells a side that run in one block
   size_t cyc = precision == SG_GMG_FP64 ? sizeof(double) : sizeof(float);
-  const int64_t budget = 220 * 1024;
   int nl = (int)p->levels.size();
-  auto generic_elems = [&](int start) {
-    int64_t acc = 0;
-    for (int k = start; k < nl; ++k) acc += ((2 * (int64_t)p->levels[k].H * p->levels[k].W + 3) & ~(int64_t)3);
-    return acc + (int64_t)p->levels[start].H * ((p->levels[start].W + 1) / 2);
-  };
-  p->tail_start = p->coarse_dct ? nl : nl - 1;  // no tail kernel above a cosine-transform solve
-  bool open_suffix = !p->coarse_dct;
+  p->tail_start = nl;  // no tail kernel above a cosine-transform solve
   for (int k = p->coarse_dct ? -1 : nl - 1; k >= 0; --k) {
     const Level& L = p->levels[k];
-    const bool open = open_suffix && L.analytic;
-    const int side = std::max(L.H, L.W);
-    const int64_t elems = open ? (int64_t)open_tail_layout(p->levels, k).total : generic_elems(k);
-    if (side > (open ? kOpenTailMaxSide : kTailMaxSide) || elems * (int64_t)cyc > budget) break;
-    open_suffix = open;
+    if (std::max(L.H, L.W) > kRgTailSide || (k < nl - 1 && !L.simple)) break;
     p->tail_start = k;
   }
-  p->tail_open = open_suffix ? 1 : 0;
   if (p->coarse_dct) {
     const Level& C = p->levels.back();
     p->tail_smem = 0;
@@ -2289,9 +2083,9 @@ int sg_gmg_plan_create(sg_gmg_plan** out, int64_t H, int64_t W, int mask_mode, c
                                       : (int64_t)(p->dct_fp64 ? coarse_dct_smem<double>(C.H, C.W)
                                                               : coarse_dct_smem<float>(C.H, C.W));
   } else {
-    p->tail_smem = (p->tail_open ? (int64_t)open_tail_layout(p->levels, p->tail_start).total
-                                 : generic_elems(p->tail_start)) *
-                   (int64_t)cyc;
+    const int cells = tail_cells(p->levels, p->tail_start, nullptr), nc = last.H * last.W;
+    p->tail_smem = (int64_t)(precision == SG_GMG_FP64 ? region_tail_smem<double>(cells, nc)
+                                                      : region_tail_smem<float>(cells, nc));
   }
   // workspace layout
   size_t fine = precision == SG_GMG_FP32 ? sizeof(float) : sizeof(double);
@@ -2303,6 +2097,9 @@ int sg_gmg_plan_create(sg_gmg_plan** out, int64_t H, int64_t W, int mask_mode, c
                           post_sweeps >= 1 && post_sweeps <= 3)
                              ? 1
                              : 0;
+    p->levels[k].region = (int)k < p->tail_start && L.simple && L.H >= 2 && L.W >= 2 && pre_sweeps >= 1 &&
+                          pre_sweeps <= 3 && post_sweeps >= 1 && post_sweeps <= 3 &&
+                          (small_tiles(L) || !p->levels[k].fused);
   }
   for (auto& L : p->levels) {
     L.ld = ((int64_t)L.W + 31) / 32 * 32;
@@ -2310,7 +2107,7 @@ int sg_gmg_plan_create(sg_gmg_plan** out, int64_t H, int64_t W, int mask_mode, c
     L.off_e = off;
     off = align256(off + n * (int64_t)cyc);
     L.off_e2 = off;
-    if (L.fused) off = align256(off + n * (int64_t)cyc);
+    if (L.fused || L.region) off = align256(off + n * (int64_t)cyc);
     L.off_b = off;
     off = align256(off + n * (int64_t)cyc);
     L.off_code = off;
@@ -2320,7 +2117,8 @@ int sg_gmg_plan_create(sg_gmg_plan** out, int64_t H, int64_t W, int mask_mode, c
   p->off_bfine = off;
   off = align256(off + p->ld_bfine * p->H * (int64_t)fine);
   p->fused_ir = (p->levels.size() >= 2 && p->tail_start >= 1 && p->levels[0].fused && !small_tiles(p->levels[0])) ? 1 : 0;
-  if (p->fused_ir) {
+  p->region_ir = p->levels.size() >= 2 && p->levels[0].region ? (precision == SG_GMG_FP32 ? 2 : 1) : 0;
+  if (p->fused_ir || p->region_ir == 1) {
     p->off_b2 = off;
     off = align256(off + p->levels[0].ld * p->H * (int64_t)cyc);
     if (precision == SG_GMG_MIXED) {
@@ -2341,6 +2139,10 @@ int sg_gmg_plan_create(sg_gmg_plan** out, int64_t H, int64_t W, int mask_mode, c
   if (p->fused_ir) {
     dim3 gf = precision == SG_GMG_FP64 ? post_final_grid<double>(p) : post_final_grid<float>(p);
     p->n_partial = std::max(p->n_partial, (int64_t)gf.x * gf.y);
+  }
+  if (p->region_ir == 1) {
+    const dim3 gr = region_grid(p->levels[0], region_halo(p->post, true));
+    p->n_partial = std::max(p->n_partial, (int64_t)gr.x * gr.y);
   }
   p->off_partial = off;
   off = align256(off + p->n_partial * 8);
@@ -2413,18 +2215,11 @@ int sg_gmg_bind(sg_gmg_plan* plan, void* workspace, void* stream) {
   SG_CUDA_TRY(cudaMemsetAsync(plan->ws + plan->off_state, 0, sizeof(GmgState), s), "sg_gmg_bind state");
   // host vectors must outlive the asynchronous copies
   SG_CUDA_TRY(cudaStreamSynchronize(s), "sg_gmg_bind sync");
-  int rc = plan->precision == SG_GMG_FP64 ? set_tiled_smem_limits<double>() : set_tiled_smem_limits<float>();
-  if (rc != SG_OK) return rc;
-  int smem = (int)plan->tail_smem;
-  if (plan->precision == SG_GMG_FP64) {
-    SG_CUDA_TRY(cudaFuncSetAttribute(k_gmg_tail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attr");
-    SG_CUDA_TRY(cudaFuncSetAttribute(k_gmg_tail_open<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                "smem attr");
-  } else {
-    SG_CUDA_TRY(cudaFuncSetAttribute(k_gmg_tail<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attr");
-    SG_CUDA_TRY(cudaFuncSetAttribute(k_gmg_tail_open<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                "smem attr");
-  }
+  const int smem = (int)plan->tail_smem;
+  SG_CUDA_TRY(plan->precision == SG_GMG_FP64
+                  ? cudaFuncSetAttribute(k_gmg_tail_region<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
+                  : cudaFuncSetAttribute(k_gmg_tail_region<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+              "smem attr");
   return SG_OK;
 }
 

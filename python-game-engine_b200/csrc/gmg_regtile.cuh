@@ -23,24 +23,24 @@
 constexpr int kRW = 64;  // tile columns: 32 lanes x 2
 
 // The first cycle of a solve from a zero guess, for the fused fine-level post kernel: p is 0
-// on entry (not read), and when div is set the carried float64 residual r64 starts as
+// on entry (not read), and when active the carried float64 residual r64 starts as
 // alpha div (- the fluid mean with sub_mean), formed here from the divergence instead of being
-// written by the prologue and read back. div: float32 (f64 = 0) or float64 values, row stride
-// ldd. active = 0: an ordinary cycle. div, ldd, alpha and mean are filled in on the device
-// from the solve state by the kernel that takes the struct.
+// written by the prologue and read back. f: the solve's fields, read where they are used (kept
+// in registers they made the fine level's kernel spill: 46.6 instead of 42.4 us at 2048^2 mixed).
+// f64: the divergence is float64. active = 0: an ordinary cycle.
 struct FirstCycle {
-  const void* div;
-  int64_t ldd;
+  const SolveFields* f;
   int f64;
   int sub_mean;
   int active;
-  double alpha, mean;
 };
-__device__ __forceinline__ double first_cycle_rhs(const FirstCycle& fc, int64_t o) {
-  const double d = fc.f64 ? ((const double*)fc.div)[o] : (double)((const float*)fc.div)[o];
-  double x = fc.alpha * d;
-  if (fc.sub_mean) x -= fc.mean;
-  return x;
+__device__ __forceinline__ double first_cycle_scale(const FirstCycle& fc, double d) {
+  const double x = __dmul_rn(fc.f->alpha, d);  // rounded as the prologue's rhs, not contracted into its use
+  return fc.sub_mean ? __dsub_rn(x, fc.f->bmean) : x;
+}
+__device__ __forceinline__ double first_cycle_rhs(const FirstCycle& fc, int64_t jj, int64_t ii) {
+  const int64_t o = jj * fc.f->ldd + ii;
+  return first_cycle_scale(fc, fc.f64 ? ((const double*)fc.f->div)[o] : (double)((const float*)fc.f->div)[o]);
 }
 
 template <typename T>
@@ -493,7 +493,8 @@ __device__ __forceinline__ void reg_post_final_body(RegXchg<TC, NWARP>& x, const
                                                     int H, int W, const TC* __restrict__ ec, int64_t ldc, int Hc,
                                                     int Wc, TC omega, TP* __restrict__ p, int64_t ldp,
                                                     TP* __restrict__ r64, int i0, int j0, double& sq,
-                                                    const FirstCycle& fc = FirstCycle{nullptr, 0, 0, 0, 0, 0.0, 0.0}) {
+                                                    const volatile int64_t* where = nullptr,
+                                                    const FirstCycle& fc = FirstCycle{nullptr, 0, 0, 0}) {
   using S = RegPre<TC, SW, RPT, NWARP>;
   // only mixed precision carries r64; the other instantiations compile without the first-cycle
   // path (which would cost them registers)
@@ -504,10 +505,12 @@ __device__ __forceinline__ void reg_post_final_body(RegXchg<TC, NWARP>& x, const
   const int r_lo = S::HALO - w * RPT, r_hi = S::HALO + S::TYO - w * RPT;
   // p and r64 are only needed after the sweeps: start bringing the owned rows into L2 now
   if (cols_owned && !first) {
+    const TP* pw = where ? reinterpret_cast<const TP*>(where[0]) : p;
+    const int64_t ldw = where ? where[1] : ldp;
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
       if (r < r_lo || r >= r_hi || (BOUNDED && j + r >= H)) continue;
-      prefetch_l2(p + (int64_t)(j + r) * ldp + i);
+      prefetch_l2(pw + (int64_t)(j + r) * ldw + i);
       if (r64) prefetch_l2(r64 + (int64_t)(j + r) * ld + i);
     }
   }
@@ -517,6 +520,10 @@ __device__ __forceinline__ void reg_post_final_body(RegXchg<TC, NWARP>& x, const
   exchange_rows<TC, RPT, NWARP>(x, (2 * SW) & 1, e, w, lane, above, below);
   using VC = typename Pair<TC>::V;
   using VP = typename Pair<TP>::V;
+  if (where) {  // the solve's pressure, from shared memory and only now
+    p = reinterpret_cast<TP*>(where[0]);
+    ldp = where[1];
+  }
 #pragma unroll
   for (int r = 0; r < RPT; ++r) {
     const TC l1 = shfl_up1(e[r][1]);
@@ -530,7 +537,7 @@ __device__ __forceinline__ void reg_post_final_body(RegXchg<TC, NWARP>& x, const
     if (first && r64) {  // the first cycle's residual, from the divergence
 #pragma unroll
       for (int q = 0; q < 2; ++q)
-        acc[q] = (!BOUNDED || i + q < W) ? (TP)first_cycle_rhs(fc, (int64_t)jj * fc.ldd + i + q) : (TP)0;
+        acc[q] = (!BOUNDED || i + q < W) ? (TP)first_cycle_rhs(fc, jj, i + q) : (TP)0;
     } else if (r64 && !BOUNDED) {
       const VP t = *reinterpret_cast<const VP*>(r64 + o);
       acc[0] = t.x;
@@ -604,6 +611,7 @@ __global__ void __launch_bounds__(32 * NWARP, MINB)
                          double* __restrict__ partial, FirstCycle fc) {
   using S = RegPre<TC, SW, RPT, NWARP>;
   __shared__ RegXchg<TC, NWARP> x;
+  __shared__ int64_t where[2];  // the pressure's address and row stride (null: the solve's own)
   const bool odd = st->cycles & 1;
   const TC* bsrc = odd ? b1 : b0;
   TC* bdst = odd ? b0 : b1;
@@ -612,20 +620,17 @@ __global__ void __launch_bounds__(32 * NWARP, MINB)
   const bool inside = i0 >= 0 && i0 + kRW <= W && j0 >= 0 && j0 + NWARP * RPT <= H;
   double sq = 0.0;
   fc.active = sizeof(TC) != sizeof(TP) && fc.active && st->cycles == 0;
-  fc.alpha = st->alpha;
-  fc.mean = st->bmean;
-  fc.div = st->div;
-  fc.ldd = st->ldd;
-  if (!p) {  // the solve's own pressure
-    p = (TP*)st->p;
-    ldp = st->ldp;
+  if (threadIdx.x == 0) {
+    where[0] = p ? reinterpret_cast<int64_t>(p) : reinterpret_cast<int64_t>(st->f.p);
+    where[1] = p ? ldp : st->f.ldp;
   }
+  __syncthreads();
   if (inside)
-    reg_post_final_body<TC, TP, SW, RPT, NWARP, false>(x, e_in, bsrc, bdst, ld, H, W, ec, ldc, Hc, Wc, omega, p, ldp,
-                                                      r64, i0, j0, sq, fc);
+    reg_post_final_body<TC, TP, SW, RPT, NWARP, false>(x, e_in, bsrc, bdst, ld, H, W, ec, ldc, Hc, Wc, omega,
+                                                      nullptr, 0, r64, i0, j0, sq, where, fc);
   else
-    reg_post_final_body<TC, TP, SW, RPT, NWARP, true>(x, e_in, bsrc, bdst, ld, H, W, ec, ldc, Hc, Wc, omega, p, ldp,
-                                                     r64, i0, j0, sq, fc);
+    reg_post_final_body<TC, TP, SW, RPT, NWARP, true>(x, e_in, bsrc, bdst, ld, H, W, ec, ldc, Hc, Wc, omega,
+                                                     nullptr, 0, r64, i0, j0, sq, where, fc);
   const double s = block_sum(sq);
   if (threadIdx.x == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = s;
 }

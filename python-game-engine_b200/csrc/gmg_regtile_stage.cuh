@@ -6,8 +6,12 @@
 // Here, on tiles that lie inside the grid, threads 0 .. 2 TYO - 1 each issue one bulk copy of
 // an owned row of p or r64 straight into shared memory when the block starts, so the transfer
 // runs under the prolongation and the sweeps without registers or issue slots, and the final
-// phase reads shared memory. Edge tiles take the unstaged body. The arithmetic is that of
-// k_gmg_post_final_reg, so both kernels write the same bits.
+// phase reads shared memory. The new p and r64 go back into their slots and from there to
+// global memory by bulk copies, one row each: the pressure's address then is not held through
+// the sweeps (with plain stores the kernel spilled at its 64 registers: 2048^2 mixed 43.6, float64
+// 56.5 us; so 42.4 and 54.7; 41.3 and 51.4 with the address in the launch, where every other
+// tensor costs a new graph, 140 us). Edge tiles take the unstaged body. The arithmetic is that
+// of k_gmg_post_final_reg, so both kernels write the same bits.
 #pragma once
 
 template <typename TP, int TXO, int TYO>
@@ -24,7 +28,7 @@ __device__ __forceinline__ void reg_post_final_body_staged(RegXchg<TC, NWARP>& x
                                                            const TC* __restrict__ e_in, const TC* __restrict__ bsrc,
                                                            TC* __restrict__ bdst, int64_t ld, int H, int W,
                                                            const TC* __restrict__ ec, int64_t ldc, int Hc, int Wc,
-                                                           TC omega, TP* __restrict__ p, int64_t ldp,
+                                                           TC omega, const volatile int64_t* __restrict__ where,
                                                            TP* __restrict__ r64, int i0, int j0, double& sq, bool& ok,
                                                            const FirstCycle& fc, bool staged_any) {
   using S = RegPre<TC, SW, RPT, NWARP>;
@@ -59,9 +63,7 @@ __device__ __forceinline__ void reg_post_final_body_staged(RegXchg<TC, NWARP>& x
         const int64_t so = (int64_t)k * S::TXO + cs + q;
         const double d = fc.f64 ? reinterpret_cast<const double*>(sp.p)[so]
                                 : (double)reinterpret_cast<const float*>(sp.p)[so];
-        double x2 = fc.alpha * d;
-        if (fc.sub_mean) x2 -= fc.mean;
-        acc[q] = (TP)x2;
+        acc[q] = (TP)first_cycle_scale(fc, d);
       }
     } else if (r64) {
       const VP t = *reinterpret_cast<const VP*>(sp.r + k * S::TXO + cs);
@@ -88,22 +90,23 @@ __device__ __forceinline__ void reg_post_final_body_staged(RegXchg<TC, NWARP>& x
         acc[q] += down - xv[q];
       }
     }
-    VP pv;
-    if (sizeof(TC) != sizeof(TP) && fc.active) {  // p is 0 on a solve's first cycle from a zero guess
-      pv.x = (TP)0;
-      pv.y = (TP)0;
+    // p and r64 go back through their staged slots, and from there by bulk copies; on a first
+    // cycle p is 0 and its slots hold the divergence that other threads may still read
+    VP pn, t;
+    pn.x = xv[0];
+    pn.y = xv[1];
+    t.x = acc[0];
+    t.y = acc[1];
+    if (sizeof(TC) != sizeof(TP) && fc.active) {
+      *reinterpret_cast<VP*>(reinterpret_cast<TP*>(where[0]) + (int64_t)jj * where[1] + i) = pn;
+      if (r64) *reinterpret_cast<VP*>(r64 + o) = t;
     } else {
-      pv = *reinterpret_cast<const VP*>(sp.p + k * S::TXO + cs);
-    }
-    VP pn;
-    pn.x = pv.x + xv[0];
-    pn.y = pv.y + xv[1];
-    *reinterpret_cast<VP*>(p + (int64_t)jj * ldp + i) = pn;
-    if (r64) {
-      VP t;
-      t.x = acc[0];
-      t.y = acc[1];
-      *reinterpret_cast<VP*>(r64 + o) = t;
+      VP* ps = reinterpret_cast<VP*>(sp.p + k * S::TXO + cs);
+      const VP pv = *ps;
+      pn.x = pv.x + xv[0];
+      pn.y = pv.y + xv[1];
+      *ps = pn;
+      if (r64) *reinterpret_cast<VP*>(sp.r + k * S::TXO + cs) = t;
     }
     VC c;
     c.x = (TC)acc[0];
@@ -129,6 +132,7 @@ __global__ void __launch_bounds__(32 * NWARP, MINB)
   static_assert(2 * S::TYO <= 32 * NWARP, "one thread per staged row");
   __shared__ RegXchg<TC, NWARP> x;
   __shared__ __align__(16) StagedPR<TP, S::TXO, S::TYO> sp;
+  __shared__ int64_t where[2];  // the pressure's address and row stride
   const bool odd = st->cycles & 1;
   const TC* bsrc = odd ? b1 : b0;
   TC* bdst = odd ? b0 : b1;
@@ -138,25 +142,21 @@ __global__ void __launch_bounds__(32 * NWARP, MINB)
   double sq = 0.0;
   // the first cycle of a solve from a zero guess (mixed precision only: the others carry no r64)
   fc.active = sizeof(TC) != sizeof(TP) && fc.active && st->cycles == 0;
-  fc.alpha = st->alpha;
-  fc.mean = st->bmean;
-  fc.div = st->div;
-  fc.ldd = st->ldd;
-  if (!p) {  // the solve's own pressure
-    p = (TP*)st->p;
-    ldp = st->ldp;
+  const TP* pw = p ? p : (const TP*)st->f.p;  // for the copies below only
+  const int64_t ldw = p ? ldp : st->f.ldp;
+  if (threadIdx.x == 0) {
+    where[0] = reinterpret_cast<int64_t>(pw);
+    where[1] = ldw;
+    mbar_init(&sp.bar, 1);
+    mbar_fence_init();
   }
+  __syncthreads();
   if (inside) {
     const int t = threadIdx.x;
     // rows to stage: p and r64 (or p alone); on the first cycle only the divergence rows that
     // form r64 (p is 0), or nothing without r64
     const int nrow = fc.active ? (r64 ? S::TYO : 0) : (r64 ? 2 * S::TYO : S::TYO);
     if (nrow > 0) {
-      if (t == 0) {
-        mbar_init(&sp.bar, 1);
-        mbar_fence_init();
-      }
-      __syncthreads();
       constexpr uint32_t kRowBytes = S::TXO * sizeof(TP);
       const uint32_t div_bytes = (uint32_t)S::TXO * (fc.f64 ? 8u : 4u);
       if (t == 0) mbar_arrive_expect_tx(&sp.bar, (uint32_t)nrow * (fc.active ? div_bytes : kRowBytes));
@@ -165,21 +165,34 @@ __global__ void __launch_bounds__(32 * NWARP, MINB)
         const int64_t jj = j0 + S::HALO + k, ii = i0 + S::HALO;
         if (fc.active)
           bulk_g2s(reinterpret_cast<unsigned char*>(sp.p) + (size_t)k * div_bytes,
-                   reinterpret_cast<const unsigned char*>(fc.div) + (jj * fc.ldd + ii) * (fc.f64 ? 8 : 4), div_bytes,
-                   &sp.bar);
+                   reinterpret_cast<const unsigned char*>(st->f.div) + (jj * st->f.ldd + ii) * (fc.f64 ? 8 : 4),
+                   div_bytes, &sp.bar);
         else if (t < S::TYO)
-          bulk_g2s(sp.p + k * S::TXO, p + jj * ldp + ii, kRowBytes, &sp.bar);
+          bulk_g2s(sp.p + k * S::TXO, pw + jj * ldw + ii, kRowBytes, &sp.bar);
         else
           bulk_g2s(sp.r + k * S::TXO, r64 + jj * ld + ii, kRowBytes, &sp.bar);
       }
     }
     bool ok = true;
-    reg_post_final_body_staged<TC, TP, SW, RPT, NWARP>(x, sp, e_in, bsrc, bdst, ld, H, W, ec, ldc, Hc, Wc, omega, p,
-                                                       ldp, r64, i0, j0, sq, ok, fc, nrow > 0);
+    reg_post_final_body_staged<TC, TP, SW, RPT, NWARP>(x, sp, e_in, bsrc, bdst, ld, H, W, ec, ldc, Hc, Wc, omega,
+                                                       where, r64, i0, j0, sq, ok, fc, nrow > 0);
     if (!ok) atomicExch(&st->dev_error, kDevErrBulkWait);
+    if (!fc.active) {
+      bulk_fence_shared();
+      __syncthreads();
+      if (t < nrow) {
+        const int k = t < S::TYO ? t : t - S::TYO;
+        const int64_t jj = j0 + S::HALO + k, ii = i0 + S::HALO;
+        if (t < S::TYO)
+          bulk_s2g(reinterpret_cast<TP*>(where[0]) + jj * where[1] + ii, sp.p + k * S::TXO, S::TXO * sizeof(TP));
+        else
+          bulk_s2g(r64 + jj * ld + ii, sp.r + k * S::TXO, S::TXO * sizeof(TP));
+        bulk_commit_wait_read();
+      }
+    }
   } else {
-    reg_post_final_body<TC, TP, SW, RPT, NWARP, true>(x, e_in, bsrc, bdst, ld, H, W, ec, ldc, Hc, Wc, omega, p, ldp,
-                                                     r64, i0, j0, sq, fc);
+    reg_post_final_body<TC, TP, SW, RPT, NWARP, true>(x, e_in, bsrc, bdst, ld, H, W, ec, ldc, Hc, Wc, omega, nullptr, 0,
+                                                      r64, i0, j0, sq, where, fc);
   }
   const double s = block_sum(sq);
   if (threadIdx.x == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = s;

@@ -248,23 +248,6 @@ __device__ __forceinline__ void pre_body(const SplitTile<T>& t, const T* __restr
   tile_store<T, INTERIOR, S::HALO, TX, TY>(t, e_out, ld);
 }
 
-// pre: SW sweeps from e_in (NULL: zero initial guess) + residual + full weighting into
-// bc (coarse tile TX/2 x TY/2); the smoothed tile goes to e_out.
-template <typename T, int SW, int TX, int TY>
-__global__ void __launch_bounds__(1024) k_gmg_pre_tiled(const T* __restrict__ e_in, T* __restrict__ e_out,
-                                                             const T* __restrict__ b, int64_t ld, int H, int W,
-                                                             T* __restrict__ bc, int64_t ldc, int Hc, int Wc, T omega) {
-  using S = PreShape<SW, TX, TY>;
-  extern __shared__ __align__(16) unsigned char smem[];
-  SplitTile<T> t = make_tile<T, TX, TY>(smem, S::HALO, S::EXh, S::EY, H, W, blockIdx.x, blockIdx.y);
-  T* X = reinterpret_cast<T*>(smem) + 4 * S::EY * S::EXh;
-  const bool interior = t.i0 >= 0 && t.i0 + S::EX <= W && t.j0 >= 0 && t.j0 + S::EY <= H;
-  if (interior)
-    pre_body<T, SW, TX, TY, true>(t, e_in, e_out, b, ld, bc, ldc, Hc, Wc, omega, X, blockIdx.x, blockIdx.y);
-  else
-    pre_body<T, SW, TX, TY, false>(t, e_in, e_out, b, ld, bc, ldc, Hc, Wc, omega, X, blockIdx.x, blockIdx.y);
-}
-
 template <typename T, int SW, int TX, int TY, bool INTERIOR>
 __device__ __forceinline__ void post_body(const SplitTile<T>& t, const T* __restrict__ e_in, T* __restrict__ e_out,
                                           const T* __restrict__ b, int64_t ld, const T* __restrict__ ec, int64_t ldc,
@@ -298,20 +281,4 @@ __device__ __forceinline__ void post_body(const SplitTile<T>& t, const T* __rest
   __syncthreads();
   relax_all<T, INTERIOR, S::HALO, S::EXh, TX, TY, 0, 2 * SW>(t, omega);
   tile_store<T, INTERIOR, S::HALO, TX, TY>(t, e_out, ld);
-}
-
-// post: e_out = smoothed (e_in + P ec).
-template <typename T, int SW, int TX, int TY>
-__global__ void __launch_bounds__(1024) k_gmg_post_tiled(const T* __restrict__ e_in, T* __restrict__ e_out,
-                                                              const T* __restrict__ b, int64_t ld, int H, int W,
-                                                              const T* __restrict__ ec, int64_t ldc, int Hc, int Wc,
-                                                              T omega) {
-  using S = PostShape<SW, TX, TY>;
-  extern __shared__ __align__(16) unsigned char smem[];
-  SplitTile<T> t = make_tile<T, TX, TY>(smem, S::HALO, S::EXh, S::EY, H, W, blockIdx.x, blockIdx.y);
-  const bool interior = t.i0 >= 0 && t.i0 + S::EX <= W && t.j0 >= 0 && t.j0 + S::EY <= H;
-  if (interior)
-    post_body<T, SW, TX, TY, true>(t, e_in, e_out, b, ld, ec, ldc, Hc, Wc, omega);
-  else
-    post_body<T, SW, TX, TY, false>(t, e_in, e_out, b, ld, ec, ldc, Hc, Wc, omega);
 }

@@ -2,6 +2,17 @@
 // batch.cu (included inside namespace sg).
 #pragma once
 
+// The fields and scale of a solve, in device memory (GmgState): the kernels of a solve's graph
+// take them from here, so that one instantiated graph serves every pressure and divergence.
+struct SolveFields {
+  void* p;
+  int64_t ldp;
+  const void* div;
+  int64_t ldd;
+  double alpha;
+  double bmean;  // mean of alpha div over the fluid cells (when the plan removes it)
+};
+
 // 1-D prolongation weight of fine index i onto coarse index I (grid of n coarse cells).
 __device__ __forceinline__ float w1(int i, int I, int n) {
   int h = i >> 1;

@@ -309,6 +309,7 @@ int sg_rbsor_mixed_solve(int64_t H, int64_t W, void* p, int64_t ld_p, const void
 
 /* All `iterations` sweeps of sg_jacobi_solve (sor = 0) or sg_rbsor_solve (sor = 1) in one
  * cooperative launch with the iterate held on the chip: the same iterates, bit for bit.
+ * from_zero (iterations >= 1): p is 0 and not read.
  * workspace (16-byte aligned, sg_sweeps_workspace_bytes; cleared by the call): the cells that
  * neighbouring blocks trade. sg_sweeps_workspace_bytes is 0, and the solve returns
  * SG_ERR_CAPACITY, for grids that do not fit the current device at once. p and div may not
@@ -317,7 +318,7 @@ int64_t sg_sweeps_workspace_bytes(int dtype, int64_t H, int64_t W);
 int sg_sweeps_solve(int dtype, int sor, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div, int64_t ld_div,
                     int mask_mode, const uint8_t* face_mask_u, int64_t ld_fmu, const uint8_t* face_mask_v,
                     int64_t ld_fmv, double alpha, double reciprocal_beta, double omega, int iterations,
-                    void* workspace, int64_t workspace_bytes, void* stream);
+                    int from_zero, void* workspace, int64_t workspace_bytes, void* stream);
 
 /* backends/numba/solvers/gauss_seidel.py:8-48 (lexicographic order), run as anti-diagonal
  * wavefronts in one thread block with the sweeps following one another two diagonals apart
@@ -347,7 +348,8 @@ int sg_mg_prolong(int dtype, int64_t Hc, int64_t Wc, const void* coarse, int64_t
  * coarsest_sweeps on the last level, red-black SOR (sor = 1) or Jacobi, in two launches per
  * level and cycle; every value equals the separate kernels'. Level k: extents, mask planes
  * (H x (W + 1) and (H + 1) x W bytes, contiguous), their cell codes (sg_mg_codes, sg_mg_codes_bytes
- * bytes, made once per mask), alpha(2^k h) and the SOR factor. Workspace
+ * bytes, made once per mask), alpha(2^k h) and the SOR factor. from_zero (cycles >= 1): p is 0
+ * and not read. Workspace
  * 256-byte aligned; sg_mg_vcycles_workspace_bytes is 0, and the call returns SG_ERR_CAPACITY,
  * for more than 4 SOR or 8 Jacobi sweeps a side or a coarsest level too large for the chip. */
 typedef struct {
@@ -363,7 +365,7 @@ int sg_mg_codes(int64_t H, int64_t W, const uint8_t* face_mask_u, const uint8_t*
 int64_t sg_mg_vcycles_workspace_bytes(int dtype, int n_levels, const sg_mg_level* levels, int sor, int sweeps);
 int sg_mg_vcycles(int dtype, int n_levels, const sg_mg_level* levels, void* p, int64_t ld_p, const void* div,
                   int64_t ld_div, double reciprocal_beta, int sor, int cycles, int sweeps, int coarsest_sweeps,
-                  void* workspace, int64_t workspace_bytes, void* stream);
+                  int from_zero, void* workspace, int64_t workspace_bytes, void* stream);
 int sg_mg_coarsen_solid(int64_t H, int64_t W, const uint8_t* solid, int64_t ld_s, uint8_t* coarse,
                         int64_t ld_c, void* stream);
 
@@ -589,6 +591,45 @@ int sg_batch_autotune(sg_batch* batch, int steps, void* scratch, int64_t scratch
 int64_t sg_field_stats_workspace_bytes(void);
 int sg_field_stats(int dtype, int64_t H, int64_t W, const void* field, int64_t ld, void* workspace, double* out,
                    void* stream);
+
+/* The operators of one substep (common/simulation.py:186-265) around its pressure solve, each
+ * through its entry above. Every member is 8 bytes. Pointers with their row strides; temperature
+ * NULL: no temperature chain. transport: emitters (0 density, 1 temperature, 2 u, 3 v), plumes,
+ * forces on v, velocity into u_temp / v_temp, density into density_temp, temperature into
+ * temperature_temp (cooled), divergence of the advected velocity. project: the projected
+ * velocity from u_temp / v_temp into u / v, its divergence and the residual of pressure.
+ * advect_f32 / operator_f32: float32 arithmetic for float32 fields. */
+typedef struct {
+  int64_t field;
+  double value, x, y, radius;
+  int64_t approach;
+} sg_emit;
+typedef struct {
+  int64_t dtype, H, W;
+  void* density; int64_t ld_density;
+  void* density_temp; int64_t ld_density_temp;
+  void* u; int64_t ld_u;
+  void* u_temp; int64_t ld_u_temp;
+  void* v; int64_t ld_v;
+  void* v_temp; int64_t ld_v_temp;
+  void* pressure; int64_t ld_pressure;
+  void* divergence; int64_t ld_divergence;
+  void* residual; int64_t ld_residual;
+  void* temperature; int64_t ld_temperature;
+  void* temperature_temp; int64_t ld_temperature_temp;
+  int64_t mask_mode;
+  const uint8_t* face_mask_u; int64_t ld_fmu;
+  const uint8_t* face_mask_v; int64_t ld_fmv;
+  const uint8_t* is_fluid; int64_t ld_fluid;
+  int64_t solid_mode;
+  const uint8_t* solid; int64_t ld_solid;
+  int64_t advect_f32, operator_f32;
+  int64_t n_plumes; const double* plumes; uint64_t seed; int64_t step;
+  int64_t n_emits; const sg_emit* emits;
+  double dt, cell_size, gravity, buoyancy, ambient, cooling_rate, dissipation, fluid_density, alpha, reciprocal_beta;
+} sg_substep;
+int sg_substep_transport(const sg_substep* substep, void* stream);
+int sg_substep_project(const sg_substep* substep, void* stream);
 
 #ifdef __cplusplus
 }

@@ -50,8 +50,10 @@ SIGNATURES = {
     "sg_jacobi_solve": [I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, I, P, P],
     "sg_jacobi_solve_noalloc": [I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, I, P],
     "sg_rbsor_solve": [I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, D, I, P],
+    "sg_substep_transport": [P, P],
+    "sg_substep_project": [P, P],
     "sg_sweeps_workspace_bytes": [I, I64, I64],
-    "sg_sweeps_solve": [I, I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, D, I, P, I64, P],
+    "sg_sweeps_solve": [I, I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, D, I, I, P, I64, P],
     "sg_gauss_seidel_solve": [I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, I, P],
     "sg_rbsor_split_workspace_bytes": [I, I64, I64],
     "sg_rbsor_split_pack": [I, I64, I64, P, I64, I, P, I64, P],
@@ -69,7 +71,7 @@ SIGNATURES = {
     "sg_mg_codes_bytes": [I64, I64],
     "sg_mg_codes": [I64, I64, P, P, P, P],
     "sg_mg_vcycles_workspace_bytes": [I, I, P, I, I],
-    "sg_mg_vcycles": [I, I, P, P, I64, P, I64, D, I, I, I, I, P, I64, P],
+    "sg_mg_vcycles": [I, I, P, P, I64, P, I64, D, I, I, I, I, I, P, I64, P],
     "sg_gmg_plan_create": [ctypes.POINTER(P), I64, I64, I, P, P, P, I, D, I, I, I, I],
     "sg_gmg_plan_destroy": [P],
     "sg_gmg_workspace_bytes": [P],

@@ -290,11 +290,11 @@ int64_t sg_sweeps_workspace_bytes(int dtype, int64_t H, int64_t W) {
 
 int sg_sweeps_solve(int dtype, int sor, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div, int64_t ld_div,
                     int mask_mode, const uint8_t* fmu, int64_t ld_fmu, const uint8_t* fmv, int64_t ld_fmv,
-                    double alpha, double reciprocal_beta, double omega, int iterations, void* workspace,
-                    int64_t workspace_bytes, void* stream) {
+                    double alpha, double reciprocal_beta, double omega, int iterations, int from_zero,
+                    void* workspace, int64_t workspace_bytes, void* stream) {
   SG_REQUIRE(H >= 1 && W >= 1 && H <= (1 << 28) && W <= (1 << 28), "bad grid %lld x %lld", (long long)H, (long long)W);
   SG_REQUIRE(p && div && ld_p >= W && ld_div >= W, "bad fields");
-  SG_REQUIRE(iterations >= 0, "iterations must be >= 0");
+  SG_REQUIRE(iterations >= (from_zero ? 1 : 0), "iterations must be >= 0, and >= 1 from zero");
   SG_REQUIRE(mask_mode == SG_MASK_OPEN || mask_mode == SG_MASK_RING || (mask_mode == SG_MASK_PLANES && fmu && fmv),
              "bad mask mode %d or missing mask planes", mask_mode);
   const int64_t need = sg_sweeps_workspace_bytes(dtype, H, W);
@@ -310,7 +310,7 @@ int sg_sweeps_solve(int dtype, int sor, int64_t H, int64_t W, void* p, int64_t l
   if (e != cudaSuccess) return fail(SG_ERR_CUDA, "sg_sweeps_solve: %s", cudaGetErrorString(e));
   SG_DISPATCH(dtype, {
     return resident_sweeps<T>(sor != 0, 0, (int)H, (int)W, (T*)p, nullptr, ld_p, (const T*)div, nullptr, ld_div, m,
-                              alpha, reciprocal_beta, omega, iterations, false, workspace, 1, s);
+                              alpha, reciprocal_beta, omega, iterations, from_zero != 0, workspace, 1, s);
   });
 }
 

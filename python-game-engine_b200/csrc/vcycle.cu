@@ -365,11 +365,11 @@ static int64_t code_pitch(int64_t W) { return (W + 1) & ~(int64_t)1; }
 
 template <typename T, bool SOR>
 static int mg_vcycles(int n, const sg_mg_level* lv, const MgPlan& P, T* p, int64_t ldp, const T* div, int64_t ldd,
-                      double rb, int cycles, int sweeps, int coarsest, char* ws, cudaStream_t s) {
+                      double rb, int cycles, int sweeps, int coarsest, bool from_zero, char* ws, cudaStream_t s) {
   const int half = SOR ? 2 * sweeps : sweeps;
   const double beta = 1.0 / rb;
   auto at = [&](int64_t o) { return (T*)(ws + o); };
-  auto level = [&](int k, bool down) {
+  auto level = [&](int k, bool down, bool zero) {
     MgLevelArgs<T> a{};
     a.H = (int)lv[k].H;
     a.W = (int)lv[k].W;
@@ -385,7 +385,7 @@ static int mg_vcycles(int n, const sg_mg_level* lv, const MgPlan& P, T* p, int64
     a.b = k == 0 ? div : at(P.rhs[k]);
     a.ldb = k == 0 ? ldd : a.W;
     if (down) {  // pa (level 0) or zero -> pb
-      a.pin = k == 0 ? p : nullptr;
+      a.pin = k == 0 && !zero ? p : nullptr;
       a.ldin = ldp;
       a.pout = at(P.pb[k]);
       a.ldout = a.W;
@@ -421,7 +421,6 @@ static int mg_vcycles(int n, const sg_mg_level* lv, const MgPlan& P, T* p, int64
       t.alpha[q] = L.alpha;
       t.omega[q] = L.omega;
     }
-    t.pin = P.tail == 0 ? p : nullptr;
     t.ldin = ldp;
     t.pout = P.tail == 0 ? p : at(P.pa[P.tail]);
     t.ldout = P.tail == 0 ? ldp : t.W[0];
@@ -441,22 +440,26 @@ static int mg_vcycles(int n, const sg_mg_level* lv, const MgPlan& P, T* p, int64
   }
   uint32_t tag = 1;
   for (int c = 0; c < cycles; ++c) {
-    for (int k = 0; k < P.tail && k < n - 1; ++k) level(k, true);
+    const bool zero = from_zero && c == 0;  // level 0 starts from p = 0 without reading it
+    for (int k = 0; k < P.tail && k < n - 1; ++k) level(k, true, zero);
     if (P.tail < n) {
+      t.pin = P.tail == 0 && !zero ? p : nullptr;
       SG_LAUNCH((k_mg_tail<T, SOR><<<1, kResThreads, smem, s>>>(t)));
     } else {
       const sg_mg_level& L = lv[n - 1];
       T* pc = n == 1 ? p : at(P.pa[n - 1]);
-      if (coarsest == 0 && n > 1) {
-        cudaError_t e = cudaMemsetAsync(pc, 0, sizeof(T) * (size_t)(L.H * L.W), s);
+      const bool fresh = n > 1 || zero;
+      if (coarsest == 0 && fresh) {
+        cudaError_t e = cudaMemset2DAsync(pc, sizeof(T) * (size_t)(n == 1 ? ldp : L.W), 0, sizeof(T) * (size_t)L.W,
+                                          (size_t)L.H, s);
         if (e != cudaSuccess) return fail(SG_ERR_CUDA, "memset: %s", cudaGetErrorString(e));
       }
       SG_CHECK(resident_sweeps<T>(SOR, 0, (int)L.H, (int)L.W, pc, nullptr, n == 1 ? ldp : L.W,
                                   n == 1 ? div : at(P.rhs[n - 1]), nullptr, n == 1 ? ldd : L.W, level_masks(L),
-                                  L.alpha, rb, L.omega, coarsest, n > 1, ws + P.xchg, tag, s));
+                                  L.alpha, rb, L.omega, coarsest, fresh, ws + P.xchg, tag, s));
       tag += (uint32_t)resident_trades(SOR, coarsest);
     }
-    for (int k = std::min(P.tail, n - 1) - 1; k >= 0; --k) level(k, false);
+    for (int k = std::min(P.tail, n - 1) - 1; k >= 0; --k) level(k, false, false);
   }
   return check_launch("sg_mg_vcycles");
 }
@@ -485,9 +488,10 @@ int64_t sg_mg_vcycles_workspace_bytes(int dtype, int n_levels, const sg_mg_level
 
 int sg_mg_vcycles(int dtype, int n_levels, const sg_mg_level* levels, void* p, int64_t ld_p, const void* div,
                   int64_t ld_div, double reciprocal_beta, int sor, int cycles, int sweeps, int coarsest_sweeps,
-                  void* workspace, int64_t workspace_bytes, void* stream) {
+                  int from_zero, void* workspace, int64_t workspace_bytes, void* stream) {
   SG_REQUIRE(levels && p && div && n_levels >= 1, "null level table or fields");
-  SG_REQUIRE(cycles >= 0 && sweeps >= 0 && coarsest_sweeps >= 0, "counts must be >= 0");
+  SG_REQUIRE(cycles >= (from_zero ? 1 : 0) && sweeps >= 0 && coarsest_sweeps >= 0,
+             "counts must be >= 0, and cycles >= 1 from zero");
   SG_REQUIRE(reciprocal_beta != 0.0, "reciprocal_beta must be non-zero");
   SG_REQUIRE(dtype == SG_F32 || dtype == SG_F64, "unsupported dtype code %d", dtype);
   MgPlan P;
@@ -502,9 +506,9 @@ int sg_mg_vcycles(int dtype, int n_levels, const sg_mg_level* levels, void* p, i
   SG_DISPATCH(dtype, {
     if (sor)
       return (mg_vcycles<T, true>(n_levels, levels, P, (T*)p, ld_p, (const T*)div, ld_div, reciprocal_beta, cycles,
-                                  sweeps, coarsest_sweeps, (char*)workspace, as_stream(stream)));
+                                  sweeps, coarsest_sweeps, from_zero != 0, (char*)workspace, as_stream(stream)));
     return (mg_vcycles<T, false>(n_levels, levels, P, (T*)p, ld_p, (const T*)div, ld_div, reciprocal_beta, cycles,
-                                 sweeps, coarsest_sweeps, (char*)workspace, as_stream(stream)));
+                                 sweeps, coarsest_sweeps, from_zero != 0, (char*)workspace, as_stream(stream)));
   });
 }
 

@@ -294,17 +294,22 @@ def emit_scalar(field, value, dt, pos_x, pos_y, radius, approach):
            float(radius), APPROACH_CODES[approach], L.stream_ptr())
 
 
+def plume_rows(sources):
+    """A host table of plume rows as a contiguous (n, 6) float64 array."""
+    if isinstance(sources, torch.Tensor):
+        if sources.is_cuda:
+            raise ValueError("sources must be a host table (it is passed in the launch parameters)")
+        sources = sources.numpy()
+    return np.ascontiguousarray(np.asarray(sources, dtype=np.float64).reshape(-1, 6))
+
+
 def plume_sources(density, velocity_u, velocity_v, sources, seed, step):
     """Overwriting disc sources (benchmark scenes). ``sources``: host table of shape (n, 6)
     (numpy array, CPU tensor or nested list) of (cx, cy, r, density, v, noise_amp) rows;
     it travels in the kernel's launch parameters."""
     dt_code = _same_dtype(density, velocity_u, velocity_v)
     H, W = density.shape
-    if isinstance(sources, torch.Tensor):
-        if sources.is_cuda:
-            raise ValueError("sources must be a host table (it is passed in the launch parameters)")
-        sources = sources.numpy()
-    src = np.ascontiguousarray(np.asarray(sources, dtype=np.float64).reshape(-1, 6))
+    src = plume_rows(sources)
     d, ldd = L.field(density, "density")
     u, ldu = L.field(velocity_u, "velocity_u")
     v, ldv = L.field(velocity_v, "velocity_v")

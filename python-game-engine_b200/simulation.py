@@ -27,6 +27,8 @@ reference computes exact zeros for it.
 from __future__ import annotations
 
 import contextlib
+import ctypes
+import struct
 
 import numpy as np
 import torch
@@ -35,7 +37,7 @@ from . import _lib as L
 from . import operators as ops
 from .operators import OPEN_BOX, RING_BOX
 from .params import DEFAULT_SOLVER_PARAMS
-from .solvers import calculate_alpha, calculate_reciprocal_beta, solve_pressure
+from .solvers import calculate_alpha, calculate_reciprocal_beta, solve_pressure, starts_from_zero
 
 
 class _NullTiming:
@@ -312,6 +314,12 @@ class SmokeSimulation2D:
         prof.tick()
         if self._mask_dirty:
             self._rebuild_masks()
+        if type(prof) is NullProfileSession and self._steps_plainly():
+            packed = self._pack_substep(dt)
+            if packed is not None:
+                self._native_substep(packed)
+                self.step_index += 1
+                return
         scope = prof.timing.scope
         with scope("simulation.substep"):
             with scope("simulation.emitters"):
@@ -347,15 +355,114 @@ class SmokeSimulation2D:
             prof.metrics.process()
         self.step_index += 1
 
+    # The operators around the solve in two native calls (csrc/substep.cu) instead of one Python
+    # call each: nothing measures them, nothing replaces them, and every field is laid out as
+    # this class makes it. Anything else takes the calls one by one, which also report errors.
+    def _steps_plainly(self):
+        return (type(self) is SmokeSimulation2D and self.__dict__.keys().isdisjoint(_STEP_METHODS)
+                and all(SmokeSimulation2D.__dict__[n] is f for n, f in _STEP_METHODS.items())
+                and all(getattr(ops, n) is f for n, f in _STEP_OPERATORS.items()))
+
+    def _pack_substep(self, dt):
+        """The arguments of sg_substep_* (read afresh from the fields), or None."""
+        H, W = self.height, self.width
+        dtype = self.density.dtype
+        code = 0 if dtype == torch.float32 else (1 if dtype == torch.float64 else None)
+        arith = {"reference": 0, "float32": 1}
+        adv, opr = arith.get(self.advection_arithmetic), arith.get(self.operator_arithmetic)
+        if code is None or H < 2 or W < 2 or adv is None or opr is None or (code == 1 and (adv or opr)):
+            return None
+        temp_on = self._temperature_needed()
+        cell, face_u, face_v = (H, W), (H, W + 1), (H + 1, W)
+        where = [code, H, W]
+        todo = [(self.density, cell), (self.density_temp, cell), (self.velocity_u, face_u),
+                (self.velocity_u_temp, face_u), (self.velocity_v, face_v), (self.velocity_v_temp, face_v),
+                (self.pressure, cell), (self.divergence, cell), (self.pressure_residual, cell)]
+        if temp_on:
+            todo += [(self._temperature, cell), (self.temperature_temp, cell)]
+        for t, shape in todo:
+            if not isinstance(t, torch.Tensor) or t.dtype != dtype or not t.is_cuda or t.shape != shape:
+                return None
+            ld, one = t.stride()
+            if one != 1 or ld < shape[1]:
+                return None
+            where += (t.data_ptr(), ld)
+        if not temp_on:
+            where += (0, 0, 0, 0)
+        fmu, fmv, fl = self._kmasks
+        if fmu is OPEN_BOX and fmv is OPEN_BOX and fl is OPEN_BOX:
+            where += (L.SG_MASK_OPEN, 0, 0, 0, 0, 0, 0)
+        elif any(isinstance(m, ops.AnalyticMask) for m in (fmu, fmv, fl)):
+            return None
+        else:
+            where.append(L.SG_MASK_PLANES)
+            for m, name, shape in ((fmu, "face_mask_u", face_u), (fmv, "face_mask_v", face_v), (fl, "is_fluid", cell)):
+                ptr, ld = L.mask_plane(m, name, shape)
+                where += (ptr.value, ld)
+        if self._ksolid is RING_BOX:
+            where += (L.SG_MASK_RING, 0, 0)
+        else:
+            mode, ptr, ld = ops._solid_arg(self._ksolid, H, W)
+            where += (mode, ptr.value if ptr is not None else 0, ld)
+        emits = self._pack_emitters(temp_on)
+        if emits is None:
+            return None
+        plumes = self._plume_rows()
+        n_emits = len(emits) // _EMIT.size
+        emits = ctypes.create_string_buffer(emits, max(len(emits), 1))
+        where += (adv, opr, len(plumes) if plumes is not None else 0,
+                  plumes.ctypes.data if plumes is not None else 0, int(self.seed) & (2**64 - 1),
+                  int(self.step_index), n_emits, ctypes.addressof(emits))
+        packed = _SUBSTEP.pack(*where, float(dt), float(self.cell_size), float(self.gravity), float(self.buoyancy),
+                               float(self.ambient_temperature), float(self.cooling_rate),
+                               float(self.density_dissipation), float(self.fluid_density),
+                               calculate_alpha(self.cell_size, self.fluid_density, dt), calculate_reciprocal_beta())
+        return packed, temp_on, (plumes, emits)  # the tables live until the calls have read them
+
+    def _pack_emitters(self, temp_on):
+        rows = b""
+        for e in self.emitters:
+            if not getattr(e, "enabled", True):
+                continue
+            approach = ops.APPROACH_CODES.get(e.approach)
+            if approach is None:
+                return None
+            x, y = e.position
+            for channel, value in ((0, e.density_value), (1, e.temperature_value if temp_on else 0.0),
+                                   (2, e.velocity_value[0]), (3, e.velocity_value[1])):
+                if value != 0.0:
+                    rows += _EMIT.pack(channel, float(value), float(x), float(y), float(e.radius), approach)
+        return rows
+
+    def _plume_rows(self):
+        """The plume table as the launch takes it, None without sources."""
+        if not self.plumes and self._plume_table is None:
+            return None
+        if self._plume_table is None:
+            self._plume_table = np.asarray([p.row() for p in self.plumes], dtype=np.float64).reshape(-1, 6)
+        return ops.plume_rows(self._plume_table)
+
+    def _native_substep(self, step):
+        packed, temp_on, _tables = step
+        stream = torch.cuda.current_stream().cuda_stream
+        L.call("sg_substep_transport", packed, stream)
+        self.velocity_u, self.velocity_u_temp = self.velocity_u_temp, self.velocity_u
+        self.velocity_v, self.velocity_v_temp = self.velocity_v_temp, self.velocity_v
+        self.density, self.density_temp = self.density_temp, self.density
+        if temp_on:
+            self._temperature, self.temperature_temp = self.temperature_temp, self._temperature
+        self._solve_pressure()
+        L.call("sg_substep_project", packed, stream)
+        self.velocity_u, self.velocity_u_temp = self.velocity_u_temp, self.velocity_u
+        self.velocity_v, self.velocity_v_temp = self.velocity_v_temp, self.velocity_v
+
     def _apply_emitters(self, dt):
         temp = self._temperature if self._temperature_needed() else None
         for e in self.emitters:
             emit_channels(e, self.density, self.velocity_u, self.velocity_v, temp, dt)
-        if self.plumes or self._plume_table is not None:
-            if self._plume_table is None:
-                self._plume_table = np.asarray([p.row() for p in self.plumes], dtype=np.float64).reshape(-1, 6)
-            ops.plume_sources(self.density, self.velocity_u, self.velocity_v, self._plume_table, self.seed,
-                              self.step_index)
+        rows = self._plume_rows()
+        if rows is not None:
+            ops.plume_sources(self.density, self.velocity_u, self.velocity_v, rows, self.seed, self.step_index)
 
     def _apply_forces(self, dt):
         temp = self._temperature if self._temperature_active else None
@@ -393,8 +500,10 @@ class SmokeSimulation2D:
         fmu, fmv, _ = self._kmasks
         # simulation.py:310 zeroes the pressure before every solve; the multigrid solve from a
         # zero guess does not read it (it writes p = 0 itself), so the fill is skipped there
+        # (nor do the other solvers that take the hint)
         if not (self.pressure_solver_method == "geometric_multigrid"
-                and not getattr(self.solver_params, "fixed_cycles", 0)):
+                and not getattr(self.solver_params, "fixed_cycles", 0)) \
+                and not starts_from_zero(self.pressure_solver_method, self.pressure_solver_backend):
             self.pressure.zero_()
         solve_pressure(self.pressure, self.divergence, fmu, fmv, self.fluid_density, self.cell_size, self.dt, self,
                        zero_initial_guess=True)
@@ -431,6 +540,19 @@ class SmokeSimulation2D:
         for t in (self.density, self.velocity_u, self.velocity_v, self._temperature, self.pressure, self.divergence):
             t.zero_()
         self.accumulator = 0.0
+
+
+# What the two native calls of a substep stand for: methods and operators that a program may
+# have replaced.
+_STEP_METHODS = {n: SmokeSimulation2D.__dict__[n] for n in (
+    "_apply_emitters", "_apply_forces", "_advect_velocity", "_advect_density", "_advect_temperature",
+    "_cool_temperature", "_compute_divergence", "_project_and_metrics", "_temperature_needed")}
+_STEP_OPERATORS = {n: getattr(ops, n) for n in (
+    "emit_scalar", "plume_sources", "apply_forces", "advect_velocity", "advect_scalar_field", "cool_temperature",
+    "compute_divergence", "project_metrics")}
+# sg_emit and sg_substep (include/smoke_b200.h): 8-byte members
+_EMIT = struct.Struct("<qddddq")
+_SUBSTEP = struct.Struct("<3q22q7q3q2q2qQq2q10d")
 
 
 class FieldReadback:

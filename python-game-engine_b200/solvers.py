@@ -13,13 +13,14 @@ from __future__ import annotations
 
 import ctypes
 import math
-from dataclasses import asdict
+from dataclasses import asdict, fields
 
 import numpy as np
 import torch
 
 from . import _lib as L
 from .operators import AnalyticMask, OPEN_BOX, RING_BOX, _face_pair, _masks, build_masks, compute_residual
+from .params import SOLVER_PARAM_TYPES
 from .registry import get_solver, register_solver
 
 
@@ -63,7 +64,8 @@ RESIDENT_MIN_JACOBI = 8
 RESIDENT_MIN_SOR = 2
 
 
-def _resident_sweeps(sor, dtc, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv, alpha, omega, iterations, device):
+def _resident_sweeps(sor, dtc, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv, alpha, omega, iterations, device,
+                     from_zero=False):
     """All sweeps in one launch with the iterate on the chip (``sg_sweeps_solve``: the same
     iterates); False when the grid does not fit there."""
     nbytes = L.load().sg_sweeps_workspace_bytes(dtc, H, W)
@@ -71,13 +73,14 @@ def _resident_sweeps(sor, dtc, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv, alpha
         return False
     ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
     L.call("sg_sweeps_solve", dtc, sor, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv, alpha, calculate_reciprocal_beta(),
-           float(omega), int(iterations), ws.data_ptr(), nbytes, L.stream_ptr())
+           float(omega), int(iterations), 1 if from_zero else 0, ws.data_ptr(), nbytes, L.stream_ptr())
     return True
 
 
 def jacobi_pressure_solver(pressure, divergence, face_mask_u, face_mask_v, fluid_density, cell_size, dt,
-                           iterations, scratch=None, **_ignored):
-    """jacobi.py:27-52: ``iterations`` ping-pong sweeps; the result ends in ``pressure``."""
+                           iterations, scratch=None, zero_initial_guess=False, **_ignored):
+    """jacobi.py:27-52: ``iterations`` ping-pong sweeps; the result ends in ``pressure``.
+    ``zero_initial_guess``: start from p = 0 whatever ``pressure`` holds."""
     H, W = pressure.shape
     dtc = L.dtype_code(pressure)
     mode, pu, lu, pv, lv = _face_pair(face_mask_u, face_mask_v, H, W)
@@ -85,8 +88,10 @@ def jacobi_pressure_solver(pressure, divergence, face_mask_u, face_mask_v, fluid
     d, ldd = L.field(divergence, "divergence", dtype=pressure.dtype)
     if scratch is None and iterations > RESIDENT_MIN_JACOBI and _resident_sweeps(
             0, dtc, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv, calculate_alpha(cell_size, fluid_density, dt), 0.0,
-            iterations, pressure.device):
+            iterations, pressure.device, zero_initial_guess):
         return
+    if zero_initial_guess:
+        pressure.zero_()
     if scratch is None:
         scratch = torch.empty((H, W), dtype=pressure.dtype, device=pressure.device)
     L.call("sg_jacobi_solve", dtc, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv,
@@ -95,8 +100,10 @@ def jacobi_pressure_solver(pressure, divergence, face_mask_u, face_mask_v, fluid
 
 
 def red_black_sor_gauss_seidel_pressure_solver(pressure, divergence, face_mask_u, face_mask_v, fluid_density,
-                                               cell_size, dt, iterations, omega: float = 0.0, **_ignored):
-    """red_black_sor_gauss_seidel.py:30-42 (omega <= 0 or > 2 selects the optimal omega)."""
+                                               cell_size, dt, iterations, omega: float = 0.0,
+                                               zero_initial_guess=False, **_ignored):
+    """red_black_sor_gauss_seidel.py:30-42 (omega <= 0 or > 2 selects the optimal omega).
+    ``zero_initial_guess``: start from p = 0 whatever ``pressure`` holds."""
     H, W = pressure.shape
     if omega <= 0.0 or omega > 2.0:
         omega = calculate_optimal_omega(max(H, W))
@@ -105,8 +112,10 @@ def red_black_sor_gauss_seidel_pressure_solver(pressure, divergence, face_mask_u
     d, ldd = L.field(divergence, "divergence", dtype=pressure.dtype)
     if iterations > RESIDENT_MIN_SOR and _resident_sweeps(
             1, L.dtype_code(pressure), H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv,
-            calculate_alpha(cell_size, fluid_density, dt), omega, iterations, pressure.device):
+            calculate_alpha(cell_size, fluid_density, dt), omega, iterations, pressure.device, zero_initial_guess):
         return
+    if zero_initial_guess:
+        pressure.zero_()
     L.call("sg_rbsor_solve", L.dtype_code(pressure), H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv,
            calculate_alpha(cell_size, fluid_density, dt), calculate_reciprocal_beta(), float(omega), int(iterations),
            L.stream_ptr())
@@ -195,7 +204,7 @@ class MultigridSolver:
         smoother(p, rhs, lv["fmu"], lv["fmv"], rho, h, dt, nu)
         return p
 
-    def _fused(self, smoother, pressure, divergence, rho, h, dt, cycles, nu, nu_c):
+    def _fused(self, smoother, pressure, divergence, rho, h, dt, cycles, nu, nu_c, from_zero):
         """The cycles in two launches per level (``sg_mg_vcycles``: the same values); False for
         what that does not take: another smoother, fields it cannot read in place, more sweeps
         a side than a tile's halo, a coarsest level too large for the chip."""
@@ -204,6 +213,8 @@ class MultigridSolver:
         elif smoother is red_black_sor_gauss_seidel_pressure_solver:
             sor = 1
         else:
+            return False
+        if from_zero and cycles < 1:
             return False
         if (divergence.dtype != pressure.dtype or divergence.shape != pressure.shape or pressure.stride(1) != 1
                 or divergence.stride(1) != 1 or divergence.device != pressure.device):
@@ -226,19 +237,21 @@ class MultigridSolver:
         p, ldp = L.field(pressure, "pressure")
         d, ldd = L.field(divergence, "divergence")
         L.call("sg_mg_vcycles", code, n, ctypes.addressof(table), p, ldp, d, ldd, calculate_reciprocal_beta(), sor,
-               int(cycles), int(nu), int(nu_c), self._workspace.data_ptr(), nbytes, L.stream_ptr())
+               int(cycles), int(nu), int(nu_c), 1 if from_zero else 0, self._workspace.data_ptr(), nbytes, L.stream_ptr())
         return True
 
     def __call__(self, pressure, divergence, face_mask_u, face_mask_v, fluid_density, cell_size, dt, v_cycles=2,
                  smoother_type="jacobi", smoother_backend="cuda", num_levels=4, smoother_iterations=2,
-                 coarsest_iterations=50, rebuild_masks=False, profiler=None, **_ignored):
+                 coarsest_iterations=50, rebuild_masks=False, profiler=None, zero_initial_guess=False, **_ignored):
         H, W = pressure.shape
         self._ensure(H, W, face_mask_u, face_mask_v, num_levels, pressure.dtype, pressure.device, rebuild_masks)
         backend = smoother_backend if smoother_backend == "cuda" else "cuda"
         smoother = get_solver(smoother_type, backend)
         if self._fused(smoother, pressure, divergence, fluid_density, cell_size, dt, v_cycles, smoother_iterations,
-                       coarsest_iterations):
+                       coarsest_iterations, zero_initial_guess):
             return
+        if zero_initial_guess:
+            pressure.zero_()
         fb = self.buffers[0]
         fb["pressure"].copy_(pressure)
         fb["rhs"].copy_(divergence)
@@ -539,12 +552,26 @@ class GeometricMultigridSolver:
 
 
 # ---------------------------------------------------------------- dispatch + registration
+# This package's parameter classes hold plain values only, so their fields need no deep copy.
+_FLAT_PARAMS = {t: tuple(f.name for f in fields(t)) for t in SOLVER_PARAM_TYPES.values()}
+
+
+def starts_from_zero(method, backend):
+    """Whether the registered solver honours the hint zero_initial_guess=True by itself (it then
+    does not read the pressure, which need not be cleared for it)."""
+    fn = get_solver(method, backend)
+    return (fn is jacobi_pressure_solver or fn is red_black_sor_gauss_seidel_pressure_solver
+            or type(fn) is MultigridSolver)
+
+
 def solve_pressure(pressure, divergence, face_mask_u, face_mask_v, fluid_density, cell_size, dt, params, **hints):
     """solvers/dispatch.py:5-12: look up (method, backend) and call with the params as kwargs.
     ``hints`` (e.g. zero_initial_guess=True from a caller that just zeroed the pressure) are
     passed along; solvers that do not use them ignore them."""
     fn = get_solver(params.pressure_solver_method, params.pressure_solver_backend)
-    kwargs = asdict(params.solver_params)
+    sp = params.solver_params
+    names = _FLAT_PARAMS.get(type(sp))
+    kwargs = asdict(sp) if names is None else {n: getattr(sp, n) for n in names}
     kwargs.update(hints)
     fn(pressure, divergence, face_mask_u, face_mask_v, fluid_density, cell_size, dt,
        profiler=getattr(params, "profiler", None), **kwargs)

@@ -63,7 +63,7 @@ def test_resident_sweeps_equal_plain_kernels(sor, dtype, shape, kind):
         got = torch.zeros((H, W + 5), dtype=dtype, device="cuda")[:, :W]
         got.copy_(dev(p0))
         rc = lib.sg_sweeps_solve(code, sor, H, W, got.data_ptr(), W + 5, d.data_ptr(), W + 3, *mask, -0.37, 0.25, 1.9,
-                                 iters, ws.data_ptr(), n, s)
+                                 iters, 0, ws.data_ptr(), n, s)
         assert rc == L.SG_OK, lib.sg_last_error()
         ref = dev(p0)
         if sor:
@@ -75,6 +75,16 @@ def test_resident_sweeps_equal_plain_kernels(sor, dtype, shape, kind):
         assert rc == L.SG_OK, lib.sg_last_error()
         torch.cuda.synchronize()
         assert torch.equal(got, ref), f"iterations {iters}: max {float((got - ref).abs().max()):.3e}"
+    # from zero: p is not read
+    got.fill_(float("nan"))
+    ref.zero_()
+    rc = lib.sg_sweeps_solve(code, sor, H, W, got.data_ptr(), W + 5, d.data_ptr(), W + 3, *mask, -0.37, 0.25, 1.9, 3, 1,
+                             ws.data_ptr(), n, s)
+    assert rc == L.SG_OK, lib.sg_last_error()
+    rc = lib.sg_sweeps_solve(code, sor, H, W, ref.data_ptr(), W, d.data_ptr(), W + 3, *mask, -0.37, 0.25, 1.9, 3, 0,
+                             ws.data_ptr(), n, s)
+    assert rc == L.SG_OK, lib.sg_last_error()
+    assert torch.equal(got, ref)
 
 
 def test_resident_sweeps_refuse_what_does_not_fit():
@@ -82,7 +92,7 @@ def test_resident_sweeps_refuse_what_does_not_fit():
     p = torch.zeros((4000, 4000), device="cuda")
     assert lib.sg_sweeps_workspace_bytes(L.SG_F32, 4000, 4000) == 0
     rc = lib.sg_sweeps_solve(L.SG_F32, 1, 4000, 4000, p.data_ptr(), 4000, p.data_ptr(), 4000, L.SG_MASK_OPEN, None, 0,
-                             None, 0, -1.0, 0.25, 1.5, 3, p.data_ptr(), p.numel() * 4, L.stream_ptr())
+                             None, 0, -1.0, 0.25, 1.5, 3, 0, p.data_ptr(), p.numel() * 4, L.stream_ptr())
     assert rc == L.SG_ERR_CAPACITY
     assert lib.sg_sweeps_workspace_bytes(7, 64, 64) == -1
 

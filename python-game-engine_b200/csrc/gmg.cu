@@ -1412,7 +1412,7 @@ static void tail_launch(const sg_gmg_plan* p, bool zero_init, cudaStream_t s) {
   a.post = p->post;
   a.wcycle = p->cycle;
   a.zero_init = zero_init ? 1 : 0;
-  SG_LAUNCH(k_gmg_tail_region<T><<<1, kRgThreads, p->tail_smem, s>>>(a));
+  SG_LAUNCH(k_gmg_tail_region<T><<<1, kRgTailThreads, p->tail_smem, s>>>(a));
 }
 
 // Register tiles on open levels of at least SG_GMG_REG_MIN_TILES 64 x 32 blocks, regions of

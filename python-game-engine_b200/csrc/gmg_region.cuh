@@ -40,25 +40,29 @@ __host__ __device__ inline int region_tiles(int n, int span, int halo) {
   return n <= span ? 1 : (n - 2 * halo + own - 1) / own;
 }
 
+// a where k has a bit of `bits`, else b; a select, never a branch
+__device__ __forceinline__ float pick_bits(uint32_t k, uint32_t bits, float a, float b) {
+  float o;
+  asm("{.reg .pred p; .reg .b32 t; and.b32 t, %1, %2; setp.ne.u32 p, t, 0; selp.f32 %0, %3, %4, p;}"
+      : "=f"(o) : "r"(k), "r"(bits), "f"(a), "f"(b));
+  return o;
+}
+__device__ __forceinline__ double pick_bits(uint32_t k, uint32_t bits, double a, double b) {
+  double o;
+  asm("{.reg .pred p; .reg .b32 t; and.b32 t, %1, %2; setp.ne.u32 p, t, 0; selp.f64 %0, %3, %4, p;}"
+      : "=d"(o) : "r"(k), "r"(bits), "d"(a), "d"(b));
+  return o;
+}
+
 struct RegionLevel {
   const uint8_t* code;  // H x W, row stride W; null on an open box
   int H, W;
-  __device__ __forceinline__ uint32_t get(int j, int i) const {
-    if (j < 0 || j >= H || i < 0 || i >= W) return 0;
-    if (code) return code[(int64_t)j * W + i];
-    uint32_t c = C_FLUID;
-    if (i > 0) c |= C_L;
-    if (i < W - 1) c |= C_R;
-    if (j > 0) c |= C_D;
-    if (j < H - 1) c |= C_U;
-    return c;
-  }
 };
 
-template <typename T>
+template <typename T, int NW>
 struct RegionEdges {
-  T top[2][kRgWarps][2][32];
-  T bot[2][kRgWarps][2][32];
+  T top[2][NW][2][32];
+  T bot[2][NW][2][32];
 };
 
 template <bool PART>
@@ -77,24 +81,40 @@ struct Region {
   uint32_t code[(RPT + 1) / 2];
 
   __device__ __forceinline__ uint32_t c(int r, int q) const { return (code[r >> 1] >> (16 * (r & 1) + 8 * q)) & 255; }
+  // Codes and weights of the cells at rows j + r, columns i + q (j, i >= 0). An open box's come
+  // from one row part and one column part each: formed cell by cell from the position they
+  // were a third of the tail's instructions.
   __device__ __forceinline__ void set_codes(const RegionLevel& m, int j, int i, T omega) {
+    uint32_t k[RPT][2];
+    if (m.code) {
+#pragma unroll
+      for (int r = 0; r < RPT; ++r)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)  // clamped, so that all loads are in flight at once
+          k[r][q] = m.code[(int64_t)min(j + r, m.H - 1) * m.W + min(i + q, m.W - 1)];
+    } else {
+      uint32_t col[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) col[q] = C_FLUID | (i + q > 0 ? C_L : 0) | (i + q < m.W - 1 ? C_R : 0);
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) {
+        const uint32_t row = (j + r > 0 ? C_D : 0) | (j + r < m.H - 1 ? C_U : 0);
+        k[r][0] = col[0] | row;
+        k[r][1] = col[1] | row;
+      }
+    }
 #pragma unroll
     for (int r = 0; r < (RPT + 1) / 2; ++r) code[r] = 0;
 #pragma unroll
     for (int r = 0; r < RPT; ++r)
 #pragma unroll
-      for (int q = 0; q < 2; ++q) code[r >> 1] |= m.get(j + r, i + q) << (16 * (r & 1) + 8 * q);
-    set_weights(omega);
-  }
-  __device__ __forceinline__ void set_weights(T omega) {
-#pragma unroll
-    for (int r = 0; r < RPT; ++r)
-#pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const uint32_t k = c(r, q);
-        const int n = __popc(k & (C_L | C_R | C_D | C_U));
-        rc[r][q] = rcp_open<T>(n);
-        om[r][q] = (k & C_FLUID) && n > 0 ? omega : (T)0;
+        if (j + r >= m.H || i + q >= m.W) k[r][q] = 0;
+        code[r >> 1] |= k[r][q] << (16 * (r & 1) + 8 * q);
+        const uint32_t n = __popc(k[r][q] & (C_L | C_R | C_D | C_U));  // 0 .. 4: bit 2 is set for 4 only
+        const T few = pick_bits(n, 1, pick_bits(n, 2, (T)(1.0 / 3.0), (T)1), (T)0.5);
+        rc[r][q] = pick_bits(n, 4, (T)0.25, few);
+        om[r][q] = pick_bits(n, 7, pick_bits(k[r][q], C_FLUID, omega, (T)0), (T)0);
       }
   }
 };
@@ -103,19 +123,17 @@ struct Region {
 // neighbouring lane's, or 0 at the region's ends (off the grid, or a halo cell).
 template <typename T>
 __device__ __forceinline__ T from_left(T v, int lane) {
-  const T t = __shfl_up_sync(0xffffffffu, v, 1);
-  return lane == 0 ? (T)0 : t;
+  return pick_bits(lane, ~0u, __shfl_up_sync(0xffffffffu, v, 1), (T)0);
 }
 template <typename T>
 __device__ __forceinline__ T from_right(T v, int lane) {
-  const T t = __shfl_down_sync(0xffffffffu, v, 1);
-  return lane == 31 ? (T)0 : t;
+  return pick_bits(31 - lane, ~0u, __shfl_down_sync(0xffffffffu, v, 1), (T)0);
 }
 
 // One half sweep of colour COL. nw: warps that hold rows of the level; the rows outside
 // the region count as 0.
-template <typename T, int COL, int RPT, bool PART>
-__device__ __forceinline__ void region_half_sweep(RegionEdges<T>& sh, int buf, int w, int lane, Region<T, RPT>& g,
+template <typename T, int COL, int RPT, bool PART, typename E>
+__device__ __forceinline__ void region_half_sweep(E& sh, int buf, int w, int lane, Region<T, RPT>& g,
                                                   int nw) {
   sh.bot[buf][w][0][lane] = g.e[RPT - 1][COL];  // for the next warp's first row
   sh.top[buf][w][0][lane] = g.e[0][1 - COL];    // for the previous warp's last row
@@ -127,8 +145,8 @@ __device__ __forceinline__ void region_half_sweep(RegionEdges<T>& sh, int buf, i
     acc[r] = g.b[r][q] + (q == 0 ? far : g.e[r][0]) + (q == 0 ? g.e[r][1] : far);
   }
   region_barrier<PART>(32 * nw);
-  const T below = w > 0 ? sh.bot[buf][w > 0 ? w - 1 : 0][0][lane] : (T)0;
-  const T above = w < nw - 1 ? sh.top[buf][w < nw - 1 ? w + 1 : w][0][lane] : (T)0;
+  const T below = pick_bits(w, ~0u, sh.bot[buf][max(w - 1, 0)][0][lane], (T)0);
+  const T above = pick_bits(nw - 1 - w, ~0u, sh.top[buf][min(w + 1, nw - 1)][0][lane], (T)0);
 #pragma unroll
   for (int r = 0; r < RPT; ++r) {
     const int q = (COL + r) & 1;
@@ -140,8 +158,8 @@ __device__ __forceinline__ void region_half_sweep(RegionEdges<T>& sh, int buf, i
   }
 }
 
-template <typename T, int RPT, bool PART>
-__device__ __forceinline__ void region_sweeps(RegionEdges<T>& sh, int& buf, int w, int lane, Region<T, RPT>& g,
+template <typename T, int RPT, bool PART, typename E>
+__device__ __forceinline__ void region_sweeps(E& sh, int& buf, int w, int lane, Region<T, RPT>& g,
                                               int sweeps, int nw) {
   for (int s = 0; s < sweeps; ++s) {
     region_half_sweep<T, 0, RPT, PART>(sh, buf, w, lane, g, nw);
@@ -152,8 +170,8 @@ __device__ __forceinline__ void region_sweeps(RegionEdges<T>& sh, int& buf, int 
 }
 
 // Rows -1 and RPT of the thread's columns.
-template <typename T, int RPT, bool PART>
-__device__ __forceinline__ void region_rows(RegionEdges<T>& sh, int& buf, int w, int lane, const Region<T, RPT>& g,
+template <typename T, int RPT, bool PART, typename E>
+__device__ __forceinline__ void region_rows(E& sh, int& buf, int w, int lane, const Region<T, RPT>& g,
                                             int nw, T (&below)[2], T (&above)[2]) {
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
@@ -163,8 +181,8 @@ __device__ __forceinline__ void region_rows(RegionEdges<T>& sh, int& buf, int w,
   region_barrier<PART>(32 * nw);
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
-    below[q] = w > 0 ? sh.bot[buf][w > 0 ? w - 1 : 0][q][lane] : (T)0;
-    above[q] = w < nw - 1 ? sh.top[buf][w < nw - 1 ? w + 1 : w][q][lane] : (T)0;
+    below[q] = pick_bits(w, ~0u, sh.bot[buf][max(w - 1, 0)][q][lane], (T)0);
+    above[q] = pick_bits(nw - 1 - w, ~0u, sh.top[buf][min(w + 1, nw - 1)][q][lane], (T)0);
   }
   buf ^= 1;
 }
@@ -185,11 +203,11 @@ __device__ __forceinline__ void region_minus_ae(const Region<T, RPT>& g, int lan
       const TP u = (TP)(r < RPT - 1 ? g.e[r < RPT - 1 ? r + 1 : r][q] : above[q]);
       // differences, not a sum less n x: they stay exact near convergence, where the sum cancels
       TP s = (TP)0;
-      s += (k & C_L) ? l - x : (TP)0;
-      s += (k & C_R) ? rt - x : (TP)0;
-      s += (k & C_D) ? d - x : (TP)0;
-      s += (k & C_U) ? u - x : (TP)0;
-      out[r][q] = (k & C_FLUID) ? s : (TP)0;
+      s += pick_bits(k, C_L, l - x, (TP)0);
+      s += pick_bits(k, C_R, rt - x, (TP)0);
+      s += pick_bits(k, C_D, d - x, (TP)0);
+      s += pick_bits(k, C_U, u - x, (TP)0);
+      out[r][q] = pick_bits(k, C_FLUID, s, (TP)0);
     }
   }
 }
@@ -198,35 +216,34 @@ __device__ __forceinline__ void region_minus_ae(const Region<T, RPT>& g, int lan
 // fine rows 2m, 2m + 1. j, i: the thread's first cell; H, W, Hc, Wc: the two levels. The
 // weights are those of the bilinear prolongation with candidates clamped to the grid
 // (separable); where a candidate is not fluid, its share is added to the home cell.
-template <typename T, int RPT, bool PART, typename F>
-__device__ __forceinline__ void region_restrict(RegionEdges<T>& sh, int& buf, int w, int lane, const Region<T, RPT>& g,
+template <typename T, int RPT, bool PART, typename E, typename F>
+__device__ __forceinline__ void region_restrict(E& sh, int& buf, int w, int lane, const Region<T, RPT>& g,
                                                 int nw, int j, int i, int H, int W, int Hc, int Wc, F store) {
   T below[2], above[2], res[RPT][2];
   region_rows<T, RPT, PART>(sh, buf, w, lane, g, nw, below, above);
   region_minus_ae<T, T, RPT>(g, lane, below, above, res);
   const int I = i >> 1;
-  const T wx0 = (2 * I - 1 >= 0 && 2 * I - 1 < W) ? (T)w1(2 * I - 1, I, Wc) : (T)0;
-  const T wx1 = 2 * I < W ? (T)w1(2 * I, I, Wc) : (T)0;
-  const T wx2 = 2 * I + 1 < W ? (T)w1(2 * I + 1, I, Wc) : (T)0;
-  const T wx3 = 2 * I + 2 < W ? (T)w1(2 * I + 2, I, Wc) : (T)0;
+  // w1 of fine columns 2I - 1 .. 2I + 2 (0 off the grid): a fine cell's outer candidate is
+  // clamped to its home one at an edge
+  const T wx0 = I > 0 ? (T)0.25 : (T)0, wx3 = 2 * I + 2 < W ? (T)0.25 : (T)0;
+  const T wx1 = I > 0 ? (T)0.75 : (T)1, wx2 = I < Wc - 1 ? (T)0.75 : (T)1;
   T X[RPT], home[RPT / 2];
-  bool fluid[RPT / 2];
+  uint32_t fluid[RPT / 2];
 #pragma unroll
   for (int m = 0; m < RPT / 2; ++m) {
     home[m] = (T)0;
-    fluid[m] = false;
+    fluid[m] = 0;
   }
 #pragma unroll
   for (int r = 0; r < RPT; ++r) {
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const uint32_t k = g.c(r, q);
-      if (k & C_FLUID) {
-        res[r][q] += g.b[r][q];
-        fluid[r >> 1] = true;
-      }
-      const int extra = ((k & C_XHOME) ? 3 : 0) + ((k & C_YHOME) ? 3 : 0) + ((k & C_DHOME) ? 1 : 0);
-      home[r >> 1] += (T)(extra * (1.0f / 16.0f)) * res[r][q];
+      res[r][q] += pick_bits(k, C_FLUID, g.b[r][q], (T)0);
+      fluid[r >> 1] |= k;
+      const T extra = pick_bits(k, C_XHOME, (T)(3.0 / 16), (T)0) + pick_bits(k, C_YHOME, (T)(3.0 / 16), (T)0) +
+                      pick_bits(k, C_DHOME, (T)(1.0 / 16), (T)0);
+      home[r >> 1] += extra * res[r][q];
     }
     const T rl = from_left(res[r][1], lane), rr = from_right(res[r][0], lane);
     T acc = wx0 * rl;
@@ -238,21 +255,19 @@ __device__ __forceinline__ void region_restrict(RegionEdges<T>& sh, int& buf, in
   sh.bot[buf][w][0][lane] = X[RPT - 1];
   sh.top[buf][w][0][lane] = X[0];
   region_barrier<PART>(32 * nw);
-  const T xa = w > 0 ? sh.bot[buf][w > 0 ? w - 1 : 0][0][lane] : (T)0;
-  const T xb = w < nw - 1 ? sh.top[buf][w < nw - 1 ? w + 1 : w][0][lane] : (T)0;
+  const T xa = pick_bits(w, ~0u, sh.bot[buf][max(w - 1, 0)][0][lane], (T)0);
+  const T xb = pick_bits(nw - 1 - w, ~0u, sh.top[buf][min(w + 1, nw - 1)][0][lane], (T)0);
   buf ^= 1;
 #pragma unroll
   for (int m = 0; m < RPT / 2; ++m) {
     const int J = (j >> 1) + m;
-    const T wy0 = (2 * J - 1 >= 0 && 2 * J - 1 < H) ? (T)w1(2 * J - 1, J, Hc) : (T)0;
-    const T wy1 = 2 * J < H ? (T)w1(2 * J, J, Hc) : (T)0;
-    const T wy2 = 2 * J + 1 < H ? (T)w1(2 * J + 1, J, Hc) : (T)0;
-    const T wy3 = 2 * J + 2 < H ? (T)w1(2 * J + 2, J, Hc) : (T)0;
+    const T wy0 = J > 0 ? (T)0.25 : (T)0, wy3 = 2 * J + 2 < H ? (T)0.25 : (T)0;
+    const T wy1 = J > 0 ? (T)0.75 : (T)1, wy2 = J < Hc - 1 ? (T)0.75 : (T)1;
     T acc = wy0 * (m > 0 ? X[m > 0 ? 2 * m - 1 : 0] : xa);
     acc += wy1 * X[2 * m];
     acc += wy2 * X[2 * m + 1];
     acc += wy3 * (2 * m + 2 < RPT ? X[2 * m + 2 < RPT ? 2 * m + 2 : 0] : xb);
-    store(m, fluid[m] ? acc + home[m] : (T)0);
+    store(m, pick_bits(fluid[m], C_FLUID, acc + home[m], (T)0));
   }
 }
 
@@ -277,10 +292,10 @@ __device__ __forceinline__ void region_prolong(Region<T, RPT>& g, int j, F coars
         const T x = q == 0 ? cl : cr, y = h == 0 ? pm : nm;
         const T d = h == 0 ? (q == 0 ? pl : pr) : (q == 0 ? nl : nr);
         T acc = w9 * cm;
-        acc += w3 * ((k & C_XHOME) ? cm : x);
-        acc += w3 * ((k & C_YHOME) ? cm : y);
-        acc += wd * ((k & C_DHOME) ? cm : d);
-        if (k & C_FLUID) g.e[r][q] = g.e[r][q] + acc;
+        acc += w3 * pick_bits(k, C_XHOME, cm, x);
+        acc += w3 * pick_bits(k, C_YHOME, cm, y);
+        acc += wd * pick_bits(k, C_DHOME, cm, d);
+        g.e[r][q] = g.e[r][q] + pick_bits(k, C_FLUID, acc, (T)0);
       }
     }
     pl = cl;
@@ -337,11 +352,15 @@ __device__ __forceinline__ void region_load(Region<T, kRgRows>& g, const RegionA
   for (int r = 0; r < kRgRows; ++r)
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      const bool in = at.j + r < a.m.H && at.i + q < a.m.W;
-      const int64_t o = (int64_t)(at.j + r) * a.ld + at.i + q;
-      g.b[r][q] = in ? b[o] : (T)0;
-      g.e[r][q] = in && a.e_in ? a.e_in[o] : (T)0;
+      const int64_t o = (int64_t)min(at.j + r, a.m.H - 1) * a.ld + min(at.i + q, a.m.W - 1);
+      g.b[r][q] = b[o];
+      g.e[r][q] = a.e_in ? a.e_in[o] : (T)0;
     }
+#pragma unroll
+  for (int r = 0; r < kRgRows; ++r)
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (at.j + r >= a.m.H || at.i + q >= a.m.W) g.b[r][q] = g.e[r][q] = (T)0;
   g.set_codes(a.m, at.j, at.i, a.omega);
 }
 
@@ -361,7 +380,7 @@ __device__ __forceinline__ void region_store(const Region<T, kRgRows>& g, const 
 
 template <typename T>
 __global__ void __launch_bounds__(kRgThreads) k_gmg_pre_region(const __grid_constant__ RegionArgs<T> a) {
-  __shared__ RegionEdges<T> sh;
+  __shared__ RegionEdges<T, kRgWarps> sh;
   RegionPlace at;
   at.set(a);
   Region<T, kRgRows> g;
@@ -384,7 +403,7 @@ __global__ void __launch_bounds__(kRgThreads) k_gmg_pre_region(const __grid_cons
 // solves, whose residual is formed from p afresh).
 template <typename T, typename TP, int FINAL>
 __global__ void __launch_bounds__(kRgThreads) k_gmg_post_region(const __grid_constant__ RegionArgs<T> a) {
-  __shared__ RegionEdges<T> sh;
+  __shared__ RegionEdges<T, kRgWarps> sh;
   RegionPlace at;
   at.set(a);
   Region<T, kRgRows> g;
@@ -446,6 +465,9 @@ __global__ void __launch_bounds__(kRgThreads) k_gmg_post_region(const __grid_con
 
 // ------------------------------------------------------------------ tail
 constexpr int kRgTailSide = 64;
+constexpr int kRgTailRows = 2;
+constexpr int kRgTailWarps = kRgTailSide / kRgTailRows;
+constexpr int kRgTailThreads = 32 * kRgTailWarps;
 constexpr int kRgPinvShared = 64;  // coarsest cells up to which the pseudo-inverse is kept in shared memory
 
 template <typename T>
@@ -465,7 +487,7 @@ struct RegionTailArgs {
 template <typename T>
 static size_t region_tail_smem(int cells, int coarsest_cells) {
   const int pinv = coarsest_cells <= kRgPinvShared ? coarsest_cells * coarsest_cells : 0;
-  return (size_t)pinv * 8 + (size_t)cells * (2 * sizeof(T) + 1);
+  return sizeof(RegionEdges<T, kRgTailWarps>) + (size_t)pinv * 8 + (size_t)cells * 2 * sizeof(T);
 }
 
 template <typename T>
@@ -473,36 +495,55 @@ struct RegionTailShared {
   double* pinv;
   T* e;
   T* b;
-  uint8_t* code;
+  // the level table, copied here: parameters indexed by a run-time level are slow constant
+  // loads (32^2 visit: 1400 of 4900 clocks for the codes alone)
+  RegionLevel m[kMaxLevels];
+  int off[kMaxLevels];
 };
 
 // Level l: its pre side (sweeps from e, or from zero; the next level's rhs) or its post side.
-template <typename T, int RPT>
+template <typename T>
 __device__ __forceinline__ void region_tail_visit(const RegionTailArgs<T>& a, const RegionTailShared<T>& t,
-                                                  RegionEdges<T>& sh, int l, bool post, bool zero) {
+                                                  RegionEdges<T, kRgTailWarps>& sh, int l, bool post, bool zero) {
+  constexpr int RPT = kRgTailRows;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int H = a.m[l].H, W = a.m[l].W, Hc = a.m[l + 1].H, Wc = a.m[l + 1].W;
+  const RegionLevel m = t.m[l];
+  const int H = m.H, W = m.W, Hc = t.m[l + 1].H, Wc = t.m[l + 1].W, o = t.off[l], oc = t.off[l + 1];
   const int nw = (H + RPT - 1) / RPT;
   if (w >= nw) return;
   const int j = w * RPT, i = 2 * lane;
   Region<T, RPT> g;
-#pragma unroll
-  for (int r = 0; r < (RPT + 1) / 2; ++r) g.code[r] = 0;
+  // the first level's rhs (and its start value) stay in global memory, the others' lie in the
+  // shared arrays; clamped addresses, so that all loads are in flight at once
+  const int j1 = min(j + 1, H - 1), i0 = min(i, W - 1), i1 = min(i + 1, W - 1);
+  static_assert(RPT == 2, "rows j and j1");
+  if (l == 0) {
+    const int64_t r0 = j * a.gld, r1 = j1 * a.gld;
+    g.b[0][0] = a.gb[r0 + i0], g.b[0][1] = a.gb[r0 + i1], g.b[1][0] = a.gb[r1 + i0], g.b[1][1] = a.gb[r1 + i1];
+    if (!post && !zero)
+      g.e[0][0] = a.ge[r0 + i0], g.e[0][1] = a.ge[r0 + i1], g.e[1][0] = a.ge[r1 + i0], g.e[1][1] = a.ge[r1 + i1];
+  } else {
+    const T* bs = t.b + o;
+    const int r0 = j * W, r1 = j1 * W;
+    g.b[0][0] = bs[r0 + i0], g.b[0][1] = bs[r0 + i1], g.b[1][0] = bs[r1 + i0], g.b[1][1] = bs[r1 + i1];
+  }
+  if (zero) {
+    g.e[0][0] = g.e[0][1] = g.e[1][0] = g.e[1][1] = (T)0;
+  } else if (post || l > 0) {
+    const T* es = t.e + o;
+    const int r0 = j * W, r1 = j1 * W;
+    g.e[0][0] = es[r0 + i0], g.e[0][1] = es[r0 + i1], g.e[1][0] = es[r1 + i0], g.e[1][1] = es[r1 + i1];
+  }
+  g.set_codes(m, j, i, a.omega);
 #pragma unroll
   for (int r = 0; r < RPT; ++r)
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const bool in = j + r < H && i + q < W;
-      const int o = a.off[l] + (j + r) * W + i + q;
-      g.e[r][q] = in && !zero ? t.e[o] : (T)0;
-      g.b[r][q] = in ? t.b[o] : (T)0;
-      g.code[r >> 1] |= (in ? (uint32_t)t.code[o] : 0u) << (16 * (r & 1) + 8 * q);
-    }
-  g.set_weights(a.omega);
+    for (int q = 0; q < 2; ++q)
+      if (j + r >= H || i + q >= W) g.b[r][q] = g.e[r][q] = (T)0;
   if (post) {
     const int I = min(i >> 1, Wc - 1), Il = max((i >> 1) - 1, 0), Ir = min((i >> 1) + 1, Wc - 1);
     region_prolong<T, RPT>(g, j, [&](int J, T& cl, T& cm, T& cr) {
-      const T* row = t.e + a.off[l + 1] + min(max(J, 0), Hc - 1) * Wc;
+      const T* row = t.e + oc + min(max(J, 0), Hc - 1) * Wc;
       cl = row[min(Il, Wc - 1)];
       cm = row[I];
       cr = row[Ir];
@@ -518,43 +559,41 @@ __device__ __forceinline__ void region_tail_visit(const RegionTailArgs<T>& a, co
         if (post && l == 0)
           a.ge[(int64_t)(j + r) * a.gld + i + q] = g.e[r][q];
         else
-          t.e[a.off[l] + (j + r) * W + i + q] = g.e[r][q];
+          t.e[o + (j + r) * W + i + q] = g.e[r][q];
       }
   if (post) return;
   region_restrict<T, RPT, true>(sh, buf, w, lane, g, nw, j, i, H, W, Hc, Wc, [&](int m, T v) {
     const int J = (j >> 1) + m, I = i >> 1;
-    if (J < Hc && I < Wc) t.b[a.off[l + 1] + J * Wc + I] = v;
+    if (J < Hc && I < Wc) t.b[oc + J * Wc + I] = v;
   });
 }
 
-// The warps whose rows lie beyond a level wait for the others at the visit's end, and levels of
-// at most 32 rows take two rows a thread: what a small level costs is the length of one warp's
-// instruction stream.
+// The warps whose rows lie beyond a level wait for the others at the visit's end. Two rows a
+// thread: what a small level costs is the length of one warp's instruction stream. That stream
+// has no branch that lanes could part at: as ternaries, the edge tests of codes, weights,
+// residual and prolongation were branches that the grid's edge lanes took apart from the others
+// (64^2 down, float32: 17.8 us with them, 15.2 us with selects).
 template <typename T>
-__global__ void __launch_bounds__(kRgThreads) k_gmg_tail_region(const __grid_constant__ RegionTailArgs<T> a) {
+__global__ void __launch_bounds__(kRgTailThreads) k_gmg_tail_region(const __grid_constant__ RegionTailArgs<T> a) {
   extern __shared__ __align__(16) unsigned char region_smem[];
-  __shared__ RegionEdges<T> sh;
+  RegionEdges<T, kRgTailWarps>& sh = *reinterpret_cast<RegionEdges<T, kRgTailWarps>*>(region_smem);
   const int last = a.n - 1, nc = a.m[last].H * a.m[last].W;
   const bool keep = nc <= kRgPinvShared;
-  RegionTailShared<T> t;
-  t.pinv = reinterpret_cast<double*>(region_smem);
-  t.e = reinterpret_cast<T*>(t.pinv + (keep ? nc * nc : 0));
-  t.b = t.e + a.cells;
-  t.code = reinterpret_cast<uint8_t*>(t.b + a.cells);
+  __shared__ RegionTailShared<T> t;
+  double* const pinv_s = reinterpret_cast<double*>(region_smem + sizeof(sh));
   const int tid = threadIdx.x;
-  for (int l = 0; l < a.n; ++l) {
-    const int n = a.m[l].H * a.m[l].W;
-    for (int q = tid; q < n; q += kRgThreads) {
-      const int j = q / a.m[l].W, i = q - j * a.m[l].W;
-      t.code[a.off[l] + q] = (uint8_t)a.m[l].get(j, i);
-      if (l == 0) {
-        t.b[q] = a.gb[(int64_t)j * a.gld + i];
-        t.e[q] = a.zero_init ? (T)0 : a.ge[(int64_t)j * a.gld + i];
-      }
-    }
+  if (tid == 0) {
+    t.pinv = pinv_s;
+    t.e = reinterpret_cast<T*>(pinv_s + (keep ? nc * nc : 0));
+    t.b = t.e + a.cells;
   }
-  if (keep)
-    for (int q = tid; q < nc * nc; q += kRgThreads) t.pinv[q] = a.pinv[q];
+  if (tid < a.n) {
+    t.m[tid] = a.m[tid];
+    t.off[tid] = a.off[tid];
+  }
+  if (keep)  // lands while the levels above run
+    for (int q = tid; q < nc * nc; q += kRgTailThreads)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_addr(pinv_s + q)), "l"(a.pinv + q) : "memory");
   __syncthreads();
   int l = 0;
   bool down = true;
@@ -562,18 +601,23 @@ __global__ void __launch_bounds__(kRgThreads) k_gmg_tail_region(const __grid_con
   unsigned fresh = a.zero_init ? ~0u : ~1u;  // bit l: level l starts from zero
   while (true) {
     if (l == last) {  // e = pinv b, eight threads a row
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+      const T* bc = last == 0 ? a.gb : t.b + t.off[l];
+      const int Wl = t.m[l].W;
       const double* pinv = keep ? t.pinv : a.pinv;
-      for (int row = tid >> 3; row < ((nc + 63) & ~63); row += kRgThreads / 8) {
+      for (int row = tid >> 3; row < ((nc + 127) & ~127); row += kRgTailThreads / 8) {
         double acc = 0.0;
         if (row < nc)
-          for (int q = tid & 7; q < nc; q += 8) acc += pinv[(int64_t)row * nc + q] * (double)t.b[a.off[l] + q];
+          for (int q = tid & 7; q < nc; q += 8)
+            acc += pinv[(int64_t)row * nc + q] * (double)(last == 0 ? bc[(int64_t)(q / Wl) * a.gld + q % Wl] : bc[q]);
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if (row < nc && (tid & 7) == 0) {
           if (last == 0)
             a.ge[(int64_t)(row / a.m[0].W) * a.gld + row % a.m[0].W] = (T)acc;
           else
-            t.e[a.off[l] + row] = (T)acc;
+            t.e[t.off[l] + row] = (T)acc;
         }
       }
       __syncthreads();
@@ -590,10 +634,7 @@ __global__ void __launch_bounds__(kRgThreads) k_gmg_tail_region(const __grid_con
       continue;
     }
     const bool zero = down && ((fresh >> l) & 1u);
-    if (a.m[l].H <= 2 * kRgWarps)
-      region_tail_visit<T, 2>(a, t, sh, l, !down, zero);
-    else
-      region_tail_visit<T, 4>(a, t, sh, l, !down, zero);
+    region_tail_visit<T>(a, t, sh, l, !down, zero);
     __syncthreads();
     if (down) {
       second &= ~(1u << l);

@@ -115,19 +115,20 @@ struct MgRegion {
 // multigrid/transfer.py:5-36 for the 2 x 2 cells at rows r, r + 1 of the thread
 template <typename T, int RPT>
 __device__ __forceinline__ T mg_restrict(const T (&res)[RPT][2], const uint32_t* code, int r, T divisor) {
-  double total = 0.0;
+  double total = 0.0;  // res is 0 off the fluid
   int count = 0;
 #pragma unroll
   for (int d = 0; d < 2; ++d)
 #pragma unroll
-    for (int q = 0; q < 2; ++q)
-      if (res_code(code, r + d, q) & K_FLUID) {
-        total += (double)res[r + d][q];
-        ++count;
-      }
+    for (int q = 0; q < 2; ++q) {
+      total += (double)res[r + d][q];
+      count += (res_code(code, r + d, q) >> 4) & 1;
+    }
+  static_assert(K_FLUID == 16, "bit 4");
   // a division by 4, 2 or 1 is the multiplication by its exact reciprocal
-  const double mean = count == 4 ? total * 0.25 : (count == 3 ? total / 3.0 : (count == 2 ? total * 0.5 : total));
-  return (count > 0 ? (T)mean : (T)0) / divisor;
+  const double by = count == 4 ? 0.25 : (count == 2 ? 0.5 : 1.0);
+  const double mean = count == 3 ? total / 3.0 : total * by;
+  return (T)mean / divisor;
 }
 
 // multigrid/transfer.py:38-72: the correction of fluid cell (j, i), sample_ref at
@@ -135,8 +136,8 @@ __device__ __forceinline__ T mg_restrict(const T (&res)[RPT][2], const uint32_t*
 // latter, exact in both forms; at an edge both are the same cell and the weight is void.
 template <typename T>
 __device__ __forceinline__ T mg_prolong(const T* c, int64_t ldc, int Hc, int Wc, int j, int i) {
-  const int x0 = max((i - 1) >> 1, 0), x1 = min((i + 1) >> 1, Wc - 1);
-  const int y0 = max((j - 1) >> 1, 0), y1 = min((j + 1) >> 1, Hc - 1);
+  const int x1 = min((i + 1) >> 1, Wc - 1), x0 = min(max((i - 1) >> 1, 0), x1);  // i, j may lie off the grid
+  const int y1 = min((j + 1) >> 1, Hc - 1), y0 = min(max((j - 1) >> 1, 0), y1);
   const double tx = (i & 1) ? 0.25 : 0.75, ty = (j & 1) ? 0.25 : 0.75;
   const T* r0 = c + (int64_t)y0 * ldc;
   const T* r1 = c + (int64_t)y1 * ldc;
@@ -259,8 +260,8 @@ __device__ __forceinline__ void mg_tail_visit(const MgTailArgs<T>& a, const MgTa
     for (int r = 0; r < RPT; ++r)
 #pragma unroll
       for (int q = 0; q < 2; ++q)
-        if (res_code(code, r, q) & K_FLUID)
-          e[r][q] = e[r][q] + mg_prolong((const T*)t.p + a.off[l + 1], W >> 1, H >> 1, W >> 1, j + r, i + q);
+        e[r][q] = e[r][q] + pick(res_code(code, r, q) & K_FLUID,
+                                 mg_prolong((const T*)t.p + a.off[l + 1], W >> 1, H >> 1, W >> 1, j + r, i + q), (T)0);
   }
   const bool plain = __all_sync(0xffffffffu, all);
   res_sweeps<T, SOR, RPT, true>(sh, buf, w, lane, e, ab, code, plain, i == 0, i + 1 == W - 1, a.rb, omega,
@@ -291,7 +292,7 @@ __device__ __forceinline__ void mg_tail_visit(const MgTailArgs<T>& a, const MgTa
 // of at most 32 rows take two rows a thread, so twice the warps: what a small level costs is
 // the length of one warp's instruction stream. (64^2 down to 8^2 with 30 coarsest SOR sweeps,
 // float32: 50 us with all 16 warps in every half sweep and the codes formed from the masks,
-// 38 us with idle warps left out and codes from global memory, 27 us so.)
+// 38 us with idle warps left out and codes from global memory, 25 us so.)
 template <typename T, bool SOR>
 __global__ void __launch_bounds__(kResThreads) k_mg_tail(const __grid_constant__ MgTailArgs<T> a) {
   extern __shared__ __align__(16) unsigned char mg_smem[];

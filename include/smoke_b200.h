@@ -328,6 +328,15 @@ int sg_gauss_seidel_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p
                           const uint8_t* fmv, int64_t ld_fmv, double alpha, double reciprocal_beta,
                           int iterations, void* stream);
 
+/* The same sweeps (the same iterates) split over a chain of blocks that hand their diagonals on
+ * through workspace (16-byte aligned, sg_gauss_seidel_workspace_bytes; cleared by the call;
+ * null: one block). 0 bytes: the call has no chain form and needs none. */
+int64_t sg_gauss_seidel_workspace_bytes(int dtype, int64_t H, int64_t W, int iterations);
+int sg_gauss_seidel_sweeps(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div,
+                           int64_t ld_div, int mask_mode, const uint8_t* fmu, int64_t ld_fmu,
+                           const uint8_t* fmv, int64_t ld_fmv, double alpha, double reciprocal_beta,
+                           int iterations, void* workspace, int64_t workspace_bytes, void* stream);
+
 /* multigrid/transfer.py:5-36 (restrict: mean of the fluid children) with the coarse
  * rhs division of multigrid/solver.py:124-125 fused (coarse = round(mean) / round(divisor)
  * in dtype; pass 1.0 for none). */

@@ -54,6 +54,8 @@ SIGNATURES = {
     "sg_substep_project": [P, P],
     "sg_sweeps_workspace_bytes": [I, I64, I64],
     "sg_sweeps_solve": [I, I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, D, I, I, P, I64, P],
+    "sg_gauss_seidel_workspace_bytes": [I, I64, I64, I],
+    "sg_gauss_seidel_sweeps": [I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, I, P, I64, P],
     "sg_gauss_seidel_solve": [I, I64, I64, P, I64, P, I64, I, P, I64, P, I64, D, D, I, P],
     "sg_rbsor_split_workspace_bytes": [I, I64, I64],
     "sg_rbsor_split_pack": [I, I64, I64, P, I64, I, P, I64, P],
@@ -146,6 +148,7 @@ _RESTYPE = {
     "sg_field_stats_workspace_bytes": ctypes.c_int64,
     "sg_rbsor_split_workspace_bytes": ctypes.c_int64,
     "sg_sweeps_workspace_bytes": ctypes.c_int64,
+    "sg_gauss_seidel_workspace_bytes": ctypes.c_int64,
     "sg_mg_codes_bytes": ctypes.c_int64,
     "sg_mg_vcycles_workspace_bytes": ctypes.c_int64,
     "sg_rbsor_mixed_workspace_bytes": ctypes.c_int64,

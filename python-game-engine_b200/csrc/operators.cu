@@ -6,6 +6,7 @@
 // Launch shape: 32x8 threads, one thread per cell/face, x along the contiguous row.
 
 #include <atomic>
+#include <climits>
 #include <cstring>
 #include <mutex>
 
@@ -907,24 +908,42 @@ int sg_rbsor_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, const
   return check_launch("sg_rbsor_solve");
 }
 
-int sg_gauss_seidel_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div, int64_t ld_div,
-                          int mask_mode, const uint8_t* fmu, int64_t ld_fmu, const uint8_t* fmv, int64_t ld_fmv,
-                          double alpha, double reciprocal_beta, int iterations, void* stream) {
+int64_t sg_gauss_seidel_workspace_bytes(int dtype, int64_t H, int64_t W, int iterations) {
+  if ((dtype != SG_F32 && dtype != SG_F64) || H < 1 || W < 1 || iterations < 0) return -1;
+  const int M = (int)std::min<int64_t>(std::min(H, W), INT_MAX);
+  return dtype == SG_F32 ? gauss_seidel_workspace<float>(M, iterations) : gauss_seidel_workspace<double>(M, iterations);
+}
+
+int sg_gauss_seidel_sweeps(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div, int64_t ld_div,
+                           int mask_mode, const uint8_t* fmu, int64_t ld_fmu, const uint8_t* fmv, int64_t ld_fmv,
+                           double alpha, double reciprocal_beta, int iterations, void* workspace,
+                           int64_t workspace_bytes, void* stream) {
   SG_CHECK(check_grid(H, W));
   SG_REQUIRE(p && div && ld_p >= W && ld_div >= W, "bad fields");
   SG_REQUIRE(iterations >= 0, "iterations must be >= 0");
   SG_CHECK(check_mask_mode(mask_mode, fmu, fmv));
   if (iterations == 0) return SG_OK;
+  const int64_t need = sg_gauss_seidel_workspace_bytes(dtype, H, W, iterations);
+  if (workspace)
+    SG_REQUIRE(!((uintptr_t)workspace & 15) && workspace_bytes >= need,
+               "workspace must be 16-byte aligned and hold %lld bytes", (long long)need);
   Masks m = make_masks(mask_mode, H, W, fmu, ld_fmu, fmv, ld_fmv, nullptr, 0);
   SG_DISPATCH(dtype, {
     bool ran = false;
     SG_CHECK(gauss_seidel_wave<T>((int)H, (int)W, (T*)p, ld_p, (const T*)div, ld_div, m, alpha, reciprocal_beta,
-                                  iterations, &ran, as_stream(stream)));
+                                  iterations, need > 0 ? workspace : nullptr, &ran, as_stream(stream)));
     if (ran) return SG_OK;
     SG_LAUNCH(k_gauss_seidel<T><<<1, 1024, 0, as_stream(stream)>>>((int)H, (int)W, (T*)p, ld_p, (const T*)div, ld_div, m, alpha,
                                                          reciprocal_beta, iterations));
   });
-  return check_launch("sg_gauss_seidel_solve");
+  return check_launch("sg_gauss_seidel_sweeps");
+}
+
+int sg_gauss_seidel_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div, int64_t ld_div,
+                          int mask_mode, const uint8_t* fmu, int64_t ld_fmu, const uint8_t* fmv, int64_t ld_fmv,
+                          double alpha, double reciprocal_beta, int iterations, void* stream) {
+  return sg_gauss_seidel_sweeps(dtype, H, W, p, ld_p, div, ld_div, mask_mode, fmu, ld_fmu, fmv, ld_fmv, alpha,
+                                reciprocal_beta, iterations, nullptr, 0, stream);
 }
 
 int sg_mg_restrict_average(int dtype, int64_t H, int64_t W, const void* fine, int64_t ld_f, int mask_mode,

@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
 }
 
 // ------------------------------------------------------------------ host side
-static int sm_count() {
+int sm_count() {
   int dev = 0, n = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return 0;

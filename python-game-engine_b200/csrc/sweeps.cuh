@@ -10,8 +10,7 @@ namespace sg {
 // cell itself), both contribute the cell's own value.
 enum : uint32_t { K_L = 1, K_R = 2, K_D = 4, K_U = 8, K_FLUID = 16, K_ALL = 31 };
 
-__device__ __forceinline__ uint32_t cell_code(const Masks& m, int H, int W, int j, int i) {
-  const bool l = m.u(j, i), r = m.u(j, i + 1), d = m.v(j, i), u = m.v(j + 1, i);
+__device__ __forceinline__ uint32_t faces_code(bool l, bool r, bool d, bool u, int H, int W, int j, int i) {
   uint32_t c = 0;
   if (l && i > 0) c |= K_L;
   if (r && i < W - 1) c |= K_R;
@@ -19,6 +18,9 @@ __device__ __forceinline__ uint32_t cell_code(const Masks& m, int H, int W, int 
   if (u && j < H - 1) c |= K_U;
   if (l || r || d || u) c |= K_FLUID;
   return c;
+}
+__device__ __forceinline__ uint32_t cell_code(const Masks& m, int H, int W, int j, int i) {
+  return faces_code(m.u(j, i), m.u(j, i + 1), m.v(j, i), m.v(j + 1, i), H, W, j, i);
 }
 
 // Rows per thread of the resident sweeps on an H x W grid, 0 when it does not fit the chip,
@@ -37,9 +39,16 @@ int resident_sweeps(int sor, int split, int H, int W, T* p, T* p1, int64_t ldp, 
                     const Masks& m, double alpha, double rb, double omega, int sweeps, bool from_zero, void* xchg,
                     uint32_t tag, cudaStream_t s);
 
+// SMs of the current device (0: unknown).
+int sm_count();
+
 // Lexicographic Gauss-Seidel sweeps; *ran is false when the grid is too wide for it.
+// workspace: gauss_seidel_workspace bytes (M: the shorter side; 0: none needed), cleared by the
+// call, or null for one block.
+template <typename T>
+int64_t gauss_seidel_workspace(int M, int iterations);
 template <typename T>
 int gauss_seidel_wave(int H, int W, T* p, int64_t ldp, const T* div, int64_t ldd, const Masks& m, double alpha,
-                      double rb, int iterations, bool* ran, cudaStream_t s);
+                      double rb, int iterations, void* workspace, bool* ran, cudaStream_t s);
 
 }  // namespace sg

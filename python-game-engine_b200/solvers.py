@@ -123,14 +123,19 @@ def red_black_sor_gauss_seidel_pressure_solver(pressure, divergence, face_mask_u
 
 def gauss_seidel_pressure_solver(pressure, divergence, face_mask_u, face_mask_v, fluid_density, cell_size, dt,
                                  iterations, **_ignored):
-    """gauss_seidel.py:29-48 (lexicographic order, as anti-diagonal wavefronts in one block)."""
+    """gauss_seidel.py:29-48 (lexicographic order, as anti-diagonal wavefronts; short grids
+    on a chain of blocks that hand diagonals on through the workspace)."""
     H, W = pressure.shape
+    iterations = int(iterations)
+    dtc = L.dtype_code(pressure)
     mode, pu, lu, pv, lv = _face_pair(face_mask_u, face_mask_v, H, W)
     p, ldp = L.field(pressure, "pressure")
     d, ldd = L.field(divergence, "divergence", dtype=pressure.dtype)
-    L.call("sg_gauss_seidel_solve", L.dtype_code(pressure), H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv,
-           calculate_alpha(cell_size, fluid_density, dt), calculate_reciprocal_beta(), int(iterations),
-           L.stream_ptr())
+    nbytes = max(0, L.load().sg_gauss_seidel_workspace_bytes(dtc, H, W, iterations))
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=pressure.device) if nbytes else None
+    L.call("sg_gauss_seidel_sweeps", dtc, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv,
+           calculate_alpha(cell_size, fluid_density, dt), calculate_reciprocal_beta(), iterations,
+           ws.data_ptr() if nbytes else None, nbytes, L.stream_ptr())
 
 
 class MultigridSolver:

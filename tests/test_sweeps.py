@@ -2,7 +2,7 @@
 kernels and the CPU oracle, bit for bit: grids at the edges of the blocks' regions (64 columns;
 32, 64 or 128 rows), odd extents, every mask kind, row strides, sweep counts that end between
 two trades of the blocks' frames, and the pipelined Gauss-Seidel wavefront in one and in
-several passes."""
+several passes, in one block and in a chain of blocks."""
 import numpy as np
 import pytest
 import torch
@@ -110,3 +110,29 @@ def test_gauss_seidel_wave_equals_oracle(dtype, shape, kind, iters):
     mu, mv = (sg.OPEN_BOX,) * 2 if kind == "open" else ((sg.RING_BOX,) * 2 if kind == "ring" else (dev(fmu), dev(fmv)))
     sg.solvers.gauss_seidel_pressure_solver(got, dev(div), mu, mv, 1.0, 1.0 / W, 0.5 / W, iterations=iters)
     assert np.array_equal(got.cpu().numpy(), exp)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("shape,kind,iters", [
+    ((2, 3), "open", 7), ((31, 33), "ring", 200), ((32, 900), "planes", 17), ((900, 32), "open", 64),
+    ((513, 520), "planes", 3), ((600, 1024), "ring", 5), ((1024, 530), "open", 150)])
+def test_gauss_seidel_chain_equals_one_block(dtype, shape, kind, iters):
+    """Blocks with loaders of their own and without, rings that wrap, more sweeps than a launch holds."""
+    H, W = shape
+    lib = L.load()
+    npdt = np.float32 if dtype == torch.float32 else np.float64
+    p0, div, fmu, fmv = _case(H, W, npdt, kind, 11 * H + W)
+    code = L.dtype_code(torch.empty((), dtype=dtype))
+    keep, mask = _mask_args(kind, fmu, fmv, W)
+    n = int(lib.sg_gauss_seidel_workspace_bytes(code, H, W, iters))
+    ws = torch.full((max(n, 16),), 1, dtype=torch.uint8, device="cuda")
+    got = torch.zeros((H, W + 5), dtype=dtype, device="cuda")[:, :W]
+    got.copy_(dev(p0))
+    ref, d = dev(p0), dev(div)
+    args = (d.data_ptr(), W, *mask, -0.37, 0.25, iters)
+    assert lib.sg_gauss_seidel_sweeps(code, H, W, got.data_ptr(), W + 5, *args, ws.data_ptr(), n, L.stream_ptr()) == 0
+    assert lib.sg_gauss_seidel_solve(code, H, W, ref.data_ptr(), W, *args, L.stream_ptr()) == 0
+    assert torch.equal(got, ref)
+    if n:
+        rc = lib.sg_gauss_seidel_sweeps(code, H, W, got.data_ptr(), W + 5, *args, ws.data_ptr(), n - 1, L.stream_ptr())
+        assert rc == L.SG_ERR_ARG

@@ -40,20 +40,6 @@ __host__ __device__ inline int region_tiles(int n, int span, int halo) {
   return n <= span ? 1 : (n - 2 * halo + own - 1) / own;
 }
 
-// a where k has a bit of `bits`, else b; a select, never a branch
-__device__ __forceinline__ float pick_bits(uint32_t k, uint32_t bits, float a, float b) {
-  float o;
-  asm("{.reg .pred p; .reg .b32 t; and.b32 t, %1, %2; setp.ne.u32 p, t, 0; selp.f32 %0, %3, %4, p;}"
-      : "=f"(o) : "r"(k), "r"(bits), "f"(a), "f"(b));
-  return o;
-}
-__device__ __forceinline__ double pick_bits(uint32_t k, uint32_t bits, double a, double b) {
-  double o;
-  asm("{.reg .pred p; .reg .b32 t; and.b32 t, %1, %2; setp.ne.u32 p, t, 0; selp.f64 %0, %3, %4, p;}"
-      : "=d"(o) : "r"(k), "r"(bits), "d"(a), "d"(b));
-  return o;
-}
-
 struct RegionLevel {
   const uint8_t* code;  // H x W, row stride W; null on an open box
   int H, W;

@@ -117,11 +117,89 @@ __device__ __forceinline__ void exchange_rows(RegXchg<T, NWARP>& x, int buf, con
   below[1] = b.y;
 }
 
+__constant__ double kRcpOpen[5] = {1.0, 1.0, 0.5, 1.0 / 3.0, 0.25};  // rcp_open
+
+// What a tile at the grid's edge knows about a thread's cells, made once: branches on it parted
+// the edge lanes from the rest of the warp in every row of every half sweep (batch of 256
+// scenes: pre 55.5 us, fused post 105.5 us).
+template <typename T, int RPT>
+struct RegEdge {
+  static_assert(RPT <= 8, "a byte of rows each");
+  static constexpr bool kInside = false, kSelect = true;
+  uint32_t on[2];   // bit r: row r of column q is on the grid
+  uint32_t rows;    // bit r: both vertical faces open; 8 + r: the upper (j - 1); 16 + r: the lower
+  uint32_t cols;    // bit q: the left face open; 2 + q: the right
+  // open faces of column q where both vertical faces are open, and where not: in float32 as
+  // their reciprocals (float64 has no registers for those)
+  using R = std::conditional_t<sizeof(T) == 4, T, int>;
+  R two[2], one[2];
+
+  __device__ __forceinline__ RegEdge(int j, int i, int H, int W) {
+    uint32_t in = 0;
+    rows = cols = 0;
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+      const int jj = j + r;
+      in |= (uint32_t)(jj >= 0 && jj < H) << r;
+      rows |= ((uint32_t)(jj > 0 && jj < H - 1) << r) | ((uint32_t)(jj > 0) << (8 + r)) |
+              ((uint32_t)(jj < H - 1) << (16 + r));
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int ii = i + q;
+      on[q] = ii >= 0 && ii < W ? in : 0u;
+      cols |= ((uint32_t)(ii > 0) << q) | ((uint32_t)(ii < W - 1) << (2 + q));
+      const int nx = (ii > 0) + (ii < W - 1), n1 = nx + (H > 1);  // one row: no vertical face
+      if constexpr (sizeof(T) == 4) {
+        two[q] = rcp_open<T>(nx + 2);
+        one[q] = rcp_open<T>(n1);
+      } else {
+        two[q] = nx + 2;
+        one[q] = n1;
+      }
+    }
+  }
+  __device__ __forceinline__ T rcp(int r, int q) const {
+    if constexpr (sizeof(T) == 4)
+      return pick_bits(rows, 1u << r, two[q], one[q]);
+    else
+      return kRcpOpen[(rows >> r & 1) ? two[q] : one[q]];
+  }
+};
+// The same by branches, for the fused post kernel in float64, whose registers are full: there
+// the selects' extra values spilt (2048^2: 53.6 -> 58.4 us).
+template <typename T, int RPT>
+struct RegEdgeBranches {
+  static constexpr bool kInside = false, kSelect = false;
+  int j, i, H, W;
+  __device__ __forceinline__ RegEdgeBranches(int j_, int i_, int H_, int W_) : j(j_), i(i_), H(H_), W(W_) {}
+  __device__ __forceinline__ bool on(int r, int q) const {
+    return j + r >= 0 && j + r < H && i + q >= 0 && i + q < W;
+  }
+  __device__ __forceinline__ bool open(int r, int q, int face) const {  // left, right, up (j - 1), down
+    return face == 0 ? i + q > 0 : face == 1 ? i + q < W - 1 : face == 2 ? j + r > 0 : j + r < H - 1;
+  }
+  __device__ __forceinline__ int faces(int r, int q) const {
+    return open(r, q, 0) + open(r, q, 1) + open(r, q, 2) + open(r, q, 3);
+  }
+};
+template <typename T, int RPT>
+struct RegInside {  // every cell of the tile on the grid and off its edge
+  static constexpr bool kInside = true, kSelect = false;
+  __device__ __forceinline__ RegInside(int, int, int, int) {}
+};
+template <typename T, int RPT, bool BOUNDED>
+using RegBounds = std::conditional_t<BOUNDED, RegEdge<T, RPT>, RegInside<T, RPT>>;
+template <typename T, int RPT, bool BOUNDED>
+using RegFinalBounds =
+    std::conditional_t<BOUNDED, std::conditional_t<sizeof(T) == 4, RegEdge<T, RPT>, RegEdgeBranches<T, RPT>>,
+                       RegInside<T, RPT>>;
+
 // One half sweep of colour COL over the thread's cells. Row r, column q has colour
-// (r + q) & 1. BOUNDED: tile touches the grid edge; (j, i) of the thread's first cell.
-template <typename T, int RPT, int COL, bool BOUNDED>
+// (r + q) & 1. G: what the tile knows of the grid's edge.
+template <typename T, int RPT, int COL, typename G>
 __device__ __forceinline__ void reg_half_sweep(T (&e)[RPT][2], const T (&b)[RPT][2], const T (&above)[2],
-                                               const T (&below)[2], T omega, int j, int i, int H, int W) {
+                                               const T (&below)[2], T omega, const G& g) {
 #pragma unroll
   for (int r = 0; r < RPT; ++r) {
     const int q = (COL + r) & 1;
@@ -134,14 +212,14 @@ __device__ __forceinline__ void reg_half_sweep(T (&e)[RPT][2], const T (&b)[RPT]
     const T down = r < RPT - 1 ? e[r < RPT - 1 ? r + 1 : 0][q] : below[q];
     const T acc = b[r][q] + left + right + up + down;
     const T x = e[r][q];
-    if (!BOUNDED) {
+    if constexpr (G::kInside) {
       e[r][q] = x + omega * (acc * (T)0.25 - x);
-    } else {
-      const int jj = j + r, ii = i + q;
-      if (jj >= 0 && jj < H && ii >= 0 && ii < W) {
-        const int n = (ii > 0) + (ii < W - 1) + (jj > 0) + (jj < H - 1);
-        if (n > 0) e[r][q] = x + omega * (acc * rcp_open<T>(n) - x);
-      }
+    } else if constexpr (G::kSelect) {
+      const T rc = g.rcp(r, q);
+      e[r][q] = pick_bits(g.on[q], 1u << r, x + omega * (acc * rc - x), x);
+    } else if (g.on(r, q)) {
+      const int n = g.faces(r, q);
+      if (n > 0) e[r][q] = x + omega * (acc * rcp_open<T>(n) - x);
     }
   }
 }
@@ -149,32 +227,32 @@ __device__ __forceinline__ void reg_half_sweep(T (&e)[RPT][2], const T (&b)[RPT]
 // The first half sweep (colour 0) from e = 0: every neighbour is 0, so the update is
 // omega * (b * 1/n) (the general formula with x = 0 and a zero neighbour sum: the same
 // value, up to the sign of a zero) and needs no row exchange.
-template <typename T, int RPT, bool BOUNDED>
-__device__ __forceinline__ void reg_first_half_sweep_from_zero(T (&e)[RPT][2], const T (&b)[RPT][2], T omega, int j,
-                                                               int i, int H, int W) {
+template <typename T, int RPT, typename G>
+__device__ __forceinline__ void reg_first_half_sweep_from_zero(T (&e)[RPT][2], const T (&b)[RPT][2], T omega,
+                                                               const G& g) {
 #pragma unroll
   for (int r = 0; r < RPT; ++r) {
     const int q = r & 1;
-    if (!BOUNDED) {
+    if constexpr (G::kInside) {
       e[r][q] = omega * (b[r][q] * (T)0.25);
-    } else {
-      const int jj = j + r, ii = i + q;
-      if (jj >= 0 && jj < H && ii >= 0 && ii < W) {
-        const int n = (ii > 0) + (ii < W - 1) + (jj > 0) + (jj < H - 1);
-        if (n > 0) e[r][q] = omega * (b[r][q] * rcp_open<T>(n));
-      }
+    } else if constexpr (G::kSelect) {
+      const T rc = g.rcp(r, q);
+      e[r][q] = pick_bits(g.on[q], 1u << r, omega * (b[r][q] * rc), (T)0);
+    } else if (g.on(r, q)) {
+      const int n = g.faces(r, q);
+      if (n > 0) e[r][q] = omega * (b[r][q] * rcp_open<T>(n));
     }
   }
 }
 
-template <typename T, int RPT, int NWARP, int NHS, int HS, bool BOUNDED>
+template <typename T, int RPT, int NWARP, int NHS, int HS, typename G>
 __device__ __forceinline__ void reg_sweeps(RegXchg<T, NWARP>& x, T (&e)[RPT][2], const T (&b)[RPT][2], T omega,
-                                           int w, int lane, int j, int i, int H, int W) {
+                                           int w, int lane, const G& g) {
   if constexpr (HS < NHS) {
     T above[2], below[2];
     exchange_rows<T, RPT, NWARP>(x, HS & 1, e, w, lane, above, below);
-    reg_half_sweep<T, RPT, HS & 1, BOUNDED>(e, b, above, below, omega, j, i, H, W);
-    reg_sweeps<T, RPT, NWARP, NHS, HS + 1, BOUNDED>(x, e, b, omega, w, lane, j, i, H, W);
+    reg_half_sweep<T, RPT, HS & 1>(e, b, above, below, omega, g);
+    reg_sweeps<T, RPT, NWARP, NHS, HS + 1>(x, e, b, omega, w, lane, g);
   }
 }
 
@@ -251,15 +329,16 @@ __device__ __forceinline__ void reg_pre_body(RegXchg<T, NWARP>& x, const T* __re
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int i = i0 + 2 * lane, j = j0 + w * RPT;
   T e[RPT][2], b[RPT][2];
+  const RegBounds<T, RPT, BOUNDED> g(j, i, H, W);
   reg_load<T, RPT, BOUNDED>(b, bsrc, ld, j, i, H, W);
   if (e_in) {
     reg_load<T, RPT, BOUNDED>(e, e_in, ld, j, i, H, W);
-    reg_sweeps<T, RPT, NWARP, 2 * SW, 0, BOUNDED>(x, e, b, omega, w, lane, j, i, H, W);
+    reg_sweeps<T, RPT, NWARP, 2 * SW, 0>(x, e, b, omega, w, lane, g);
   } else {
 #pragma unroll
     for (int r = 0; r < RPT; ++r) e[r][0] = e[r][1] = (T)0;
-    reg_first_half_sweep_from_zero<T, RPT, BOUNDED>(e, b, omega, j, i, H, W);
-    reg_sweeps<T, RPT, NWARP, 2 * SW, 1, BOUNDED>(x, e, b, omega, w, lane, j, i, H, W);
+    reg_first_half_sweep_from_zero<T, RPT>(e, b, omega, g);
+    reg_sweeps<T, RPT, NWARP, 2 * SW, 1>(x, e, b, omega, w, lane, g);
   }
   // residual b - A e in place of b
   T above[2], below[2];
@@ -275,22 +354,18 @@ __device__ __forceinline__ void reg_pre_body(RegXchg<T, NWARP>& x, const T* __re
       const T right = q == 0 ? e[r][1] : r0;
       const T up = r > 0 ? e[r > 0 ? r - 1 : 0][q] : above[q];
       const T down = r < RPT - 1 ? e[r < RPT - 1 ? r + 1 : 0][q] : below[q];
-      if (!BOUNDED) {
+      if constexpr (!BOUNDED) {
         if constexpr (sizeof(T) == 8)  // float64: the cheaper sum form (see the fused post kernel)
           b[r][q] = b[r][q] + (((left + right) + (up + down)) - (T)4 * xv);
         else
           b[r][q] = b[r][q] + (left - xv) + (right - xv) + (up - xv) + (down - xv);
       } else {
-        const int jj = j + r, ii = i + q;
-        T acc = (T)0;
-        if (jj >= 0 && jj < H && ii >= 0 && ii < W) {
-          acc = b[r][q];
-          if (ii > 0) acc += left - xv;
-          if (ii < W - 1) acc += right - xv;
-          if (jj > 0) acc += up - xv;
-          if (jj < H - 1) acc += down - xv;
-        }
-        b[r][q] = acc;
+        T acc = b[r][q];
+        acc = pick_bits(g.cols, 1u << q, acc + (left - xv), acc);
+        acc = pick_bits(g.cols, 4u << q, acc + (right - xv), acc);
+        acc = pick_bits(g.rows, 256u << r, acc + (up - xv), acc);
+        acc = pick_bits(g.rows, 65536u << r, acc + (down - xv), acc);
+        b[r][q] = pick_bits(g.on[q], 1u << r, acc, (T)0);
       }
     }
   }
@@ -376,11 +451,11 @@ __global__ void __launch_bounds__(32 * NWARP, MINB) k_gmg_pre_reg(const T* __res
 #endif
 
 // e = e_in + P ec on the thread's cells, then SW sweeps (e and b stay in registers).
-template <typename T, int SW, int RPT, int NWARP, bool BOUNDED>
+template <typename T, int SW, int RPT, int NWARP, bool BOUNDED, typename G>
 __device__ __forceinline__ void reg_prolong_smooth(RegXchg<T, NWARP>& x, T (&e)[RPT][2], T (&b)[RPT][2],
                                                    const T* __restrict__ e_in, const T* __restrict__ bsrc, int64_t ld,
                                                    int H, int W, const T* __restrict__ ec, int64_t ldc, int Hc, int Wc,
-                                                   T omega, int i0, int j0) {
+                                                   T omega, int i0, int j0, const G& g) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int i = i0 + 2 * lane, j = j0 + w * RPT;
   reg_load<T, RPT, BOUNDED>(b, bsrc, ld, j, i, H, W);
@@ -427,7 +502,13 @@ __device__ __forceinline__ void reg_prolong_smooth(RegXchg<T, NWARP>& x, T (&e)[
         acc += w3 * (q == 0 ? cl : cr);
         acc += w3 * ym;
         acc += wd * (q == 0 ? yl : yr);
-        if (!BOUNDED || (j + r >= 0 && j + r < H && i + q >= 0 && i + q < W)) e[r][q] = e[r][q] + acc;
+        if constexpr (!BOUNDED) {
+          e[r][q] = e[r][q] + acc;
+        } else if constexpr (G::kSelect) {
+          e[r][q] = pick_bits(g.on[q], 1u << r, e[r][q] + acc, e[r][q]);
+        } else {
+          if (g.on(r, q)) e[r][q] = e[r][q] + acc;
+        }
       }
     }
     pl = cl;
@@ -437,7 +518,7 @@ __device__ __forceinline__ void reg_prolong_smooth(RegXchg<T, NWARP>& x, T (&e)[
     cm = nm;
     cr = nr;
   }
-  reg_sweeps<T, RPT, NWARP, 2 * SW, 0, BOUNDED>(x, e, b, omega, w, lane, j, i, H, W);
+  reg_sweeps<T, RPT, NWARP, 2 * SW, 0>(x, e, b, omega, w, lane, g);
 }
 
 template <typename T, int SW, int RPT, int NWARP, bool BOUNDED>
@@ -448,8 +529,9 @@ __device__ __forceinline__ void reg_post_body(RegXchg<T, NWARP>& x, const T* __r
   using S = RegPost<T, SW, RPT, NWARP>;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int i = i0 + 2 * lane, j = j0 + w * RPT;
+  const RegBounds<T, RPT, BOUNDED> g(j, i, H, W);
   T e[RPT][2], b[RPT][2];
-  reg_prolong_smooth<T, SW, RPT, NWARP, BOUNDED>(x, e, b, e_in, bsrc, ld, H, W, ec, ldc, Hc, Wc, omega, i0, j0);
+  reg_prolong_smooth<T, SW, RPT, NWARP, BOUNDED>(x, e, b, e_in, bsrc, ld, H, W, ec, ldc, Hc, Wc, omega, i0, j0, g);
   const int r_lo = S::HALO - w * RPT, r_hi = S::HALO + S::TYO - w * RPT;
   reg_store<T, RPT, BOUNDED>(e, e_out, ld, j, i, H, W, 2 * lane >= S::HALO && 2 * lane < S::HALO + S::TXO, r_lo,
                              r_hi);
@@ -514,8 +596,9 @@ __device__ __forceinline__ void reg_post_final_body(RegXchg<TC, NWARP>& x, const
       if (r64) prefetch_l2(r64 + (int64_t)(j + r) * ld + i);
     }
   }
+  const RegFinalBounds<TC, RPT, BOUNDED> g(j, i, H, W);
   TC e[RPT][2], b[RPT][2];
-  reg_prolong_smooth<TC, SW, RPT, NWARP, BOUNDED>(x, e, b, e_in, bsrc, ld, H, W, ec, ldc, Hc, Wc, omega, i0, j0);
+  reg_prolong_smooth<TC, SW, RPT, NWARP, BOUNDED>(x, e, b, e_in, bsrc, ld, H, W, ec, ldc, Hc, Wc, omega, i0, j0, g);
   TC above[2], below[2];
   exchange_rows<TC, RPT, NWARP>(x, (2 * SW) & 1, e, w, lane, above, below);
   using VC = typename Pair<TC>::V;
@@ -549,13 +632,12 @@ __device__ __forceinline__ void reg_post_final_body(RegXchg<TC, NWARP>& x, const
     TP xv[2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      const int ii = i + q;
       xv[q] = (TP)e[r][q];
       const TP left = (TP)(q == 0 ? l1 : e[r][0]);
       const TP right = (TP)(q == 0 ? e[r][1] : r0);
       const TP up = (TP)(r > 0 ? e[r > 0 ? r - 1 : 0][q] : above[q]);
       const TP down = (TP)(r < RPT - 1 ? e[r < RPT - 1 ? r + 1 : 0][q] : below[q]);
-      if (!BOUNDED) {
+      if constexpr (!BOUNDED) {
         if constexpr (sizeof(TP) == 8) {
           // float64: one sum and one fused multiply-add (the float32 form below keeps the
           // differences, which stay exact near convergence where the sum would cancel)
@@ -566,11 +648,16 @@ __device__ __forceinline__ void reg_post_final_body(RegXchg<TC, NWARP>& x, const
           acc[q] += up - xv[q];
           acc[q] += down - xv[q];
         }
+      } else if constexpr (sizeof(TC) == 8) {  // RegEdgeBranches
+        if (g.open(r, q, 0)) acc[q] += left - xv[q];
+        if (g.open(r, q, 1)) acc[q] += right - xv[q];
+        if (g.open(r, q, 2)) acc[q] += up - xv[q];
+        if (g.open(r, q, 3)) acc[q] += down - xv[q];
       } else {
-        if (ii > 0) acc[q] += left - xv[q];
-        if (ii < W - 1) acc[q] += right - xv[q];
-        if (jj > 0) acc[q] += up - xv[q];
-        if (jj < H - 1) acc[q] += down - xv[q];
+        acc[q] = pick_bits(g.cols, 1u << q, acc[q] + (left - xv[q]), acc[q]);
+        acc[q] = pick_bits(g.cols, 4u << q, acc[q] + (right - xv[q]), acc[q]);
+        acc[q] = pick_bits(g.rows, 256u << r, acc[q] + (up - xv[q]), acc[q]);
+        acc[q] = pick_bits(g.rows, 65536u << r, acc[q] + (down - xv[q]), acc[q]);
       }
     }
     TP* pc = p + (int64_t)jj * ldp + i;

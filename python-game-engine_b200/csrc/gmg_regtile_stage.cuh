@@ -37,7 +37,8 @@ __device__ __forceinline__ void reg_post_final_body_staged(RegXchg<TC, NWARP>& x
   const bool cols_owned = 2 * lane >= S::HALO && 2 * lane < S::HALO + S::TXO;
   const int r_lo = S::HALO - w * RPT, r_hi = S::HALO + S::TYO - w * RPT;
   TC e[RPT][2], b[RPT][2];
-  reg_prolong_smooth<TC, SW, RPT, NWARP, false>(x, e, b, e_in, bsrc, ld, H, W, ec, ldc, Hc, Wc, omega, i0, j0);
+  reg_prolong_smooth<TC, SW, RPT, NWARP, false>(x, e, b, e_in, bsrc, ld, H, W, ec, ldc, Hc, Wc, omega, i0, j0,
+                                               RegInside<TC, RPT>(0, 0, 0, 0));
   TC above[2], below[2];
   exchange_rows<TC, RPT, NWARP>(x, (2 * SW) & 1, e, w, lane, above, below);
   // every thread waits, so the block cannot retire while a copy is still landing

@@ -21,6 +21,20 @@ __device__ __forceinline__ float w1(int i, int I, int n) {
   return (h == I ? 0.75f : 0.0f) + (x == I ? 0.25f : 0.0f);
 }
 
+// a where k has a bit of `bits`, else b; a select, never a branch
+__device__ __forceinline__ float pick_bits(uint32_t k, uint32_t bits, float a, float b) {
+  float o;
+  asm("{.reg .pred p; .reg .b32 t; and.b32 t, %1, %2; setp.ne.u32 p, t, 0; selp.f32 %0, %3, %4, p;}"
+      : "=f"(o) : "r"(k), "r"(bits), "f"(a), "f"(b));
+  return o;
+}
+__device__ __forceinline__ double pick_bits(uint32_t k, uint32_t bits, double a, double b) {
+  double o;
+  asm("{.reg .pred p; .reg .b32 t; and.b32 t, %1, %2; setp.ne.u32 p, t, 0; selp.f64 %0, %3, %4, p;}"
+      : "=d"(o) : "r"(k), "r"(bits), "d"(a), "d"(b));
+  return o;
+}
+
 // 1 / (number of open faces), n in 1..4.
 template <typename T>
 __device__ __forceinline__ T rcp_open(int n) {

@@ -456,6 +456,42 @@ static int launch_tiles(int H, int W, const SplitWs& w, bool a_to_b, MasksT<MM> 
   return SG_OK;
 }
 
+// The resident sweeps' exchange buffer holds no tags before the first use.
+static int resident_ready(SplitWs& w, cudaStream_t s) {
+  if (w.tag != 0) return SG_OK;
+  cudaError_t e = cudaMemsetAsync(w.xchg, 0, w.xchg_bytes, s);
+  if (e != cudaSuccess) return fail(SG_ERR_CUDA, "memset: %s", cudaGetErrorString(e));
+  w.tag = 1;
+  return SG_OK;
+}
+
+// Sweeps until the check in u says stop, of which at most `iterations` are left; the launches
+// hold kResidentSweeps each or one check's sweeps. *sweeps: how many were made, *sq: the last
+// check's sum of squares.
+template <typename T>
+static int sweeps_until(int H, int W, SplitWs& w, const Masks& m, double alpha, double rb, double omega,
+                        SweepsUntil u, int64_t iterations, int64_t* sweeps, double* sq, cudaStream_t s) {
+  SG_CHECK(resident_ready(w, s));
+  *sweeps = 0;
+  while (true) {
+    const int whole = std::max(1, kResidentSweeps / u.check_every) * u.check_every;
+    u.max_sweeps = (int)std::min<int64_t>(whole, iterations - *sweeps);
+    SweepsReached x{};
+    SG_CHECK(resident_sweeps_until<T>(H, W, (T*)w.a[0], (T*)w.a[1], w.ldh, (const T*)w.d[0], (const T*)w.d[1], w.ldh,
+                                      m, alpha, rb, 1.0 / rb, omega, u, w.xchg, w.tag, &x, s));
+    for (int64_t n = 0; n < x.sweeps; n += u.check_every)
+      w.tag += (uint32_t)resident_trades(1, (int)std::min<int64_t>(u.check_every, x.sweeps - n));
+    *sweeps += x.sweeps;
+    *sq = x.sq;
+    const double rel = u.r0 > 0.0 ? std::sqrt(x.sq) / u.r0 : 0.0;
+    if (!(rel > u.tol) || !std::isfinite(rel) || *sweeps >= iterations ||
+        (u.stall_limit > 0 && x.stalls >= u.stall_limit))
+      return SG_OK;
+    u.best = x.best;
+    u.stalls = (int)x.stalls;
+  }
+}
+
 // `iterations` sweeps on state a (the result ends in a). variant 0: two streaming half-sweep
 // launches per sweep; variant 1: tile launches of up to kTileHalo / 2 sweeps each, an even
 // number of them (a -> b -> a ...), or streaming launches for a single sweep.
@@ -464,11 +500,7 @@ static int split_sweeps(int H, int W, SplitWs& w, MasksT<MM> m, double alpha, do
                         int64_t iterations, int variant, cudaStream_t s) {
   if (iterations <= 0) return SG_OK;
   if (variant == 2) {
-    if (w.tag == 0) {
-      cudaError_t e = cudaMemsetAsync(w.xchg, 0, w.xchg_bytes, s);
-      if (e != cudaSuccess) return fail(SG_ERR_CUDA, "memset: %s", cudaGetErrorString(e));
-      w.tag = 1;
-    }
+    SG_CHECK(resident_ready(w, s));
     while (iterations > 0) {
       const int n = (int)std::min<int64_t>(iterations, kResidentSweeps);
       SG_CHECK(resident_sweeps<T>(1, 1, H, W, (T*)w.a[0], (T*)w.a[1], w.ldh, (const T*)w.d[0], (const T*)w.d[1], w.ldh,
@@ -628,7 +660,13 @@ int sg_rbsor_tol_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, c
       split_sumsq<T, MM>((int)H, (int)W, w, mm, alpha, beta, 0, w.result, s);
       SG_CHECK(read_scalar(w.result, &sq, s));
       rel = r0 > 0.0 ? std::sqrt(sq) / r0 : 0.0;
-      while (rel > tol && it < max_iterations) {
+      if (var == 2 && check_every <= kResidentSweeps && resident_until_fits(H, W) && rel > tol &&
+          it < max_iterations) {
+        SG_CHECK(sweeps_until<T>((int)H, (int)W, w, m, alpha, reciprocal_beta, omega,
+                                 SweepsUntil{r0, tol, 0.0, (int)check_every, 0, 0, 0}, max_iterations, &it, &sq, s));
+        rel = r0 > 0.0 ? std::sqrt(sq) / r0 : 0.0;
+      }
+      while (std::isfinite(rel) && rel > tol && it < max_iterations) {
         const int64_t n = std::min(check_every, max_iterations - it);
         SG_CHECK((split_sweeps<T, MM>((int)H, (int)W, w, mm, alpha, reciprocal_beta, omega, n, var, s)));
         it += n;
@@ -712,7 +750,16 @@ int sg_rbsor_mixed_solve(int64_t H, int64_t W, void* p, int64_t ld_p, const void
       const double ir0 = std::sqrt(isq0);
       double irel = 1.0, best = 1.0;
       int stalls = 0;
-      while (irel > inner_tol && it < max_iterations) {
+      if (var == 2 && check_every <= kResidentSweeps && resident_until_fits(H, W)) {
+        int64_t n = 0;
+        SG_CHECK(sweeps_until<float>((int)H, (int)W, w, m, 1.0, reciprocal_beta, omega,
+                                     SweepsUntil{ir0, inner_tol, 1.0, (int)check_every, 0, 0, 3}, max_iterations - it,
+                                     &n, &isq, s));
+        it += n;
+        irel = ir0 > 0.0 ? std::sqrt(isq) / ir0 : 0.0;
+        stalls = 3;  // that was the whole inner solve
+      }
+      while (stalls < 3 && irel > inner_tol && it < max_iterations) {
         const int64_t n = std::min(check_every, max_iterations - it);
         SG_CHECK((split_sweeps<float, MM>((int)H, (int)W, w, mm, 1.0, reciprocal_beta, omega, n, var, s)));
         it += n;

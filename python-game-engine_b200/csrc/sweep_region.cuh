@@ -228,4 +228,41 @@ __device__ __forceinline__ void res_residual(ResEdges<T>& sh, int& buf, int w, i
   buf ^= 1;
 }
 
+// The thread's share of the residual's sum of squares: rows [r_lo, r_hi) of its columns, each
+// residual rounded as above. The edge rows must have come with res_edges and a barrier.
+template <typename T, int RPT>
+__device__ __forceinline__ void res_edges(ResEdges<T>& sh, int buf, int w, int lane, const T (&e)[RPT][2]) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    sh.bot[buf][w][q][lane] = e[RPT - 1][q];
+    sh.top[buf][w][q][lane] = e[0][q];
+  }
+}
+template <typename T, int RPT>
+__device__ __forceinline__ double res_sumsq(const ResEdges<T>& sh, int buf, int w, int lane, const T (&e)[RPT][2],
+                                            const double (&ab)[RPT][2], const uint32_t* code, double beta, int r_lo,
+                                            int r_hi) {
+  const int wb = w > 0 ? w - 1 : w, wa = w < kResWarps - 1 ? w + 1 : w;
+  double sq = 0.0;
+#pragma unroll
+  for (int r = 0; r < RPT; ++r) {
+    const T fl = __shfl_up_sync(0xffffffffu, e[r][1], 1), fr = __shfl_down_sync(0xffffffffu, e[r][0], 1);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const T c = e[r][q];
+      const uint32_t k = res_code(code, r, q);
+      const T l = pick(k & K_L, q == 0 ? fl : e[r][0], c);
+      const T rt = pick(k & K_R, q == 0 ? e[r][1] : fr, c);
+      const T d = pick(k & K_D, r > 0 ? e[r > 0 ? r - 1 : 0][q] : sh.bot[buf][wb][q][lane], c);
+      const T u = pick(k & K_U, r < RPT - 1 ? e[r < RPT - 1 ? r + 1 : r][q] : sh.top[buf][wa][q][lane], c);
+      T s = l + rt;
+      s = s + d;
+      s = s + u;
+      const T x = (T)(((double)s + ab[r][q]) - beta * (double)c);
+      if (r >= r_lo && r < r_hi) sq += pick(k & K_FLUID, (double)x * (double)x, 0.0);
+    }
+  }
+  return sq;
+}
+
 }  // namespace sg

@@ -53,6 +53,11 @@ struct ResArgs {
   uint64_t* xchg;  // two parities of H x Wx cells, one or two tagged words each; null: one tile
   int64_t ldx;     // cells per row of xchg (even)
   uint32_t tag;    // tag of the launch's first trade; the words hold smaller tags or 0 before it
+  // sweeps to a tolerance: the checks' sums, two parities of a block's two words, and the outcome
+  double beta;
+  SweepsUntil u;
+  uint64_t* sums;
+  SweepsReached* reached;
 };
 
 // A trade moves tagged words: 32 bits of a value beside the 32-bit number of the trade, so the
@@ -98,11 +103,17 @@ __device__ __forceinline__ bool trade_get(const uint64_t* x, int64_t o, double (
   return ok;
 }
 
-template <typename T, bool SOR, bool SPLIT, int RPT>
+// UNTIL: to a tolerance (SweepsUntil) instead of a.sweeps. A check comes right after a trade, when
+// the cells beside the block's own are current: each block sums its own residuals, publishes the
+// sum as a trade does its cells, and adds up all blocks' sums in the same order, so all take the
+// same decision. 512^2 float64, 100 sweeps a check: 168 us a check with a launch for the sweeps,
+// two for the sum and a host read, 135 in one launch.
+template <typename T, bool SOR, bool SPLIT, int RPT, bool UNTIL>
 __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid_constant__ ResArgs<T> a) {
   constexpr int RR = kResWarps * RPT;
   __shared__ ResEdges<T> sh;
   __shared__ int s_lost;
+  __shared__ double s_sq;
   const int H = a.H, W = a.W;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int r0 = blockIdx.y * (RR - 2 * kHalo), c0 = blockIdx.x * kResOwnCols;
@@ -147,6 +158,9 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
 
   const bool many = gridDim.x * gridDim.y > 1;
   int left = SOR ? 2 * a.sweeps : a.sweeps;
+  int done = 0, stalls = a.u.stalls, par = 0;
+  double best = a.u.best;
+  if (UNTIL) left = 2 * min(a.u.check_every, a.u.max_sweeps);
   int buf = 0;
   uint32_t tag = a.tag;
   bool traded = !many, lost = false;
@@ -155,7 +169,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
     res_sweeps<T, SOR, RPT>(sh, buf, w, lane, e, ab, code, plain, edge0, edge1, rb, omega, keep, n);
     left -= n;
     // one trade at least: no block may write p before its neighbours have read it
-    if (left <= 0 && traded) break;
+    if (!UNTIL && left <= 0 && traded) break;
     if (many) {
       if (!traded) __syncthreads();  // the whole block has read its region of p
       uint64_t* x = a.xchg + (tag & 1) * parity;
@@ -195,7 +209,52 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
       traded = true;
       ++tag;
     }
-    if (left <= 0) break;
+    if (left > 0) continue;
+    if (!UNTIL) break;
+    const int nblk = gridDim.x * gridDim.y, bid = blockIdx.y * gridDim.x + blockIdx.x, tid = threadIdx.x;
+    res_edges<T, RPT>(sh, buf, w, lane, e);
+    __syncthreads();
+    double sq = res_sumsq<T, RPT>(sh, buf, w, lane, e, ab, code, a.beta, own_col ? oy0 - j : RPT,
+                                  own_col ? oy1 - j : 0);
+    buf ^= 1;
+    sq = block_sum(sq);
+    if (many) {
+      uint64_t* sums = a.sums + (int64_t)par * nblk * 2;
+      par ^= 1;
+      if (tid == 0)
+        st_words(sums + 2 * bid, tagged((uint32_t)__double2loint(sq), tag), tagged((uint32_t)__double2hiint(sq), tag));
+      sq = 0.0;
+      if (tid < nblk) {
+        uint64_t lo, hi;
+        int spins = 0;
+        do {
+          ld_words(sums + 2 * tid, lo, hi);
+        } while (((uint32_t)(lo >> 32) != tag || (uint32_t)(hi >> 32) != tag) && *(volatile int*)&s_lost == 0 &&
+                 ++spins < kTradeSpins);
+        if ((uint32_t)(lo >> 32) != tag || (uint32_t)(hi >> 32) != tag) s_lost = 1;
+        sq = __hiloint2double((int)(uint32_t)hi, (int)(uint32_t)lo);
+      }
+      __syncwarp();
+      sq = block_sum(sq);
+    }
+    if (tid == 0) s_sq = s_lost ? (double)__int_as_float(0x7fc00000) : sq;
+    __syncthreads();
+    sq = s_sq;
+    done += min(a.u.check_every, a.u.max_sweeps - done);
+    const double rel = a.u.r0 > 0.0 ? sqrt(sq) / a.u.r0 : 0.0;
+    bool stop = !(rel > a.u.tol) || !isfinite(rel) || done >= a.u.max_sweeps;
+    if (rel < 0.99 * best) {
+      best = rel;
+      stalls = 0;
+    } else {
+      ++stalls;
+      stop = stop || (a.u.stall_limit > 0 && stalls >= a.u.stall_limit);
+    }
+    if (stop) {
+      if (bid == 0 && tid == 0) *a.reached = SweepsReached{sq, best, done, stalls};
+      break;
+    }
+    left = 2 * min(a.u.check_every, a.u.max_sweeps - done);
   }
   __syncthreads();
   // a wait that gave up (its neighbour never arrived) leaves no usable iterate: say so in p
@@ -233,17 +292,27 @@ int resident_rows(int64_t H, int64_t W) {
   return 0;
 }
 
+// Up to four rows a thread: with eight the check's registers spill in the sweeps (1000 x 901
+// float64, 100 sweeps 874 us, 944 with the check in the launch, about 920 with one from the host).
+bool resident_until_fits(int64_t H, int64_t W) {
+  const int rpt = resident_rows(H, W);
+  return rpt == 2 || rpt == 4;
+}
+
+static int64_t resident_trade_bytes(int64_t elem, int64_t H, int64_t W) {
+  return 2 * H * ((W + 1) & ~(int64_t)1) * 2 * elem;
+}
 int64_t resident_workspace_bytes(int64_t elem, int64_t H, int64_t W) {
   const int rpt = resident_rows(H, W);
   if (rpt == 0) return 0;
-  return 2 * H * ((W + 1) & ~(int64_t)1) * 2 * elem;
+  return resident_trade_bytes(elem, H, W) + (int64_t)sm_count() * 4 * 8 + (int64_t)sizeof(SweepsReached);
 }
 
-template <typename T, bool SOR, bool SPLIT, int RPT>
+template <typename T, bool SOR, bool SPLIT, int RPT, bool UNTIL>
 static int launch_resident_rpt(ResArgs<T>& a, cudaStream_t s) {
   dim3 grid((unsigned)res_tiles(a.W, kResCols, kHalo), (unsigned)res_tiles(a.H, kResWarps * RPT, kHalo));
   void* args[] = {&a};
-  cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_sweeps_resident<T, SOR, SPLIT, RPT>, grid,
+  cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_sweeps_resident<T, SOR, SPLIT, RPT, UNTIL>, grid,
                                               dim3(kResThreads), args, 0, s);
   note_launch();
   return e == cudaSuccess ? SG_OK : fail(SG_ERR_CUDA, "resident sweeps: %s", cudaGetErrorString(e));
@@ -261,12 +330,13 @@ int resident_sweeps(int sor, int split, int H, int W, T* p, T* p1, int64_t ldp, 
   const int rpt = resident_rows(H, W);
   if (rpt == 0) return fail(SG_ERR_CAPACITY, "%d x %d cells do not fit the resident sweeps", H, W);
   if (sweeps <= 0) return SG_OK;
-  ResArgs<T> a{H, W, p, p1, ldp, b, b1, ldb, m, alpha, rb, omega, sweeps, from_zero, (uint64_t*)xchg, (W + 1) & ~1, tag};
+  ResArgs<T> a{H, W, p, p1, ldp, b, b1, ldb, m, alpha, rb, omega, sweeps, from_zero, (uint64_t*)xchg, (W + 1) & ~1, tag,
+               0.0, SweepsUntil{}, nullptr, nullptr};
   auto go = [&](auto SOR_, auto SPLIT_) {
     constexpr bool S = decltype(SOR_)::value, P = decltype(SPLIT_)::value;
-    if (rpt == 2) return launch_resident_rpt<T, S, P, 2>(a, s);
-    if (rpt == 4) return launch_resident_rpt<T, S, P, 4>(a, s);
-    return launch_resident_rpt<T, S, P, 8>(a, s);
+    if (rpt == 2) return launch_resident_rpt<T, S, P, 2, false>(a, s);
+    if (rpt == 4) return launch_resident_rpt<T, S, P, 4, false>(a, s);
+    return launch_resident_rpt<T, S, P, 8, false>(a, s);
   };
   if (!sor) return go(std::false_type{}, std::false_type{});
   return split ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
@@ -276,6 +346,29 @@ template int resident_sweeps<float>(int, int, int, int, float*, float*, int64_t,
 template int resident_sweeps<double>(int, int, int, int, double*, double*, int64_t, const double*, const double*,
                                      int64_t, const Masks&, double, double, double, int, bool, void*, uint32_t,
                                      cudaStream_t);
+
+template <typename T>
+int resident_sweeps_until(int H, int W, T* p0, T* p1, int64_t ldp, const T* b0, const T* b1, int64_t ldb,
+                          const Masks& m, double alpha, double rb, double beta, double omega, const SweepsUntil& u,
+                          void* xchg, uint32_t tag, SweepsReached* reached, cudaStream_t s) {
+  const int rpt = resident_rows(H, W);
+  if (!resident_until_fits(H, W) || u.max_sweeps <= 0 || u.check_every <= 0)
+    return fail(SG_ERR_CAPACITY, "%d x %d cells do not fit the resident sweeps", H, W);
+  uint64_t* sums = (uint64_t*)((char*)xchg + resident_trade_bytes(sizeof(T), H, W));
+  ResArgs<T> a{H, W, p0, p1, ldp, b0, b1, ldb, m, alpha, rb, omega, 0, 0, (uint64_t*)xchg, (W + 1) & ~1, tag,
+               beta, u, sums, (SweepsReached*)(sums + (int64_t)sm_count() * 4)};
+  SG_CHECK(rpt == 2 ? (launch_resident_rpt<T, true, true, 2, true>(a, s))
+                    : (launch_resident_rpt<T, true, true, 4, true>(a, s)));
+  cudaError_t e = cudaMemcpyAsync(reached, a.reached, sizeof(*reached), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  return e == cudaSuccess ? SG_OK : fail(SG_ERR_CUDA, "resident sweeps: %s", cudaGetErrorString(e));
+}
+template int resident_sweeps_until<float>(int, int, float*, float*, int64_t, const float*, const float*, int64_t,
+                                          const Masks&, double, double, double, double, const SweepsUntil&, void*,
+                                          uint32_t, SweepsReached*, cudaStream_t);
+template int resident_sweeps_until<double>(int, int, double*, double*, int64_t, const double*, const double*, int64_t,
+                                           const Masks&, double, double, double, double, const SweepsUntil&, void*,
+                                           uint32_t, SweepsReached*, cudaStream_t);
 
 }  // namespace sg
 

@@ -39,6 +39,24 @@ int resident_sweeps(int sor, int split, int H, int W, T* p, T* p1, int64_t ldp, 
                     const Masks& m, double alpha, double rb, double omega, int sweeps, bool from_zero, void* xchg,
                     uint32_t tag, cudaStream_t s);
 
+// Red-black SOR sweeps of the colour planes p0, p1 until the residual's norm over r0 is at most
+// tol: checked after every check_every sweeps, at most max_sweeps of them (a multiple of
+// check_every, or fewer). best, stalls, stall_limit: also stops when stall_limit checks in a row
+// gained less than 1 % on the best one (0: never).
+struct SweepsUntil {
+  double r0, tol, best;
+  int check_every, max_sweeps, stalls, stall_limit;
+};
+struct SweepsReached {
+  double sq, best;  // the last check's sum of squares
+  int64_t sweeps, stalls;
+};
+bool resident_until_fits(int64_t H, int64_t W);
+template <typename T>
+int resident_sweeps_until(int H, int W, T* p0, T* p1, int64_t ldp, const T* b0, const T* b1, int64_t ldb,
+                          const Masks& m, double alpha, double rb, double beta, double omega, const SweepsUntil& u,
+                          void* xchg, uint32_t tag, SweepsReached* reached, cudaStream_t s);
+
 // SMs of the current device (0: unknown).
 int sm_count();
 

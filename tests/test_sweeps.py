@@ -136,3 +136,26 @@ def test_gauss_seidel_chain_equals_one_block(dtype, shape, kind, iters):
     if n:
         rc = lib.sg_gauss_seidel_sweeps(code, H, W, got.data_ptr(), W + 5, *args, ws.data_ptr(), n - 1, L.stream_ptr())
         assert rc == L.SG_ERR_ARG
+
+
+@pytest.mark.parametrize("precision", ["native64", "native32", "mixed"])
+@pytest.mark.parametrize("shape,kind,check,most", [((40, 60), "open", 7, 60), ((97, 161), "planes", 10, 95),
+                                                   ((300, 310), "ring", 25, 400), ((1000, 901), "open", 3, 9)])
+def test_sweeps_to_a_tolerance_equal_checked_launches(precision, shape, kind, check, most):
+    """All checks in one launch against a launch per half sweep and a host check: the sweeps made, the iterate."""
+    H, W = shape
+    npdt = np.float64 if precision == "native64" else np.float32
+    p0, div, fmu, fmv = _case(H, W, npdt, kind, 5 * H + W)
+    mu, mv = (sg.OPEN_BOX,) * 2 if kind == "open" else ((sg.RING_BOX,) * 2 if kind == "ring" else (dev(fmu), dev(fmv)))
+    out = []
+    for variant in (-1, 0):
+        for tol in (0.3, 1e-9):
+            s = sg.solvers.SORToleranceSolver()
+            p = dev(p0)
+            s(p, dev(div), mu, mv, 1.0, 1.0 / W, 0.5 / W, omega=1.7, tol=tol, max_iterations=most, check_every=check,
+              variant=variant, precision="mixed" if precision == "mixed" else "native")
+            out.append((s.last_iterations, s.last_refinements, s.converged, s.last_relres, p))
+    for a, b in zip(out[:2], out[2:]):
+        assert a[:3] == b[:3]
+        assert a[3] == pytest.approx(b[3], rel=1e-12)
+        assert torch.equal(a[4], b[4])

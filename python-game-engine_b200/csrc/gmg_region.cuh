@@ -18,11 +18,13 @@
 //
 // What bounds them: these levels sit in L2 and a launch is a few microseconds of latency
 // (load, one barrier chain per half sweep, store), so what counts is the number of dependent
-// launches and the length of one warp's instruction stream. Measured, us: a 421 x 300 mixed
-// cycle around obstacles (5 levels of half-sweep launches, 55 in all, before) 117 -> 46; a 512^2
-// float64 cycle (4 levels of 16 x 16 shared-memory tiles and a 16^2 tail before) 71 -> 63; the
-// tail from 64^2 down 18.8 in float32, 22.8 in float64, for 27.2 as two tiled levels and a
-// 16^2 tail.
+// launches and the length of one warp's instruction stream. Edge tests are selects: as branches
+// they parted the edge lanes from the rest of every warp (tail 18.8 and 22.8 us in float32 and
+// float64, pre / post 3.6 / 3.4). Measured, us: a 421 x 300 mixed cycle around obstacles (5
+// levels of half-sweep launches, 55 in all, before) 117 -> 36; a 512^2 float64 cycle (4 levels of
+// 16 x 16 shared-memory tiles and a 16^2 tail before) 71 -> 59; pre and post of a level 3.1 and
+// 3.1 in float32, 3.8 and 3.8 in float64 (5.1 and 3.8 on the tiles); the tail from 64^2 down 15.2
+// in float32, 20.7 in float64, for 27.2 as two tiled levels and a 16^2 tail.
 #pragma once
 
 // Bits 5..7 of a cell's code, for its transfer to the next coarser level: that the coarse

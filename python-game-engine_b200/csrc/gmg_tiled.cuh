@@ -1,5 +1,5 @@
-// Fused tiled level kernels of the convergent multigrid (included by gmg.cu and batch.cu
-// inside namespace sg; uses w1 and rcp_open of gmg_weights.cuh).
+// Fused tiled level bodies of the convergent multigrid, for the batch's deep levels (included by
+// batch.cu inside namespace sg; uses w1 and rcp_open of gmg_weights.cuh).
 //
 // For open-box levels (every cell fluid, every interior face open) one launch runs a whole
 // side of a cycle on a tile of fine cells held in shared memory (64 x 32 on large levels,

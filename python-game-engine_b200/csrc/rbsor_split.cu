@@ -17,6 +17,8 @@
 //                       per half sweep is staged in shared memory (split planes), swept
 //                       there with the valid region shrinking by one cell per half sweep,
 //                       and the tile's own cells are written to the other state buffer
+//   (k_sweeps_resident, sweeps.cu: all sweeps of a call, and those to a tolerance with their
+//   checks, in one launch, where the grid fits on the chip)
 //   k_rbsor_split_sumsq / k_sumsq_finalize  deterministic sum of squares of the reference
 //                       residual (residual.py:39-40) over the split planes
 //   k_mixed_residual, k_add_correction, k_widen, k_narrow  float64 iterative refinement

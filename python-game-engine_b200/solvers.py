@@ -275,8 +275,9 @@ class SORToleranceSolver:
     (red_black_sor_gauss_seidel.py:8-27) bit for bit; the tolerance loop has no reference
     counterpart (the reference runs a fixed sweep count). ``variant``: 1 sweeps
     shared-memory tiles up to four sweeps per launch, 0 launches one streaming kernel per
-    half sweep, -1 (default) picks the tiles for grids that sit in L2 and the streaming
-    kernel above.
+    half sweep, -1 (default) keeps the iterate in registers for the whole solve where the grid
+    fits on the chip, else picks the tiles for grids that sit in L2 and the streaming kernel
+    above.
 
     ``precision="mixed"`` (float32 fields): float64 iterative refinement around float32
     sweeps (``sg_rbsor_mixed_solve``), which reaches tolerances below float32's residual

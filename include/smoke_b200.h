@@ -357,8 +357,9 @@ int sg_mg_prolong(int dtype, int64_t Hc, int64_t Wc, const void* coarse, int64_t
  * coarsest_sweeps on the last level, red-black SOR (sor = 1) or Jacobi, in two launches per
  * level and cycle; every value equals the separate kernels'. Level k: extents, mask planes
  * (H x (W + 1) and (H + 1) x W bytes, contiguous), their cell codes (sg_mg_codes, sg_mg_codes_bytes
- * bytes, made once per mask), alpha(2^k h) and the SOR factor. from_zero (cycles >= 1): p is 0
- * and not read. Workspace
+ * bytes, made once per hierarchy), alpha(2^k h) and the SOR factor. The sweeps of level 0 follow its
+ * planes as they are at the call; which of its cells the residual and the transfers count as fluid
+ * is what its codes say. from_zero (cycles >= 1): p is 0 and not read. Workspace
  * 256-byte aligned; sg_mg_vcycles_workspace_bytes is 0, and the call returns SG_ERR_CAPACITY,
  * for more than 4 SOR or 8 Jacobi sweeps a side or a coarsest level too large for the chip. */
 typedef struct {

@@ -196,11 +196,12 @@ __device__ __forceinline__ bool res_is_plain(uint32_t k, int ii, int W) {
   return k == (K_ALL & ~(ii == 0 ? (uint32_t)K_L : 0u) & ~(ii == W - 1 ? (uint32_t)K_R : 0u));
 }
 
-// Residual of every cell of the thread (residual.py:39-40; 0 off the fluid).
+// Residual of every cell of the thread (residual.py:39-40; 0 off the fluid). cells: bit
+// 2 r + q, whether the cell is fluid there.
 template <typename T, int RPT, bool PART = false>
 __device__ __forceinline__ void res_residual(ResEdges<T>& sh, int& buf, int w, int lane, const T (&e)[RPT][2],
-                                             const double (&ab)[RPT][2], const uint32_t* code, double beta,
-                                             T (&res)[RPT][2], int threads = 0) {
+                                             const double (&ab)[RPT][2], const uint32_t* code, uint32_t cells,
+                                             double beta, T (&res)[RPT][2], int threads = 0) {
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
     sh.bot[buf][w][q][lane] = e[RPT - 1][q];
@@ -222,7 +223,7 @@ __device__ __forceinline__ void res_residual(ResEdges<T>& sh, int& buf, int w, i
       T s = l + rt;
       s = s + d;
       s = s + u;
-      res[r][q] = pick(k & K_FLUID, (T)(((double)s + ab[r][q]) - beta * (double)c), (T)0);
+      res[r][q] = pick(cells >> (2 * r + q) & 1, (T)(((double)s + ab[r][q]) - beta * (double)c), (T)0);
     }
   }
   buf ^= 1;

@@ -1,5 +1,6 @@
 // The reference's V-cycles (multigrid/solver.py:94-176) in two launches per level and cycle.
 //
+//   k_mg_codes level 0's cell codes from the caller's planes, once a call
 //   k_mg_down  smoothing sweeps, the residual, its mean over fluid children divided by
 //              alpha(2h) as the next level's rhs
 //   k_mg_up    bilinear prolongation added to the pressure, smoothing sweeps
@@ -42,7 +43,7 @@ struct MgLevelArgs {
   int64_t ldout;
   const T* b;
   int64_t ldb;
-  const uint8_t* code;  // cell codes, row stride W rounded up to even
+  const uint8_t* code;  // cell codes (k_mg_codes)
   double alpha, omega, rb, beta;
   int n;          // half sweeps (SOR) or sweeps (Jacobi) a side
   int halo;       // even, at least n, or n + 1 where the residual is formed too
@@ -51,11 +52,20 @@ struct MgLevelArgs {
   T divisor;      // down: alpha(2h)
 };
 
-// Codes of the cell pair (j, i), (j, i + 1), i even: ten bits (0 off the grid).
-__device__ __forceinline__ uint32_t mg_codes(const uint8_t* code, int H, int W, int j, int i) {
+// A level's code bytes, row stride W rounded up to even: the K_ bits of the faces, and K_CELL,
+// that the cell is fluid in the hierarchy. The sweeps go by the faces, the residual and the
+// transfers by the hierarchy's cells, as the separate kernels do with is_fluid; the two differ on
+// the fine level where the caller has edited its planes since the hierarchy was built.
+enum : uint32_t { K_CELL = 32 };
+
+// Codes of the cell pair (j, i), (j, i + 1), i even: ten bits (0 off the grid). cells: their
+// K_CELL bits, from bit 2 r on.
+__device__ __forceinline__ uint32_t mg_codes(const uint8_t* code, int H, int W, int j, int i, int r,
+                                             uint32_t& cells) {
   if (j >= H || i >= W) return 0;
   const uchar2 c = *reinterpret_cast<const uchar2*>(code + (int64_t)j * ((W + 1) & ~1) + i);
-  return (uint32_t)c.x | ((uint32_t)c.y << 5);
+  cells |= (((uint32_t)c.x >> 5) | (((uint32_t)c.y >> 5) << 1)) << (2 * r);
+  return (c.x & K_ALL) | ((c.y & K_ALL) << 5);
 }
 
 // Loads the region's cells: values (pin, or 0), alpha * rhs and codes; the block's own range.
@@ -65,7 +75,7 @@ struct MgRegion {
   bool own_col, plain, edge0, edge1;
   T e[RPT][2];
   double ab[RPT][2];
-  uint32_t code[(RPT + 1) / 2];
+  uint32_t code[(RPT + 1) / 2], cells;
 
   __device__ __forceinline__ void load(const MgLevelArgs<T>& a) {
     constexpr int RR = kResWarps * RPT;
@@ -80,11 +90,12 @@ struct MgRegion {
               i < (blockIdx.x == gridDim.x - 1 ? a.W : c0 + kResCols - a.halo);
 #pragma unroll
     for (int r = 0; r < (RPT + 1) / 2; ++r) code[r] = 0;
+    cells = 0;
     bool all = i + 1 < a.W;
 #pragma unroll
     for (int r = 0; r < RPT; ++r) {
       const int jj = j + r;
-      const uint32_t kk = mg_codes(a.code, a.H, a.W, jj, i);
+      const uint32_t kk = mg_codes(a.code, a.H, a.W, jj, i, r, cells);
       all = all && res_is_plain(kk & K_ALL, i, a.W) && res_is_plain(kk >> 5, i + 1, a.W);
       code[r >> 1] |= kk << (10 * (r & 1));
 #pragma unroll
@@ -115,17 +126,13 @@ struct MgRegion {
 
 // multigrid/transfer.py:5-36 for the 2 x 2 cells at rows r, r + 1 of the thread
 template <typename T, int RPT>
-__device__ __forceinline__ T mg_restrict(const T (&res)[RPT][2], const uint32_t* code, int r, T divisor) {
+__device__ __forceinline__ T mg_restrict(const T (&res)[RPT][2], uint32_t cells, int r, T divisor) {
   double total = 0.0;  // res is 0 off the fluid
-  int count = 0;
 #pragma unroll
   for (int d = 0; d < 2; ++d)
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      total += (double)res[r + d][q];
-      count += (res_code(code, r + d, q) >> 4) & 1;
-    }
-  static_assert(K_FLUID == 16, "bit 4");
+    for (int q = 0; q < 2; ++q) total += (double)res[r + d][q];
+  const int count = __popc((cells >> (2 * r)) & 15);
   // a division by 4, 2 or 1 is the multiplication by its exact reciprocal
   const double by = count == 4 ? 0.25 : (count == 2 ? 0.5 : 1.0);
   const double mean = count == 3 ? total / 3.0 : total * by;
@@ -147,13 +154,19 @@ __device__ __forceinline__ T mg_prolong(const T* c, int64_t ldc, int Hc, int Wc,
   return (T)(c0 + (c1 - c0) * ty);
 }
 
-// Codes of a level from its face masks.
-__global__ void k_mg_codes(int H, int W, Masks m, uint8_t* __restrict__ code, int ld) {
+// Codes of a level from its face masks; K_CELL from the codes `built` at the hierarchy's making
+// (null: from the masks).
+__global__ void k_mg_codes(int H, int W, Masks m, const uint8_t* __restrict__ built, uint8_t* __restrict__ code,
+                           int ld) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= ld || j >= H) return;
-  code[(int64_t)j * ld + i] = i < W ? (uint8_t)cell_code(m, H, W, j, i) : 0;
+  const int64_t o = (int64_t)j * ld + i;
+  const uint32_t c = i < W ? cell_code(m, H, W, j, i) : 0;
+  const uint32_t cell = built ? built[o] & K_CELL : (c & K_FLUID) << 1;
+  code[o] = (uint8_t)(c | cell);
 }
+static_assert(K_CELL == K_FLUID << 1, "the next bit");
 
 template <typename T, bool SOR>
 __global__ void __launch_bounds__(kResThreads) k_mg_down(const __grid_constant__ MgLevelArgs<T> a) {
@@ -166,13 +179,13 @@ __global__ void __launch_bounds__(kResThreads) k_mg_down(const __grid_constant__
                           1.0 - a.omega, a.n);
   g.store(a);
   T res[RPT][2];
-  res_residual<T, RPT>(sh, buf, g.w, g.lane, g.e, g.ab, g.code, a.beta, res);
+  res_residual<T, RPT>(sh, buf, g.w, g.lane, g.e, g.ab, g.code, g.cells, a.beta, res);
   if (!g.own_col) return;
 #pragma unroll
   for (int r = 0; r < RPT; r += 2) {
     const int jj = g.j + r;
     if (jj < g.oy0 || jj >= g.oy1 || !SG_IN_BOUNDS(jj + 1 < a.H && g.i + 1 < a.W)) continue;
-    a.bc[(int64_t)(jj >> 1) * (a.W >> 1) + (g.i >> 1)] = mg_restrict<T, RPT>(res, g.code, r, a.divisor);
+    a.bc[(int64_t)(jj >> 1) * (a.W >> 1) + (g.i >> 1)] = mg_restrict<T, RPT>(res, g.cells, r, a.divisor);
   }
 }
 
@@ -186,7 +199,7 @@ __global__ void __launch_bounds__(kResThreads) k_mg_up(const __grid_constant__ M
   for (int r = 0; r < RPT; ++r)
 #pragma unroll
     for (int q = 0; q < 2; ++q)
-      if (res_code(g.code, r, q) & K_FLUID)
+      if (g.cells >> (2 * r + q) & 1)
         g.e[r][q] = g.e[r][q] + mg_prolong(a.ec, a.W >> 1, a.H >> 1, a.W >> 1, g.j + r, g.i + q);
   int buf = 0;
   res_sweeps<T, SOR, RPT>(sh, buf, g.w, g.lane, g.e, g.ab, g.code, g.plain, g.edge0, g.edge1, a.rb, a.omega,
@@ -232,14 +245,14 @@ __device__ __forceinline__ void mg_tail_visit(const MgTailArgs<T>& a, const MgTa
   int buf = 0;
   T e[RPT][2];
   double ab[RPT][2];
-  uint32_t code[(RPT + 1) / 2];
+  uint32_t code[(RPT + 1) / 2], cells = 0;
 #pragma unroll
   for (int r = 0; r < (RPT + 1) / 2; ++r) code[r] = 0;
   bool all = i + 1 < W;
 #pragma unroll
   for (int r = 0; r < RPT; ++r) {
     const int jj = j + r;
-    const uint32_t kk = mg_codes(t.code + a.off_code[l], H, W, jj, i);
+    const uint32_t kk = mg_codes(t.code + a.off_code[l], H, W, jj, i, r, cells);
     all = all && res_is_plain(kk & K_ALL, i, W) && res_is_plain(kk >> 5, i + 1, W);
     code[r >> 1] |= kk << (10 * (r & 1));
 #pragma unroll
@@ -261,7 +274,7 @@ __device__ __forceinline__ void mg_tail_visit(const MgTailArgs<T>& a, const MgTa
     for (int r = 0; r < RPT; ++r)
 #pragma unroll
       for (int q = 0; q < 2; ++q)
-        e[r][q] = e[r][q] + pick(res_code(code, r, q) & K_FLUID,
+        e[r][q] = e[r][q] + pick(cells >> (2 * r + q) & 1,
                                  mg_prolong((const T*)t.p + a.off[l + 1], W >> 1, H >> 1, W >> 1, j + r, i + q), (T)0);
   }
   const bool plain = __all_sync(0xffffffffu, all);
@@ -282,11 +295,11 @@ __device__ __forceinline__ void mg_tail_visit(const MgTailArgs<T>& a, const MgTa
     }
   if (up || coarsest) return;
   T res[RPT][2];
-  res_residual<T, RPT, true>(sh, buf, w, lane, e, ab, code, a.beta, res, threads);
+  res_residual<T, RPT, true>(sh, buf, w, lane, e, ab, code, cells, a.beta, res, threads);
 #pragma unroll
   for (int r = 0; r < RPT; r += 2)
     if (j + r + 1 < H && i + 1 < W)
-      t.b[a.off[l + 1] + ((j + r) >> 1) * (W >> 1) + (i >> 1)] = mg_restrict<T, RPT>(res, code, r, (T)a.alpha[l + 1]);
+      t.b[a.off[l + 1] + ((j + r) >> 1) * (W >> 1) + (i >> 1)] = mg_restrict<T, RPT>(res, cells, r, (T)a.alpha[l + 1]);
 }
 
 // The warps whose rows lie beyond a level wait for the others at the visit's end, and levels
@@ -325,8 +338,10 @@ __global__ void __launch_bounds__(kResThreads) k_mg_tail(const __grid_constant__
 struct MgPlan {  // offsets (bytes) of the levels' arrays in the workspace
   int tail;      // first level of the tail, n when the coarsest runs as resident sweeps
   int64_t pa[kMgMaxLevels], pb[kMgMaxLevels], rhs[kMgMaxLevels];
-  int64_t xchg, bytes;
+  int64_t code, xchg, bytes;  // code: level 0's
 };
+
+static int64_t code_pitch(int64_t W) { return (W + 1) & ~(int64_t)1; }
 
 // false: a level or sweep count these kernels do not take
 static bool mg_plan(int64_t elem, int n, const sg_mg_level* lv, int sor, int sweeps, MgPlan* p) {
@@ -348,6 +363,7 @@ static bool mg_plan(int64_t elem, int n, const sg_mg_level* lv, int sor, int swe
     p->rhs[k] = k > 0 ? take(bytes) : 0;
     p->pb[k] = k + 1 < n ? take(bytes) : 0;
   }
+  p->code = take(lv[0].H * code_pitch(lv[0].W));
   p->xchg = off;
   if (p->tail == n) {
     const int64_t x = resident_workspace_bytes(elem, lv[n - 1].H, lv[n - 1].W);
@@ -363,19 +379,24 @@ static Masks level_masks(const sg_mg_level& L) {
                     L.W, nullptr, 0);
 }
 
-static int64_t code_pitch(int64_t W) { return (W + 1) & ~(int64_t)1; }
-
 template <typename T, bool SOR>
 static int mg_vcycles(int n, const sg_mg_level* lv, const MgPlan& P, T* p, int64_t ldp, const T* div, int64_t ldd,
                       double rb, int cycles, int sweeps, int coarsest, bool from_zero, char* ws, cudaStream_t s) {
   const int half = SOR ? 2 * sweeps : sweeps;
   const double beta = 1.0 / rb;
   auto at = [&](int64_t o) { return (T*)(ws + o); };
+  // level 0's codes of this call: its planes are the caller's, who may edit them between calls
+  uint8_t* const code0 = (uint8_t*)(ws + P.code);
+  if (cycles > 0 && (n > 1 || P.tail < n)) {
+    const int ld = (int)code_pitch(lv[0].W);
+    SG_LAUNCH(k_mg_codes<<<grid2d(ld, lv[0].H), block2d(), 0, s>>>((int)lv[0].H, (int)lv[0].W, level_masks(lv[0]),
+                                                                  (const uint8_t*)lv[0].code, code0, ld));
+  }
   auto level = [&](int k, bool down, bool zero) {
     MgLevelArgs<T> a{};
     a.H = (int)lv[k].H;
     a.W = (int)lv[k].W;
-    a.code = (const uint8_t*)lv[k].code;
+    a.code = k == 0 ? code0 : (const uint8_t*)lv[k].code;
     a.alpha = lv[k].alpha;
     a.omega = lv[k].omega;
     a.rb = rb;
@@ -417,7 +438,7 @@ static int mg_vcycles(int n, const sg_mg_level* lv, const MgPlan& P, T* p, int64
       t.W[q] = (int)L.W;
       t.off[q] = t.cells;
       t.cells += (int)(L.H * L.W);
-      t.code[q] = (const uint8_t*)L.code;
+      t.code[q] = P.tail + q == 0 ? code0 : (const uint8_t*)L.code;
       t.off_code[q] = codes;
       codes += (int)(L.H * code_pitch(L.W));
       t.alpha[q] = L.alpha;
@@ -478,7 +499,7 @@ int sg_mg_codes(int64_t H, int64_t W, const uint8_t* fmu, const uint8_t* fmv, ui
   SG_REQUIRE(H >= 1 && W >= 1 && H <= (1 << 15) && W <= (1 << 15) && fmu && fmv && code, "bad grid or planes");
   const Masks m = make_masks(SG_MASK_PLANES, H, W, fmu, W + 1, fmv, W, nullptr, 0);
   const int ld = (int)code_pitch(W);
-  SG_LAUNCH(k_mg_codes<<<grid2d(ld, H), block2d(), 0, as_stream(stream)>>>((int)H, (int)W, m, code, ld));
+  SG_LAUNCH(k_mg_codes<<<grid2d(ld, H), block2d(), 0, as_stream(stream)>>>((int)H, (int)W, m, nullptr, code, ld));
   return check_launch("sg_mg_codes");
 }
 

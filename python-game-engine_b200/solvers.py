@@ -138,6 +138,19 @@ def gauss_seidel_pressure_solver(pressure, divergence, face_mask_u, face_mask_v,
            ws.data_ptr() if nbytes else None, nbytes, L.stream_ptr())
 
 
+def _rows_apart(t):
+    """Whether the rows of a 2-D field are unit-stride and do not overlap."""
+    H, W = t.shape
+    return (W == 1 or t.stride(1) == 1) and (H == 1 or t.stride(0) >= W)
+
+
+def _share_memory(a, b):
+    """Whether the address ranges of two 2-D fields of ascending rows overlap."""
+    (a0, a1), (b0, b1) = ((t.data_ptr(), t.data_ptr() + t.element_size() * ((t.shape[0] - 1) * t.stride(0) + t.shape[1]))
+                          for t in (a, b))
+    return a0 < b1 and b0 < a1
+
+
 class MultigridSolver:
     """The reference's V-cycle (multigrid/solver.py:16-176) on CUDA kernels.
 
@@ -162,6 +175,8 @@ class MultigridSolver:
             return
         fmu = materialize_mask(fmu, H, W, "u", device)
         fmv = materialize_mask(fmv, H, W, "v", device)
+        L.mask_plane(fmu, "face_mask_u", (H, W + 1))  # refuses what the kernels cannot read
+        L.mask_plane(fmv, "face_mask_v", (H + 1, W))
         fl = is_fluid_from_faces(fmu.bool(), fmv.bool())
         solid = ~fl
         levels = [dict(is_fluid=fl, fmu=fmu, fmv=fmv, solid=solid)]
@@ -178,8 +193,8 @@ class MultigridSolver:
         for lv in levels:
             h, w = lv["is_fluid"].shape
             lv["code"] = torch.empty(L.load().sg_mg_codes_bytes(h, w), dtype=torch.uint8, device=device)
-            L.call("sg_mg_codes", h, w, lv["fmu"].data_ptr(), lv["fmv"].data_ptr(), lv["code"].data_ptr(),
-                   L.stream_ptr())
+            L.call("sg_mg_codes", h, w, lv["fmu"].contiguous().data_ptr(), lv["fmv"].contiguous().data_ptr(),
+                   lv["code"].data_ptr(), L.stream_ptr())
         self.levels = levels
         self.buffers = [{k: torch.zeros(lv["is_fluid"].shape, dtype=dtype, device=device)
                          for k in ("pressure", "residual", "rhs")} for lv in levels]
@@ -211,18 +226,26 @@ class MultigridSolver:
 
     def _fused(self, smoother, pressure, divergence, rho, h, dt, cycles, nu, nu_c, from_zero):
         """The cycles in two launches per level (``sg_mg_vcycles``: the same values); False for
-        what that does not take: another smoother, fields it cannot read in place, more sweeps
-        a side than a tile's halo, a coarsest level too large for the chip."""
+        what that does not take: another smoother, fields it cannot read in place (other types or
+        strides, rows that share memory), mask planes in wider rows, more sweeps a side than a
+        tile's halo, a coarsest level too large for the chip."""
         if smoother is jacobi_pressure_solver:
             sor = 0
         elif smoother is red_black_sor_gauss_seidel_pressure_solver:
             sor = 1
         else:
             return False
-        if from_zero and cycles < 1:
+        if cycles < 1:
             return False
-        if (divergence.dtype != pressure.dtype or divergence.shape != pressure.shape or pressure.stride(1) != 1
-                or divergence.stride(1) != 1 or divergence.device != pressure.device):
+        H, W = pressure.shape
+        if (divergence.dtype != pressure.dtype or divergence.shape != pressure.shape
+                or divergence.device != pressure.device or not _rows_apart(pressure) or not _rows_apart(divergence)
+                or _share_memory(pressure, divergence)):
+            return False
+        # the caller's own planes: the level table has no row strides
+        fine = self.levels[0]
+        if not (fine["fmu"].is_contiguous() and fine["fmv"].is_contiguous() and fine["fmu"].shape == (H, W + 1)
+                and fine["fmv"].shape == (H + 1, W)):
             return False
         n = len(self.levels)
         table = (L.MgLevel * n)()
@@ -232,6 +255,8 @@ class MultigridSolver:
             e.H, e.W = H, W
             e.face_mask_u, e.face_mask_v, e.code = (lv[m].data_ptr() for m in ("fmu", "fmv", "code"))
             e.alpha, e.omega = calculate_alpha(h, rho, dt), calculate_optimal_omega(max(H, W))
+            if e.alpha == 0.0:
+                return False
             h *= 2.0
         code = L.dtype_code(pressure)
         nbytes = L.load().sg_mg_vcycles_workspace_bytes(code, n, ctypes.addressof(table), sor, int(nu))

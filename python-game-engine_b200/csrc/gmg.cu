@@ -1183,8 +1183,7 @@ struct sg_gmg_plan {
   // the residual in the precision of p when that differs from the cycle precision
   int fused_ir = 0;
   int64_t off_b2 = 0, off_r64 = 0;
-  // the same on a region fine level: 1 carries the residual likewise; 2 (float32 solves) only
-  // adds the correction to p, and the residual is formed from p afresh
+  // a region fine level: its post kernel adds the correction to p
   int region_ir = 0;
   // cycles per refinement step (classical iterative refinement): with inner >= 2 the body
   // runs `inner` cycles on the cycle-precision correction from zero, then one p += e and one
@@ -1451,36 +1450,30 @@ static dim3 region_grid(const Level& L, int halo) {
 // restriction's reach, rounded up to even.
 static int region_halo(int sweeps, bool residual) { return 2 * sweeps + (residual ? 2 : 0); }
 
-// E0 (nothing for a zero initial guess) -> E1 and the coarse rhs; b_alt: see k_gmg_pre_region
+// E0 (nothing for a zero initial guess) -> E1 and the coarse rhs
 template <typename T>
-static void launch_pre_region(const sg_gmg_plan* p, int k, bool zero_init, T* b_alt, cudaStream_t s) {
+static void launch_pre_region(const sg_gmg_plan* p, int k, bool zero_init, cudaStream_t s) {
   const Level& L = p->levels[k];
   RegionArgs<T> a = region_args<T>(p, k);
   a.e_in = zero_init ? nullptr : ws_ptr<T>(p, L.off_e);
   a.e_out = ws_ptr<T>(p, L.off_e2);
-  a.b_alt = b_alt;
   a.bc = ws_ptr<T>(p, p->levels[k + 1].off_b);
   a.sweeps = p->pre;
   a.halo = region_halo(p->pre, true);
   SG_LAUNCH(k_gmg_pre_region<T><<<region_grid(L, a.halo), kRgThreads, 0, s>>>(a));
 }
 
-// E1 and the coarse correction (the coarse level's E0) -> E0, or the end of a solve's cycle
-template <typename T, typename TP, int FINAL>
-static dim3 launch_post_region(const sg_gmg_plan* p, int k, T* b_alt, cudaStream_t s) {
+// E1 and the coarse correction (the coarse level's E0) -> E0, or (FINAL) added to p
+template <typename T, typename TP, bool FINAL>
+static void launch_post_region(const sg_gmg_plan* p, int k, cudaStream_t s) {
   const Level& L = p->levels[k];
   RegionArgs<T> a = region_args<T>(p, k);
   a.e_in = ws_ptr<T>(p, L.off_e2);
   a.e_out = ws_ptr<T>(p, L.off_e);
-  a.b_alt = b_alt;
   a.ec = ws_ptr<T>(p, p->levels[k + 1].off_e);
   a.sweeps = p->post;
-  a.halo = region_halo(p->post, FINAL == 1);
-  a.r64 = FINAL == 1 && p->off_r64 ? (void*)(p->ws + p->off_r64) : nullptr;
-  a.partial = (double*)(p->ws + p->off_partial);
-  const dim3 g = region_grid(L, a.halo);
-  SG_LAUNCH((k_gmg_post_region<T, TP, FINAL><<<g, kRgThreads, 0, s>>>(a)));
-  return g;
+  a.halo = region_halo(p->post, false);
+  SG_LAUNCH((k_gmg_post_region<T, TP, FINAL><<<region_grid(L, a.halo), kRgThreads, 0, s>>>(a)));
 }
 
 template <typename T, int SW>
@@ -1678,9 +1671,9 @@ static void cycle(const sg_gmg_plan* p, int k, bool zero_init, cudaStream_t s) {
   const int nl = (int)p->levels.size();
   const int reps = (p->cycle == 1 && k + 1 < nl - 1) ? 2 : 1;
   if (p->levels[k].region) {
-    launch_pre_region<T>(p, k, zero_init, nullptr, s);
+    launch_pre_region<T>(p, k, zero_init, s);
     for (int q = 0; q < reps; ++q) cycle<T>(p, k + 1, q == 0, s);
-    launch_post_region<T, T, 0>(p, k, nullptr, s);
+    launch_post_region<T, T, false>(p, k, s);
     return;
   }
   if (p->levels[k].fused) {
@@ -1740,7 +1733,7 @@ static void prologue(const sg_gmg_plan* p, cudaGraphConditionalHandle h, int use
   }
   // from a zero guess the fused fine level carries the residual from here on (b0 / r64), so
   // the FP64 rhs itself is not kept
-  TP* bkeep = (zero_guess && (p->fused_ir || p->region_ir == 1) && p->inner <= 1) ? nullptr : bf;
+  TP* bkeep = (zero_guess && p->fused_ir && p->inner <= 1) ? nullptr : bf;
   // the first cycle of such a solve forms r64 from the divergence itself (FirstCycle), so the
   // prologue does not write it
   SG_LAUNCH(k_gmg_rhs<TD, TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, st, m, bkeep, p->ld_bfine, part,
@@ -1788,19 +1781,11 @@ static void body(const sg_gmg_plan* p, cudaGraphConditionalHandle h, int use_han
   dim3 g = grid_wide(L.W, L.H);
   const int inner = p->inner < 1 ? 1 : p->inner;
   if (p->region_ir && inner == 1) {
-    constexpr bool kCarried = !std::is_same<TP, float>::value;  // region_ir 1
-    TC* b_alt = kCarried ? ws_ptr<TC>(p, p->off_b2) : nullptr;
     const int nl = (int)p->levels.size();
-    launch_pre_region<TC>(p, 0, true, b_alt, s);
+    launch_pre_region<TC>(p, 0, true, s);
     const int reps = (p->cycle == 1 && 1 < nl - 1) ? 2 : 1;
     for (int q = 0; q < reps; ++q) cycle<TC>(p, 1, q == 0, s);
-    if constexpr (kCarried) {
-      const dim3 gr = launch_post_region<TC, TP, 1>(p, 0, b_alt, s);
-      SG_LAUNCH(k_gmg_finalize_rel<<<1, 1024, 0, s>>>(part, (int)(gr.x * gr.y), st, h, use_handle, 1));
-      return;
-    } else {
-      launch_post_region<TC, TP, 2>(p, 0, nullptr, s);
-    }
+    launch_post_region<TC, TP, true>(p, 0, s);
   } else {
     for (int q = 0; q < inner; ++q) cycle<TC>(p, 0, q == 0, s);
     SG_LAUNCH(k_gmg_correct<TP, TC><<<g, block2d(), 0, s>>>(L.H, L.W, st, ws_ptr<TC>(p, L.off_e), L.ld));
@@ -2117,8 +2102,8 @@ int sg_gmg_plan_create(sg_gmg_plan** out, int64_t H, int64_t W, int mask_mode, c
   p->off_bfine = off;
   off = align256(off + p->ld_bfine * p->H * (int64_t)fine);
   p->fused_ir = (p->levels.size() >= 2 && p->tail_start >= 1 && p->levels[0].fused && !small_tiles(p->levels[0])) ? 1 : 0;
-  p->region_ir = p->levels.size() >= 2 && p->levels[0].region ? (precision == SG_GMG_FP32 ? 2 : 1) : 0;
-  if (p->fused_ir || p->region_ir == 1) {
+  p->region_ir = p->levels.size() >= 2 && p->levels[0].region ? 1 : 0;
+  if (p->fused_ir) {
     p->off_b2 = off;
     off = align256(off + p->levels[0].ld * p->H * (int64_t)cyc);
     if (precision == SG_GMG_MIXED) {
@@ -2139,10 +2124,6 @@ int sg_gmg_plan_create(sg_gmg_plan** out, int64_t H, int64_t W, int mask_mode, c
   if (p->fused_ir) {
     dim3 gf = precision == SG_GMG_FP64 ? post_final_grid<double>(p) : post_final_grid<float>(p);
     p->n_partial = std::max(p->n_partial, (int64_t)gf.x * gf.y);
-  }
-  if (p->region_ir == 1) {
-    const dim3 gr = region_grid(p->levels[0], region_halo(p->post, true));
-    p->n_partial = std::max(p->n_partial, (int64_t)gr.x * gr.y);
   }
   p->off_partial = off;
   off = align256(off + p->n_partial * 8);

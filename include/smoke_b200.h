@@ -206,11 +206,22 @@ int sg_build_masks(int64_t H, int64_t W, const uint8_t* solid, int64_t ld_s, uin
  * tiled kernels check their index arithmetic before each access, skip an access that fails
  * and record the source line of the first failure per compilation unit; nothing traps.
  * sg_bounds_check reports the first recorded line (0: none) and its unit (0 operators,
- * 1 gmg, 2 batch, 3 rbsor_split, 4 advect_fast, 5 adjoint, 6 metrics; -1: none) and, with
+ * 1 gmg, 2 batch, 3 rbsor_split, 4 advect_fast, 5 adjoint, 6 metrics, 7 sweeps, 8 vcycle;
+ * -1: none) and, with
  * clear != 0, resets the records. sg_bounds_check_enabled: 1 in that build, 0 otherwise (where
  * sg_bounds_check always reports none). No counterpart in the reference. */
 int sg_bounds_check_enabled(void);
 int sg_bounds_check(unsigned int* first_line, int* unit, int clear);
+
+/* Launches whose blocks trade cells (sg_sweeps_solve, sg_rbsor_tol_solve, sg_rbsor_mixed_solve and
+ * sg_rbsor_split_sweeps on grids that fit the chip, sg_gauss_seidel_sweeps with a workspace, the
+ * coarsest sweeps of sg_mg_vcycles) wait for one another, at most some seconds. What depends on a
+ * wait that ran out is NaN; solves to a tolerance then end with SG_ERR_NONFINITE, the others have
+ * returned before. sg_lost_waits: such waits on the current device since the last call with
+ * clear != 0 (synchronises). sg_bounds_lose_waits (bounds-check build only, for tests): the
+ * blocks of that index give up every wait at once; -1 for none. */
+int sg_lost_waits(int64_t* count, int clear);
+int sg_bounds_lose_waits(int block);
 
 /* ---------------------------------------------------------------- reference solvers */
 
@@ -313,7 +324,8 @@ int sg_rbsor_mixed_solve(int64_t H, int64_t W, void* p, int64_t ld_p, const void
  * workspace (16-byte aligned, sg_sweeps_workspace_bytes; cleared by the call): the cells that
  * neighbouring blocks trade. sg_sweeps_workspace_bytes is 0, and the solve returns
  * SG_ERR_CAPACITY, for grids that do not fit the current device at once. p and div may not
- * overlap. A block whose neighbour never answers gives up after a bounded wait and writes NaN. */
+ * overlap. A block whose neighbour never answers gives up after a bounded wait, and what depends
+ * on it is NaN (sg_lost_waits). */
 int64_t sg_sweeps_workspace_bytes(int dtype, int64_t H, int64_t W);
 int sg_sweeps_solve(int dtype, int sor, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div, int64_t ld_div,
                     int mask_mode, const uint8_t* face_mask_u, int64_t ld_fmu, const uint8_t* face_mask_v,
@@ -330,7 +342,7 @@ int sg_gauss_seidel_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p
 
 /* The same sweeps (the same iterates) split over a chain of blocks that hand their diagonals on
  * through workspace (16-byte aligned, sg_gauss_seidel_workspace_bytes; cleared by the call;
- * null: one block). 0 bytes: the call has no chain form and needs none. */
+ * null: one block), waiting for one another (sg_lost_waits). 0 bytes: the call has no chain form and needs none. */
 int64_t sg_gauss_seidel_workspace_bytes(int dtype, int64_t H, int64_t W, int iterations);
 int sg_gauss_seidel_sweeps(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div,
                            int64_t ld_div, int mask_mode, const uint8_t* fmu, int64_t ld_fmu,

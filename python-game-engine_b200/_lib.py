@@ -129,6 +129,8 @@ SIGNATURES = {
     "sg_gmg_set_inner_cycles": [P, I],
     "sg_field_stats_workspace_bytes": [],
     "sg_field_stats": [I, I64, I64, P, I64, P, P, P],
+    "sg_lost_waits": [ctypes.POINTER(I64), I],
+    "sg_bounds_lose_waits": [I],
     "sg_bounds_check_enabled": [],
     "sg_bounds_check": [ctypes.POINTER(ctypes.c_uint), PI, I],
     "sg_version": [],
@@ -199,6 +201,14 @@ def bounds_check(clear=True):
     line, unit = ctypes.c_uint(0), ctypes.c_int(-1)
     check(load().sg_bounds_check(ctypes.byref(line), ctypes.byref(unit), 1 if clear else 0), "sg_bounds_check")
     return line.value, unit.value
+
+
+def lost_waits(clear=True):
+    """Waits of a launch's blocks for one another that ran out on the current device since the
+    last clear (their solves hold NaN); synchronises."""
+    n = ctypes.c_int64(0)
+    check(load().sg_lost_waits(ctypes.byref(n), 1 if clear else 0), "sg_lost_waits")
+    return n.value
 
 
 def exported_symbols():

@@ -5,6 +5,7 @@
 #include <algorithm>
 
 #include "sweep_region.cuh"
+#include "waits.cuh"
 
 namespace sg {
 
@@ -165,12 +166,14 @@ __device__ __forceinline__ void gs_run(const GsArgs<T>& g, int* s_lost, unsigned
         if (on && !gs_there(q[u].g, (uint32_t)d + 1)) {
           int spins = 0;
           do {
-            if (++spins > kGsSpins) *(volatile int*)s_lost = 1;
+            if (++spins > kGsSpins) give_up_wait(s_lost);
             gs_get(in + slot(d, lc), q[u].g);
           } while (!gs_there(q[u].g, (uint32_t)d + 1) && *(volatile int*)s_lost == 0);
         }
-        // a block that never came leaves no usable iterate: say so in p, down the chain
-        v = gs_there(q[u].g, (uint32_t)d + 1) ? gs_value(q[u].g) : (T)__int_as_float(0x7fc00000);
+        // a block that never came (waits.cuh) leaves no usable iterate: say so in p, down the chain
+        const bool lose = lose_waits(blockIdx.x);
+        if (lose) give_up_wait(s_lost);
+        v = gs_there(q[u].g, (uint32_t)d + 1) && !lose ? gs_value(q[u].g) : (T)__int_as_float(0x7fc00000);
       }
       uint32_t c;
       if (PLANES) {
@@ -223,7 +226,7 @@ __device__ __forceinline__ void gs_run(const GsArgs<T>& g, int* s_lost, unsigned
       const int need = min(t0 + kGsAhead - 2 * (k - 1), D) - kGsRing;  // read before this round's diagonals go out
       int spins = 0;
       while (read < need && *(volatile int*)s_lost == 0) {
-        if (++spins > kGsSpins) *(volatile int*)s_lost = 1;
+        if (++spins > kGsSpins) give_up_wait(s_lost);
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(read) : "l"(credit_out) : "memory");
       }
       __syncwarp();
@@ -370,3 +373,5 @@ template int gauss_seidel_wave<double>(int, int, double*, int64_t, const double*
                                        double, int, void*, bool*, cudaStream_t);
 
 }  // namespace sg
+
+SG_WAITS_ACCESSOR(gauss_seidel)

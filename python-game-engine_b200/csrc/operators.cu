@@ -1004,6 +1004,26 @@ int sg_bounds_line_metrics(unsigned* line, int clear);
 int sg_bounds_line_sweeps(unsigned* line, int clear);
 int sg_bounds_line_vcycle(unsigned* line, int clear);
 
+int sg_lost_waits_sweeps(unsigned* count, int clear);
+int sg_lost_waits_gauss_seidel(unsigned* count, int clear);
+int sg_lose_waits_sweeps(int block);
+int sg_lose_waits_gauss_seidel(int block);
+
+int sg_lost_waits(int64_t* count, int clear) {
+  SG_REQUIRE(count, "null output");
+  unsigned a = 0, b = 0;
+  if (sg_lost_waits_sweeps(&a, clear) != SG_OK || sg_lost_waits_gauss_seidel(&b, clear) != SG_OK)
+    return fail(SG_ERR_CUDA, "sg_lost_waits: %s", cudaGetErrorString(cudaGetLastError()));
+  *count = (int64_t)a + b;
+  return SG_OK;
+}
+
+int sg_bounds_lose_waits(int block) {
+  if (sg_lose_waits_sweeps(block) != SG_OK || sg_lose_waits_gauss_seidel(block) != SG_OK)
+    return fail(SG_ERR_ARG, "only the bounds-check build gives up waits");
+  return SG_OK;
+}
+
 int sg_bounds_check_enabled(void) { return SG_BOUNDS_CHECK; }
 
 int sg_bounds_check(unsigned* first_line, int* unit, int clear) {

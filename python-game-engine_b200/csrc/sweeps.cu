@@ -11,6 +11,7 @@
 
 #include "sweeps.cuh"
 #include "sweep_region.cuh"
+#include "waits.cuh"
 
 namespace sg {
 
@@ -156,6 +157,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
   const double rb = a.rb, omega = a.omega, keep = 1.0 - a.omega;
   const int64_t parity = (int64_t)H * a.ldx * (sizeof(T) / 4);  // words of one parity
 
+  const int bid = blockIdx.y * gridDim.x + blockIdx.x;
   const bool many = gridDim.x * gridDim.y > 1;
   int left = SOR ? 2 * a.sweeps : a.sweeps;
   int done = 0, stalls = a.u.stalls, par = 0;
@@ -173,6 +175,10 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
     if (many) {
       if (!traded) __syncthreads();  // the whole block has read its region of p
       uint64_t* x = a.xchg + (tag & 1) * parity;
+      if (*(volatile int*)&s_lost != 0) {  // a wait that ran out, in a trade before this one's sweeps and barriers
+#pragma unroll
+        for (int r = 0; r < RPT; ++r) e[r][0] = e[r][1] = (T)__int_as_float(0x7fc00000);
+      }
 #pragma unroll
       for (int r = 0; r < RPT; ++r) {
         const int jj = j + r;
@@ -199,8 +205,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
             }
           }
         } while (!all && ++spins < kTradeSpins);
-        if (!all) {
-          s_lost = 1;
+        if (!all || lose_waits(bid)) {
+          give_up_wait(&s_lost);
           lost = true;
         }
       }
@@ -211,13 +217,14 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
     }
     if (left > 0) continue;
     if (!UNTIL) break;
-    const int nblk = gridDim.x * gridDim.y, bid = blockIdx.y * gridDim.x + blockIdx.x, tid = threadIdx.x;
+    const int nblk = gridDim.x * gridDim.y, tid = threadIdx.x;
     res_edges<T, RPT>(sh, buf, w, lane, e);
     __syncthreads();
     double sq = res_sumsq<T, RPT>(sh, buf, w, lane, e, ab, code, a.beta, own_col ? oy0 - j : RPT,
                                   own_col ? oy1 - j : 0);
     buf ^= 1;
     sq = block_sum(sq);
+    if (s_lost) sq = (double)__int_as_float(0x7fc00000);  // and so every block's sum of them all
     if (many) {
       uint64_t* sums = a.sums + (int64_t)par * nblk * 2;
       par ^= 1;
@@ -231,7 +238,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
           ld_words(sums + 2 * tid, lo, hi);
         } while (((uint32_t)(lo >> 32) != tag || (uint32_t)(hi >> 32) != tag) && *(volatile int*)&s_lost == 0 &&
                  ++spins < kTradeSpins);
-        if ((uint32_t)(lo >> 32) != tag || (uint32_t)(hi >> 32) != tag) s_lost = 1;
+        if ((uint32_t)(lo >> 32) != tag || (uint32_t)(hi >> 32) != tag) give_up_wait(&s_lost);
         sq = __hiloint2double((int)(uint32_t)hi, (int)(uint32_t)lo);
       }
       __syncwarp();
@@ -257,7 +264,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
     left = 2 * min(a.u.check_every, a.u.max_sweeps - done);
   }
   __syncthreads();
-  // a wait that gave up (its neighbour never arrived) leaves no usable iterate: say so in p
+  // a wait that ran out (waits.cuh) leaves no usable iterate: say so in p
   const bool bad = s_lost != 0;
 #pragma unroll
   for (int r = 0; r < RPT; ++r) {
@@ -410,3 +417,4 @@ int sg_sweeps_solve(int dtype, int sor, int64_t H, int64_t W, void* p, int64_t l
 }  // extern "C"
 
 SG_BOUNDS_ACCESSOR(sweeps)
+SG_WAITS_ACCESSOR(sweeps)

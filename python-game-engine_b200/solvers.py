@@ -67,7 +67,8 @@ RESIDENT_MIN_SOR = 2
 def _resident_sweeps(sor, dtc, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv, alpha, omega, iterations, device,
                      from_zero=False):
     """All sweeps in one launch with the iterate on the chip (``sg_sweeps_solve``: the same
-    iterates); False when the grid does not fit there."""
+    iterates); False when the grid does not fit there. What depends on a block's wait for its
+    neighbours that ran out is NaN (``_lib.lost_waits``)."""
     nbytes = L.load().sg_sweeps_workspace_bytes(dtc, H, W)
     if nbytes <= 0:
         return False

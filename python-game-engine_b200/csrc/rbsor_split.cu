@@ -668,7 +668,9 @@ int sg_rbsor_tol_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, c
                                  SweepsUntil{r0, tol, 0.0, (int)check_every, 0, 0, 0}, max_iterations, &it, &sq, s));
         rel = r0 > 0.0 ? std::sqrt(sq) / r0 : 0.0;
       }
-      while (std::isfinite(rel) && rel > tol && it < max_iterations) {
+      // not after a solve above, which ends on each of these; an initial guess whose residual
+      // overflows still gets its first sweeps
+      while (it < max_iterations && rel > tol && (it == 0 || std::isfinite(rel))) {
         const int64_t n = std::min(check_every, max_iterations - it);
         SG_CHECK((split_sweeps<T, MM>((int)H, (int)W, w, mm, alpha, reciprocal_beta, omega, n, var, s)));
         it += n;
@@ -676,7 +678,6 @@ int sg_rbsor_tol_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, c
         SG_CHECK(check_launch("sg_rbsor_tol_solve"));
         SG_CHECK(read_scalar(w.result, &sq, s));
         rel = r0 > 0.0 ? std::sqrt(sq) / r0 : 0.0;
-        if (!std::isfinite(rel)) break;
       }
     });
   });

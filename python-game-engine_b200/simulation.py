@@ -37,7 +37,7 @@ from . import _lib as L
 from . import operators as ops
 from .operators import OPEN_BOX, RING_BOX
 from .params import DEFAULT_SOLVER_PARAMS
-from .solvers import calculate_alpha, calculate_reciprocal_beta, solve_pressure, starts_from_zero
+from .solvers import calculate_alpha, calculate_reciprocal_beta, is_own_solver, solve_pressure, starts_from_zero
 
 
 class _NullTiming:
@@ -356,12 +356,15 @@ class SmokeSimulation2D:
         self.step_index += 1
 
     # The operators around the solve in two native calls (csrc/substep.cu) instead of one Python
-    # call each: nothing measures them, nothing replaces them, and every field is laid out as
-    # this class makes it. Anything else takes the calls one by one, which also report errors.
+    # call each: nothing measures them, nothing replaces them, the solve between them is this
+    # package's (another may put other tensors in the fields' place, and the second call has the
+    # first one's addresses), and every field is laid out as this class makes it. Anything else
+    # takes the calls one by one, which also report errors.
     def _steps_plainly(self):
         return (type(self) is SmokeSimulation2D and self.__dict__.keys().isdisjoint(_STEP_METHODS)
                 and all(SmokeSimulation2D.__dict__[n] is f for n, f in _STEP_METHODS.items())
-                and all(getattr(ops, n) is f for n, f in _STEP_OPERATORS.items()))
+                and all(getattr(ops, n) is f for n, f in _STEP_OPERATORS.items())
+                and is_own_solver(self.pressure_solver_method, self.pressure_solver_backend))
 
     def _pack_substep(self, dt):
         """The arguments of sg_substep_* (read afresh from the fields), or None."""
@@ -546,7 +549,8 @@ class SmokeSimulation2D:
 # have replaced.
 _STEP_METHODS = {n: SmokeSimulation2D.__dict__[n] for n in (
     "_apply_emitters", "_apply_forces", "_advect_velocity", "_advect_density", "_advect_temperature",
-    "_cool_temperature", "_compute_divergence", "_project_and_metrics", "_temperature_needed")}
+    "_cool_temperature", "_compute_divergence", "_solve_pressure", "_project_and_metrics",
+    "_temperature_needed")}
 _STEP_OPERATORS = {n: getattr(ops, n) for n in (
     "emit_scalar", "plume_sources", "apply_forces", "advect_velocity", "advect_scalar_field", "cool_temperature",
     "compute_divergence", "project_metrics")}

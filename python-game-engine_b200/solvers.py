@@ -21,7 +21,7 @@ import torch
 from . import _lib as L
 from .operators import AnalyticMask, OPEN_BOX, RING_BOX, _face_pair, _masks, build_masks, compute_residual
 from .params import SOLVER_PARAM_TYPES
-from .registry import get_solver, register_solver
+from .registry import SOLVER_REGISTRY, get_solver, register_solver
 
 
 # ---------------------------------------------------------------- coefficients (solvers/common.py)
@@ -586,6 +586,15 @@ class GeometricMultigridSolver:
 # ---------------------------------------------------------------- dispatch + registration
 # This package's parameter classes hold plain values only, so their fields need no deep copy.
 _FLAT_PARAMS = {t: tuple(f.name for f in fields(t)) for t in SOLVER_PARAM_TYPES.values()}
+
+
+def is_own_solver(method, backend):
+    """Whether (method, backend) names a solver of this package, which writes the pressure it is
+    given and leaves the caller's tensors where they are."""
+    fn = SOLVER_REGISTRY.get((method, backend))
+    return (type(fn) in (MultigridSolver, SORToleranceSolver, GeometricMultigridSolver)
+            or fn is jacobi_pressure_solver or fn is red_black_sor_gauss_seidel_pressure_solver
+            or fn is gauss_seidel_pressure_solver)
 
 
 def starts_from_zero(method, backend):

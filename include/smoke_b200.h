@@ -319,7 +319,8 @@ int sg_rbsor_mixed_solve(int64_t H, int64_t W, void* p, int64_t ld_p, const void
                          int64_t* out_refinements, void* stream);
 
 /* All `iterations` sweeps of sg_jacobi_solve (sor = 0) or sg_rbsor_solve (sor = 1) in one
- * cooperative launch with the iterate held on the chip: the same iterates, bit for bit.
+ * cooperative launch (one per 16384 sweeps) with the iterate held on the chip: the same iterates,
+ * bit for bit.
  * from_zero (iterations >= 1): p is 0 and not read.
  * workspace (16-byte aligned, sg_sweeps_workspace_bytes; cleared by the call): the cells that
  * neighbouring blocks trade. sg_sweeps_workspace_bytes is 0, and the solve returns
@@ -373,7 +374,8 @@ int sg_mg_prolong(int dtype, int64_t Hc, int64_t Wc, const void* coarse, int64_t
  * planes as they are at the call; which of its cells the residual and the transfers count as fluid
  * is what its codes say. from_zero (cycles >= 1): p is 0 and not read. Workspace
  * 256-byte aligned; sg_mg_vcycles_workspace_bytes is 0, and the call returns SG_ERR_CAPACITY,
- * for more than 4 SOR or 8 Jacobi sweeps a side or a coarsest level too large for the chip. */
+ * for more than 4 SOR or 8 Jacobi sweeps a side, 2^29 coarsest sweeps or a coarsest level too
+ * large for the chip. */
 typedef struct {
   int64_t H, W;
   const void* face_mask_u;

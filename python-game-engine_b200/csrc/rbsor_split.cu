@@ -438,7 +438,6 @@ static void launch_half(int H, int W, const SplitWs& w, MasksT<MM> m, double alp
                                                              (const T*)w.d[color], w.ldh, m, alpha, rb, omega, color));
 }
 
-constexpr int kResidentSweeps = 1 << 14;  // sweeps of one resident launch (some tens of ms)
 constexpr int kTileHalo = 8;  // halo of the tile kernel: up to 4 sweeps per launch
 
 template <typename T, int MM>
@@ -503,14 +502,8 @@ static int split_sweeps(int H, int W, SplitWs& w, MasksT<MM> m, double alpha, do
   if (iterations <= 0) return SG_OK;
   if (variant == 2) {
     SG_CHECK(resident_ready(w, s));
-    while (iterations > 0) {
-      const int n = (int)std::min<int64_t>(iterations, kResidentSweeps);
-      SG_CHECK(resident_sweeps<T>(1, 1, H, W, (T*)w.a[0], (T*)w.a[1], w.ldh, (const T*)w.d[0], (const T*)w.d[1], w.ldh,
-                                  m.template as<-1>(), alpha, rb, omega, n, false, w.xchg, w.tag, s));
-      w.tag += (uint32_t)resident_trades(1, n);
-      iterations -= n;
-    }
-    return SG_OK;
+    return resident_sweeps<T>(1, 1, H, W, (T*)w.a[0], (T*)w.a[1], w.ldh, (const T*)w.d[0], (const T*)w.d[1], w.ldh,
+                              m.template as<-1>(), alpha, rb, omega, iterations, false, w.xchg, &w.tag, s);
   }
   if (variant == 0 || iterations == 1) {
     for (int64_t it = 0; it < iterations; ++it)

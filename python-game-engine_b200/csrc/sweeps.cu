@@ -332,12 +332,11 @@ int resident_trades(int sor, int sweeps) {
 
 template <typename T>
 int resident_sweeps(int sor, int split, int H, int W, T* p, T* p1, int64_t ldp, const T* b, const T* b1, int64_t ldb,
-                    const Masks& m, double alpha, double rb, double omega, int sweeps, bool from_zero, void* xchg,
-                    uint32_t tag, cudaStream_t s) {
+                    const Masks& m, double alpha, double rb, double omega, int64_t sweeps, bool from_zero, void* xchg,
+                    uint32_t* tag, cudaStream_t s) {
   const int rpt = resident_rows(H, W);
   if (rpt == 0) return fail(SG_ERR_CAPACITY, "%d x %d cells do not fit the resident sweeps", H, W);
-  if (sweeps <= 0) return SG_OK;
-  ResArgs<T> a{H, W, p, p1, ldp, b, b1, ldb, m, alpha, rb, omega, sweeps, from_zero, (uint64_t*)xchg, (W + 1) & ~1, tag,
+  ResArgs<T> a{H, W, p, p1, ldp, b, b1, ldb, m, alpha, rb, omega, 0, from_zero, (uint64_t*)xchg, (W + 1) & ~1, 0,
                0.0, SweepsUntil{}, nullptr, nullptr};
   auto go = [&](auto SOR_, auto SPLIT_) {
     constexpr bool S = decltype(SOR_)::value, P = decltype(SPLIT_)::value;
@@ -345,13 +344,21 @@ int resident_sweeps(int sor, int split, int H, int W, T* p, T* p1, int64_t ldp, 
     if (rpt == 4) return launch_resident_rpt<T, S, P, 4, false>(a, s);
     return launch_resident_rpt<T, S, P, 8, false>(a, s);
   };
-  if (!sor) return go(std::false_type{}, std::false_type{});
-  return split ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
+  for (; sweeps > 0; sweeps -= a.sweeps) {
+    a.sweeps = (int)std::min<int64_t>(sweeps, kResidentSweeps);
+    a.tag = *tag;
+    *tag += (uint32_t)resident_trades(sor, a.sweeps);
+    SG_CHECK(!sor ? go(std::false_type{}, std::false_type{})
+                  : split ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{}));
+    a.from_zero = 0;
+  }
+  return SG_OK;
 }
 template int resident_sweeps<float>(int, int, int, int, float*, float*, int64_t, const float*, const float*, int64_t,
-                                    const Masks&, double, double, double, int, bool, void*, uint32_t, cudaStream_t);
+                                    const Masks&, double, double, double, int64_t, bool, void*, uint32_t*,
+                                    cudaStream_t);
 template int resident_sweeps<double>(int, int, int, int, double*, double*, int64_t, const double*, const double*,
-                                     int64_t, const Masks&, double, double, double, int, bool, void*, uint32_t,
+                                     int64_t, const Masks&, double, double, double, int64_t, bool, void*, uint32_t*,
                                      cudaStream_t);
 
 template <typename T>
@@ -408,9 +415,10 @@ int sg_sweeps_solve(int dtype, int sor, int64_t H, int64_t W, void* p, int64_t l
   cudaStream_t s = as_stream(stream);
   cudaError_t e = cudaMemsetAsync(workspace, 0, (size_t)need, s);
   if (e != cudaSuccess) return fail(SG_ERR_CUDA, "sg_sweeps_solve: %s", cudaGetErrorString(e));
+  uint32_t tag = 1;
   SG_DISPATCH(dtype, {
     return resident_sweeps<T>(sor != 0, 0, (int)H, (int)W, (T*)p, nullptr, ld_p, (const T*)div, nullptr, ld_div, m,
-                              alpha, reciprocal_beta, omega, iterations, from_zero != 0, workspace, 1, s);
+                              alpha, reciprocal_beta, omega, iterations, from_zero != 0, workspace, &tag, s);
   });
 }
 

@@ -28,16 +28,18 @@ __device__ __forceinline__ uint32_t cell_code(const Masks& m, int H, int W, int 
 int resident_rows(int64_t H, int64_t W);
 int64_t resident_workspace_bytes(int64_t elem, int64_t H, int64_t W);
 
-// Trades that a call of so many sweeps makes (each takes one tag).
+constexpr int kResidentSweeps = 1 << 14;  // sweeps of one resident launch (some tens of ms)
+// Trades that a launch of so many sweeps makes (each takes one tag).
 int resident_trades(int sor, int sweeps);
 
 // `sweeps` Jacobi (sor = 0) or red-black SOR sweeps of p in place. split: p, p1 and b, b1 are
-// colour planes. xchg: resident_workspace_bytes bytes, zeroed before the first call that uses
-// it; tag: 1 + the trades of the calls before on the same buffer. from_zero: p is 0 and not read.
+// colour planes. Launches of kResidentSweeps. xchg: resident_workspace_bytes bytes, zeroed before
+// the first call that uses it; *tag: 1 + the trades of the calls before on the same buffer, moved
+// on. from_zero: p is 0 and not read.
 template <typename T>
 int resident_sweeps(int sor, int split, int H, int W, T* p, T* p1, int64_t ldp, const T* b, const T* b1, int64_t ldb,
-                    const Masks& m, double alpha, double rb, double omega, int sweeps, bool from_zero, void* xchg,
-                    uint32_t tag, cudaStream_t s);
+                    const Masks& m, double alpha, double rb, double omega, int64_t sweeps, bool from_zero, void* xchg,
+                    uint32_t* tag, cudaStream_t s);
 
 // Red-black SOR sweeps of the colour planes p0, p1 until the residual's norm over r0 is at most
 // tol: checked after every check_every sweeps, at most max_sweeps of them (a multiple of

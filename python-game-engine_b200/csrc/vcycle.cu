@@ -479,8 +479,7 @@ static int mg_vcycles(int n, const sg_mg_level* lv, const MgPlan& P, T* p, int64
       }
       SG_CHECK(resident_sweeps<T>(SOR, 0, (int)L.H, (int)L.W, pc, nullptr, n == 1 ? ldp : L.W,
                                   n == 1 ? div : at(P.rhs[n - 1]), nullptr, n == 1 ? ldd : L.W, level_masks(L),
-                                  L.alpha, rb, L.omega, coarsest, fresh, ws + P.xchg, tag, s));
-      tag += (uint32_t)resident_trades(SOR, coarsest);
+                                  L.alpha, rb, L.omega, coarsest, fresh, ws + P.xchg, &tag, s));
     }
     for (int k = std::min(P.tail, n - 1) - 1; k >= 0; --k) level(k, false, false);
   }
@@ -518,7 +517,7 @@ int sg_mg_vcycles(int dtype, int n_levels, const sg_mg_level* levels, void* p, i
   SG_REQUIRE(reciprocal_beta != 0.0, "reciprocal_beta must be non-zero");
   SG_REQUIRE(dtype == SG_F32 || dtype == SG_F64, "unsupported dtype code %d", dtype);
   MgPlan P;
-  if (!mg_plan(dtype == SG_F32 ? 4 : 8, n_levels, levels, sor, sweeps, &P))
+  if (coarsest_sweeps > (1 << 29) || !mg_plan(dtype == SG_F32 ? 4 : 8, n_levels, levels, sor, sweeps, &P))
     return fail(SG_ERR_CAPACITY, "these levels or sweeps do not fit the fused V-cycle");
   SG_REQUIRE(ld_p >= levels[0].W && ld_div >= levels[0].W, "row stride below row length");
   for (int k = 0; k < n_levels; ++k)

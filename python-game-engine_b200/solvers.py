@@ -139,17 +139,17 @@ def gauss_seidel_pressure_solver(pressure, divergence, face_mask_u, face_mask_v,
            ws.data_ptr() if nbytes else None, nbytes, L.stream_ptr())
 
 
-def _rows_apart(t):
-    """Whether the rows of a 2-D field are unit-stride and do not overlap."""
-    H, W = t.shape
-    return (W == 1 or t.stride(1) == 1) and (H == 1 or t.stride(0) >= W)
-
-
-def _share_memory(a, b):
-    """Whether the address ranges of two 2-D fields of ascending rows overlap."""
-    (a0, a1), (b0, b1) = ((t.data_ptr(), t.data_ptr() + t.element_size() * ((t.shape[0] - 1) * t.stride(0) + t.shape[1]))
-                          for t in (a, b))
-    return a0 < b1 and b0 < a1
+def _readable_together(a, b):
+    """Whether two fields of one shape, type and device have unit-stride rows that do not overlap,
+    within each and between the two."""
+    if a.dtype != b.dtype or a.shape != b.shape or a.device != b.device:
+        return False
+    H, W = a.shape
+    (lda, one_a), (ldb, one_b) = a.stride(), b.stride()
+    if one_a != 1 or one_b != 1 or lda < W or ldb < W:
+        return False
+    gap = (b.data_ptr() - a.data_ptr()) // a.element_size()
+    return gap >= (H - 1) * lda + W or -gap >= (H - 1) * ldb + W
 
 
 class MultigridSolver:
@@ -236,17 +236,10 @@ class MultigridSolver:
             sor = 1
         else:
             return False
-        if cycles < 1:
+        if cycles < 1 or nu_c > 1 << 29 or not _readable_together(pressure, divergence):
             return False
-        H, W = pressure.shape
-        if (divergence.dtype != pressure.dtype or divergence.shape != pressure.shape
-                or divergence.device != pressure.device or not _rows_apart(pressure) or not _rows_apart(divergence)
-                or _share_memory(pressure, divergence)):
-            return False
-        # the caller's own planes: the level table has no row strides
-        fine = self.levels[0]
-        if not (fine["fmu"].is_contiguous() and fine["fmv"].is_contiguous() and fine["fmu"].shape == (H, W + 1)
-                and fine["fmv"].shape == (H + 1, W)):
+        # the fine level's planes are the caller's: the level table has no row strides
+        if not (self.levels[0]["fmu"].is_contiguous() and self.levels[0]["fmv"].is_contiguous()):
             return False
         n = len(self.levels)
         table = (L.MgLevel * n)()

@@ -131,13 +131,17 @@ __device__ __forceinline__ void gs_run(const GsArgs<T>& g, int* s_lost, unsigned
   const uint8_t* fu = g.m.fmu + (rows ? (int64_t)lc * g.m.ldu : lc);
   const uint8_t* fv = g.m.fmv + (rows ? (int64_t)lc * g.m.ldv : lc);
   int fy = -lc;  // y of the next diagonal to fetch
+  // whether the pointer lies on a plane of h rows of w values, ld apart
+  auto on_plane = [&](auto* at, auto* base, int h, int w, int64_t ld) {
+    return at >= base && (at - base) / ld < h && (at - base) % ld < w;
+  };
   auto fetch = [&](int d, int u) {
     if (FIRST)
-      q[u].p = *fp;
-    else
+      q[u].p = SG_IN_BOUNDS(on_plane(fp, (const T*)g.p, g.H, g.W, g.ldp)) ? *fp : (T)0;
+    else if (SG_IN_BOUNDS(slot(d, lc) >= 0 && slot(d, lc) + GsWords<T>::N <= ring))
       gs_get(in + slot(d, lc), q[u].g);
-    q[u].d = *fd;
-    if (PLANES) {
+    q[u].d = SG_IN_BOUNDS(on_plane(fd, g.div, g.H, g.W, g.ldd)) ? *fd : (T)0;
+    if (PLANES && SG_IN_BOUNDS(on_plane(fu, g.m.fmu, g.H, g.W, g.m.ldu) && on_plane(fv, g.m.fmv, g.H, g.W, g.m.ldv))) {
       q[u].f[0] = fu[0];
       q[u].f[1] = fu[1];
       q[u].f[2] = fv[0];
@@ -184,9 +188,11 @@ __device__ __forceinline__ void gs_run(const GsArgs<T>& g, int* s_lost, unsigned
         c = xin && y >= e && y <= N - 1 - e && c ? c | K_FLUID : 0u;
       }
       const int o = row * Mp + lx;
-      sp[o] = on ? v : (T)0;
-      sa[o] = g.alpha * (double)q[u].d;
-      sc[o] = (uint8_t)(on ? c : 0);
+      if (SG_IN_BOUNDS(row >= 0 && row < R && lx >= 0 && lx < Mp)) {
+        sp[o] = on ? v : (T)0;
+        sa[o] = g.alpha * (double)q[u].d;
+        sc[o] = (uint8_t)(on ? c : 0);
+      }
     }
     __syncwarp();  // the lanes leave the polls at different times
   };
@@ -237,7 +243,7 @@ __device__ __forceinline__ void gs_run(const GsArgs<T>& g, int* s_lost, unsigned
       if (ROLE != 2) {
         op += Mp;
         op -= op >= R * Mp ? R * Mp : 0;
-        if (own) {
+        if (own && SG_IN_BOUNDS(om + xm >= 0 && om < R * Mp && o >= 0 && o < R * Mp && op >= 0 && op + xp < R * Mp)) {
           const int d = t - 2 * cs, y = d - cx;
           const T m1 = sp[om + xm], p0 = sp[op], p1 = sp[op + xp];
           const double an = sa[op];
@@ -374,4 +380,5 @@ template int gauss_seidel_wave<double>(int, int, double*, int64_t, const double*
 
 }  // namespace sg
 
+SG_BOUNDS_ACCESSOR(gauss_seidel)
 SG_WAITS_ACCESSOR(gauss_seidel)

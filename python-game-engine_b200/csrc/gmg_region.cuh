@@ -513,7 +513,7 @@ __device__ __forceinline__ void region_tail_visit(const RegionTailArgs<T>& a, co
   for (int r = 0; r < RPT; ++r)
 #pragma unroll
     for (int q = 0; q < 2; ++q)
-      if (j + r < H && i + q < W) {
+      if (j + r < H && i + q < W && SG_IN_BOUNDS(o + (j + r) * W + i + q < a.cells)) {
         if (post && l == 0)
           a.ge[(int64_t)(j + r) * a.gld + i + q] = g.e[r][q];
         else
@@ -522,7 +522,7 @@ __device__ __forceinline__ void region_tail_visit(const RegionTailArgs<T>& a, co
   if (post) return;
   region_restrict<T, RPT, true>(sh, buf, w, lane, g, nw, j, i, H, W, Hc, Wc, [&](int m, T v) {
     const int J = (j >> 1) + m, I = i >> 1;
-    if (J < Hc && I < Wc) t.b[oc + J * Wc + I] = v;
+    if (J < Hc && I < Wc && SG_IN_BOUNDS(oc + J * Wc + I < a.cells)) t.b[oc + J * Wc + I] = v;
   });
 }
 

@@ -1003,6 +1003,7 @@ int sg_bounds_line_adjoint(unsigned* line, int clear);
 int sg_bounds_line_metrics(unsigned* line, int clear);
 int sg_bounds_line_sweeps(unsigned* line, int clear);
 int sg_bounds_line_vcycle(unsigned* line, int clear);
+int sg_bounds_line_gauss_seidel(unsigned* line, int clear);
 
 int sg_lost_waits_sweeps(unsigned* count, int clear);
 int sg_lost_waits_gauss_seidel(unsigned* count, int clear);
@@ -1031,7 +1032,7 @@ int sg_bounds_check(unsigned* first_line, int* unit, int clear) {
   int (*const fns[])(unsigned*, int) = {sg_bounds_line_operators,   sg_bounds_line_gmg,     sg_bounds_line_batch,
                                         sg_bounds_line_rbsor_split, sg_bounds_line_advect_fast,
                                         sg_bounds_line_adjoint,     sg_bounds_line_metrics, sg_bounds_line_sweeps,
-                                        sg_bounds_line_vcycle};
+                                        sg_bounds_line_vcycle,     sg_bounds_line_gauss_seidel};
   *first_line = 0;
   *unit = -1;
   for (int k = 0; k < (int)(sizeof(fns) / sizeof(fns[0])); ++k) {

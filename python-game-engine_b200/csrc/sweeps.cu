@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
 #pragma unroll
           for (int r = 0; r < RPT; ++r) {
             const int jj = j + r;
-            if (jj < H && (halo_col || jj < oy0 || jj >= oy1)) {
+            if (jj < H && (halo_col || jj < oy0 || jj >= oy1) && SG_IN_BOUNDS(i + 1 < a.ldx)) {
               if (!trade_get(x, (int64_t)jj * a.ldx + i, e[r], tag)) all = false;
             }
           }
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
       if (tid == 0)
         st_words(sums + 2 * bid, tagged((uint32_t)__double2loint(sq), tag), tagged((uint32_t)__double2hiint(sq), tag));
       sq = 0.0;
-      if (tid < nblk) {
+      if (tid < nblk && SG_IN_BOUNDS(nblk <= kResThreads)) {
         uint64_t lo, hi;
         int spins = 0;
         do {
@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const int ii = i + q;
-      if (ii >= W) continue;
+      if (ii >= W || !SG_IN_BOUNDS(jj < H)) continue;
       const int64_t o = SPLIT ? (int64_t)jj * a.ldp + (ii >> 1) : (int64_t)jj * a.ldp + ii;
       (SPLIT && ((jj + ii) & 1) ? a.p1 : a.p)[o] = bad ? (T)__int_as_float(0x7fc00000) : e[r][q];
     }

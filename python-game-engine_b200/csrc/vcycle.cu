@@ -102,7 +102,7 @@ struct MgRegion {
       for (int q = 0; q < 2; ++q) {
         e[r][q] = (T)0;
         ab[r][q] = 0.0;
-        if (jj < a.H && i + q < a.W) {
+        if (jj < a.H && i + q < a.W && SG_IN_BOUNDS(jj >= 0 && i >= 0)) {
           if (a.pin) e[r][q] = a.pin[(int64_t)jj * a.ldin + i + q];
           ab[r][q] = a.alpha * (double)a.b[(int64_t)jj * a.ldb + i + q];
         }
@@ -147,6 +147,7 @@ __device__ __forceinline__ T mg_prolong(const T* c, int64_t ldc, int Hc, int Wc,
   const int x1 = min((i + 1) >> 1, Wc - 1), x0 = min(max((i - 1) >> 1, 0), x1);  // i, j may lie off the grid
   const int y1 = min((j + 1) >> 1, Hc - 1), y0 = min(max((j - 1) >> 1, 0), y1);
   const double tx = (i & 1) ? 0.25 : 0.75, ty = (j & 1) ? 0.25 : 0.75;
+  if (!SG_IN_BOUNDS(x0 >= 0 && x1 < Wc && y0 >= 0 && y1 < Hc)) return (T)0;
   const T* r0 = c + (int64_t)y0 * ldc;
   const T* r1 = c + (int64_t)y1 * ldc;
   const double c0 = lerp_ref(r0[x0], r0[x1], tx);
@@ -260,7 +261,7 @@ __device__ __forceinline__ void mg_tail_visit(const MgTailArgs<T>& a, const MgTa
       const int ii = i + q;
       e[r][q] = (T)0;
       ab[r][q] = 0.0;
-      if (jj >= H || ii >= W) continue;
+      if (jj >= H || ii >= W || !SG_IN_BOUNDS(o + jj * W + ii < a.cells)) continue;
       const int c = o + jj * W + ii;
       if (up)
         e[r][q] = t.p[c];
@@ -287,7 +288,7 @@ __device__ __forceinline__ void mg_tail_visit(const MgTailArgs<T>& a, const MgTa
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const int jj = j + r, ii = i + q;
-      if (jj >= H || ii >= W) continue;
+      if (jj >= H || ii >= W || !SG_IN_BOUNDS(o + jj * W + ii < a.cells)) continue;
       if (last)
         a.pout[(int64_t)jj * a.ldout + ii] = e[r][q];
       else
@@ -298,7 +299,8 @@ __device__ __forceinline__ void mg_tail_visit(const MgTailArgs<T>& a, const MgTa
   res_residual<T, RPT, true>(sh, buf, w, lane, e, ab, code, cells, a.beta, res, threads);
 #pragma unroll
   for (int r = 0; r < RPT; r += 2)
-    if (j + r + 1 < H && i + 1 < W)
+    if (j + r + 1 < H && i + 1 < W &&
+        SG_IN_BOUNDS(a.off[l + 1] + ((j + r) >> 1) * (W >> 1) + (i >> 1) < a.cells))
       t.b[a.off[l + 1] + ((j + r) >> 1) * (W >> 1) + (i >> 1)] = mg_restrict<T, RPT>(res, cells, r, (T)a.alpha[l + 1]);
 }
 

@@ -6,7 +6,11 @@ Runs: one multigrid cycle in FP64, FP32 and mixed precision on 3 x 65, 9 x 33, 6
 130 x 67 and 1100 x 1300 open boxes and on a 40 x 40 box whose obstacle leaves one fluid
 cell open; the split-layout SOR (both kernel variants) and the multi-sweep Jacobi tiles on
 the small shapes; a batch of odd-sized scenes for two steps. Writes every result and the
-bounds-check record (first failed source line and unit, or 0 / -1) to OUT.npz."""
+bounds-check record (first failed source line and unit, or 0 / -1) to OUT.npz.
+
+The Jacobi count is one that the solver runs on the sweeps resident on the chip; the tiles, which
+larger grids and callers' scratch buffers take, are in bounds_cases_sweeps.py with the other kernels
+of the sweep solvers, the V-cycles and levels with obstacles."""
 import importlib
 import os
 import sys

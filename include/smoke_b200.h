@@ -216,8 +216,8 @@ int sg_bounds_check(unsigned int* first_line, int* unit, int clear);
  * sg_rbsor_split_sweeps on grids that fit the chip, sg_gauss_seidel_sweeps with a workspace, the
  * coarsest sweeps of sg_mg_vcycles) wait for one another, at most some seconds. What depends on a
  * wait that ran out is NaN; solves to a tolerance then end with SG_ERR_NONFINITE, the others have
- * returned before. sg_lost_waits: such waits on the current device since the last call with
- * clear != 0 (synchronises). sg_bounds_lose_waits (bounds-check build only, for tests): the
+ * returned before. sg_lost_waits: blocks with such waits on the current device since the last call
+ * with clear != 0 (synchronises). sg_bounds_lose_waits (bounds-check build only, for tests): the
  * blocks of that index give up every wait at once; -1 for none. */
 int sg_lost_waits(int64_t* count, int clear);
 int sg_bounds_lose_waits(int block);

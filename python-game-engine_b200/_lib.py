@@ -204,7 +204,7 @@ def bounds_check(clear=True):
 
 
 def lost_waits(clear=True):
-    """Waits of a launch's blocks for one another that ran out on the current device since the
+    """Blocks whose wait for another block of their launch ran out on the current device since the
     last clear (their solves hold NaN); synchronises."""
     n = ctypes.c_int64(0)
     check(load().sg_lost_waits(ctypes.byref(n), 1 if clear else 0), "sg_lost_waits")

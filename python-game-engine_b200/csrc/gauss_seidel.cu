@@ -170,13 +170,13 @@ __device__ __forceinline__ void gs_run(const GsArgs<T>& g, int* s_lost, unsigned
         if (on && !gs_there(q[u].g, (uint32_t)d + 1)) {
           int spins = 0;
           do {
-            if (++spins > kGsSpins) give_up_wait(s_lost);
+            if (++spins > kGsSpins) *(volatile int*)s_lost = 1;
             gs_get(in + slot(d, lc), q[u].g);
           } while (!gs_there(q[u].g, (uint32_t)d + 1) && *(volatile int*)s_lost == 0);
         }
         // a block that never came (waits.cuh) leaves no usable iterate: say so in p, down the chain
         const bool lose = lose_waits(blockIdx.x);
-        if (lose) give_up_wait(s_lost);
+        if (lose) *(volatile int*)s_lost = 1;
         v = gs_there(q[u].g, (uint32_t)d + 1) && !lose ? gs_value(q[u].g) : (T)__int_as_float(0x7fc00000);
       }
       uint32_t c;
@@ -232,7 +232,7 @@ __device__ __forceinline__ void gs_run(const GsArgs<T>& g, int* s_lost, unsigned
       const int need = min(t0 + kGsAhead - 2 * (k - 1), D) - kGsRing;  // read before this round's diagonals go out
       int spins = 0;
       while (read < need && *(volatile int*)s_lost == 0) {
-        if (++spins > kGsSpins) give_up_wait(s_lost);
+        if (++spins > kGsSpins) *(volatile int*)s_lost = 1;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(read) : "l"(credit_out) : "memory");
       }
       __syncwarp();
@@ -307,6 +307,7 @@ __global__ void __launch_bounds__(kGsThreads, 1) k_gauss_seidel_wave(__grid_cons
     gs_run<T, PLANES, true, 0>(g, &s_lost, gs_smem);
   else
     gs_run<T, PLANES, false, 0>(g, &s_lost, gs_smem);
+  count_lost_wait(s_lost);  // every step ends with a barrier
 }
 
 // ------------------------------------------------------------------ host side

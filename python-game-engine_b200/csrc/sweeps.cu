@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
           }
         } while (!all && ++spins < kTradeSpins);
         if (!all || lose_waits(bid)) {
-          give_up_wait(&s_lost);
+          s_lost = 1;
           lost = true;
         }
       }
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
           ld_words(sums + 2 * tid, lo, hi);
         } while (((uint32_t)(lo >> 32) != tag || (uint32_t)(hi >> 32) != tag) && *(volatile int*)&s_lost == 0 &&
                  ++spins < kTradeSpins);
-        if ((uint32_t)(lo >> 32) != tag || (uint32_t)(hi >> 32) != tag) give_up_wait(&s_lost);
+        if ((uint32_t)(lo >> 32) != tag || (uint32_t)(hi >> 32) != tag) s_lost = 1;
         sq = __hiloint2double((int)(uint32_t)hi, (int)(uint32_t)lo);
       }
       __syncwarp();
@@ -266,6 +266,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_sweeps_resident(const __grid
   __syncthreads();
   // a wait that ran out (waits.cuh) leaves no usable iterate: say so in p
   const bool bad = s_lost != 0;
+  count_lost_wait(s_lost);
 #pragma unroll
   for (int r = 0; r < RPT; ++r) {
     const int jj = j + r;

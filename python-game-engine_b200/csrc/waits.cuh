@@ -1,7 +1,7 @@
 // Waits of a launch's blocks for one another, for the units whose blocks trade cells. Every such
 // wait is bounded. A block whose wait runs out has no usable iterate from there on: what it stores,
 // hands to other blocks or adds to a sum is NaN, so that no finite value depends on it, and the
-// unit counts the wait (sg_lost_waits), which a call that returns before its kernels have run
+// unit counts the block (sg_lost_waits), which a call that returns before its kernels have run
 // cannot report.
 //
 // In the bounds-check build a test can name a block that gives up each wait at once
@@ -14,9 +14,10 @@ namespace sg {
 
 static __device__ unsigned int g_lost_waits;  // one word per translation unit
 
-// s_lost: the block's mark. Safe from any number of its threads.
-__device__ __forceinline__ void give_up_wait(int* s_lost) {
-  if (atomicExch(s_lost, 1) == 0) atomicAdd(&g_lost_waits, 1u);
+// At the block's end, by every thread: s_lost is the block's mark, settled by a barrier. (Counted
+// in the poll loops, the atomics cost the Gauss-Seidel chain 2 %.)
+__device__ __forceinline__ void count_lost_wait(int s_lost) {
+  if (s_lost && threadIdx.x == 0) atomicAdd(&g_lost_waits, 1u);
 }
 
 #if SG_BOUNDS_CHECK

@@ -2,8 +2,7 @@
 // batch.cu inside namespace sg; uses w1 and rcp_open of gmg_weights.cuh).
 //
 // For open-box levels (every cell fluid, every interior face open) one launch runs a whole
-// side of a cycle on a tile of fine cells held in shared memory (64 x 32 on large levels,
-// 16 x 16 on levels too small to fill the GPU with large tiles):
+// side of a cycle on a tile of 16 x 16 fine cells held in shared memory:
 //   pre:  SW red-black sweeps, the residual and its full-weighting restriction; reads e
 //         (not at all for a zero initial guess) and b once, writes e and the coarse rhs;
 //   post: bilinear prolongation of the coarse correction plus SW sweeps.
@@ -18,8 +17,7 @@
 // all but the outermost) take a path without bounds checks (every cell has 4 neighbours).
 #pragma once
 
-constexpr int kTX = 64, kTY = 32;   // fine cells of a large-level tile
-constexpr int kSX = 16, kSY = 16;   // fine cells of a small-level tile (more blocks per level)
+constexpr int kSX = 16, kSY = 16;   // fine cells of a tile
 constexpr int kTBX = 32, kTBY = 8;  // threads of a tile block
 constexpr int kTThreads = kTBX * kTBY;
 
@@ -36,8 +34,7 @@ struct SplitTile {
 };
 
 __device__ __forceinline__ int tile_tid() { return threadIdx.y * kTBX + threadIdx.x; }
-// threads of the block: kTThreads, or more on levels with few tiles (shorter phases)
-__device__ __forceinline__ int tile_nt() { return kTBX * blockDim.y; }
+__device__ __forceinline__ int tile_nt() { return kTThreads; }
 
 // Relax the cells of colour col in the tile grown by RING rings (smem rows/cols
 // [HALO - RING, HALO + TY|TX + RING)); every neighbour is inside the loaded tile.

@@ -823,7 +823,7 @@ def other_workloads(sg, dev, lib, peak_gbs):
         entry = {"value": sc.cells / (ms / 1e3), "unit": "cell-steps/s", "ms_per_step": ms, "steps": steps}
         if method == "rb_sor_tolerance":
             entry["mean_sweeps_per_step"] = sum(work[2:]) / max(len(work) - 2, 1)
-            entry["timing"] = "host-synchronised tolerance loop (residual read every 200 sweeps)"
+            entry["timing"] = "host-synchronised solve (residual checked every 200 sweeps inside the sweeps' launch)"
         else:
             cyc, rel, ok = solver.last_cycles, solver.last_relres, solver.converged
             entry["last_cycles"], entry["last_relres"], entry["converged"] = cyc, rel, bool(ok)
@@ -839,8 +839,8 @@ def other_workloads(sg, dev, lib, peak_gbs):
     out["plume_128"] = {"value": sc.cells / (ms / 1e3), "unit": "cell-steps/s", "ms_per_step": ms, "steps": 20,
                         "solver": "Jacobi x 100 (reference iterates), float64",
                         "hbm_ceiling_cell_steps_per_s": peak_gbs * 1e9 / 2568,
-                        "note": "ceiling at (21 + 100 x 3) x 8 B per cell-step; 16384 cells sit in L2 and the step "
-                                "is launch-bound (one launch per sweep)"}
+                        "note": "ceiling at (21 + 100 x 3) x 8 B per cell-step; 16384 cells sit on the chip and the "
+                                "step is bound by its chain of 100 dependent sweeps (one launch)"}
     del sim
     # ---- batch of 256 scenes
     scenes = sg.scenes.batch_256(256, steps=10)

@@ -264,11 +264,13 @@ int sg_rbsor_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, const
  * Cell (j, i) of colour c = (i + j) & 1 lives in plane c at row j, column i >> 1, so each
  * colour streams contiguously. The iterates equal sg_rbsor_solve's bit for bit.
  * Workspace (256-byte aligned, sg_rbsor_split_workspace_bytes): two state buffers of two
- * planes each, the two divergence planes and the residual partial sums.
+ * planes each, the two divergence planes, the residual partial sums and, on grids that fit the
+ * chip, the cells that the resident sweeps' blocks trade.
  *   pack:   which = 0 copies the pressure into the state, 1 the divergence
  *   sweeps: `iterations` sweeps (colour 0 then 1) on the state; variant 0 launches one
  *           streaming kernel per half sweep, variant 1 sweeps 32 x 64 tiles staged in shared
- *           memory up to 4 sweeps per launch (same iterates), -1 picks the tiles while
+ *           memory up to 4 sweeps per launch (same iterates), -1 holds the state on the chip
+ *           through all sweeps where the grid fits (sg_sweeps_solve), else picks the tiles while
  *           2 * H * W * sizeof(dtype) <= 8 MiB (L2-resident, launch-bound) and the
  *           streaming launches above (bandwidth-bound)
  *   sumsq:  *out (device) = sum over fluid cells of the squared reference residual
@@ -276,7 +278,8 @@ int sg_rbsor_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, const
  *   unpack: the state back to a natural-layout field
  *   tol_solve: pack, then sweeps in chunks of check_every until ||r(p)|| <= tol ||r(0)||
  *           (fluid cells) or max_iterations, then unpack into p; synchronises the stream
- *           after every chunk to read the residual. Returns SG_ERR_NOT_CONVERGED (p still
+ *           after every chunk to read the residual, or, on grids whose resident sweeps hold at
+ *           most four rows a thread, after launches that check by themselves. Returns SG_ERR_NOT_CONVERGED (p still
  *           written, *out_iterations / *out_relres set) when the tolerance is not reached. */
 int64_t sg_rbsor_split_workspace_bytes(int dtype, int64_t H, int64_t W);
 int sg_rbsor_split_pack(int dtype, int64_t H, int64_t W, const void* src, int64_t ld_src, int which,
@@ -307,7 +310,8 @@ int sg_rbsor_tol_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, c
  * max(1e-3, tol / (2 relres)) (at most 0.5) or until three chunks in a row gain < 1 %;
  * then p += e. Stops at ||r(p)|| <= tol ||r(0)|| (fluid cells) or max_iterations sweeps.
  * variant as for sg_rbsor_split_sweeps. Workspace: sg_rbsor_mixed_workspace_bytes
- * (256-byte aligned). Synchronises the stream after every chunk. SG_ERR_NOT_CONVERGED when
+ * (256-byte aligned). Synchronises the stream after every chunk, or with the checks inside the
+ * launch (sg_rbsor_tol_solve) after every launch. SG_ERR_NOT_CONVERGED when
  * the tolerance is not reached (p written). */
 int64_t sg_rbsor_mixed_workspace_bytes(int64_t H, int64_t W);
 int sg_rbsor_mixed_solve(int64_t H, int64_t W, void* p, int64_t ld_p, const void* div, int64_t ld_div,
@@ -342,7 +346,8 @@ int sg_gauss_seidel_solve(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p
 
 /* The same sweeps (the same iterates) split over a chain of blocks that hand their diagonals on
  * through workspace (16-byte aligned, sg_gauss_seidel_workspace_bytes; cleared by the call;
- * null: one block), waiting for one another (sg_lost_waits). 0 bytes: the call has no chain form and needs none. */
+ * null: one block), waiting for one another (sg_lost_waits). 0 bytes: the call has no chain form
+ * and needs none. */
 int64_t sg_gauss_seidel_workspace_bytes(int dtype, int64_t H, int64_t W, int iterations);
 int sg_gauss_seidel_sweeps(int dtype, int64_t H, int64_t W, void* p, int64_t ld_p, const void* div,
                            int64_t ld_div, int mask_mode, const uint8_t* fmu, int64_t ld_fmu,
@@ -363,7 +368,6 @@ int sg_mg_prolong(int dtype, int64_t Hc, int64_t Wc, const void* coarse, int64_t
                   int mask_mode, const uint8_t* is_fluid, int64_t ld_fluid, void* fine, int64_t ld_f,
                   int accumulate, void* stream);
 
-/* multigrid/masks.py:3-27 (any solid child makes the coarse cell solid). */
 /* The reference's V-cycles (multigrid/solver.py:94-176) on a hierarchy whose levels halve
  * exactly: `cycles` cycles of p in place with `sweeps` smoothing sweeps a side and
  * coarsest_sweeps on the last level, red-black SOR (sor = 1) or Jacobi, in two launches per
@@ -389,6 +393,8 @@ int64_t sg_mg_vcycles_workspace_bytes(int dtype, int n_levels, const sg_mg_level
 int sg_mg_vcycles(int dtype, int n_levels, const sg_mg_level* levels, void* p, int64_t ld_p, const void* div,
                   int64_t ld_div, double reciprocal_beta, int sor, int cycles, int sweeps, int coarsest_sweeps,
                   int from_zero, void* workspace, int64_t workspace_bytes, void* stream);
+
+/* multigrid/masks.py:3-27 (any solid child makes the coarse cell solid). */
 int sg_mg_coarsen_solid(int64_t H, int64_t W, const uint8_t* solid, int64_t ld_s, uint8_t* coarse,
                         int64_t ld_c, void* stream);
 

@@ -21,7 +21,7 @@
 // launches and the length of one warp's instruction stream. Edge tests are selects: as branches
 // they parted the edge lanes from the rest of every warp (tail 18.8 and 22.8 us in float32 and
 // float64, pre / post 3.6 / 3.4). Measured, us: a 421 x 300 mixed cycle around obstacles (5
-// levels of half-sweep launches, 55 in all, before) 117 -> 36; a 512^2 float64 cycle (4 levels of
+// levels of half-sweep launches, 55 in all, before) 117 -> 38; a 512^2 float64 cycle (4 levels of
 // 16 x 16 shared-memory tiles and a 16^2 tail before) 71 -> 59; pre and post of a level 3.1 and
 // 3.1 in float32, 3.8 and 3.8 in float64 (5.1 and 3.8 on the tiles); the tail from 64^2 down 15.2
 // in float32, 20.7 in float64, for 27.2 as two tiled levels and a 16^2 tail.

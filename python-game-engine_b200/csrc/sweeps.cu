@@ -300,8 +300,10 @@ int resident_rows(int64_t H, int64_t W) {
   return 0;
 }
 
-// Up to four rows a thread: with eight the check's registers spill in the sweeps (1000 x 901
-// float64, 100 sweeps 874 us, 944 with the check in the launch, about 920 with one from the host).
+// Up to four rows a thread: with eight the check's registers spill in the float64 sweeps. us a
+// check, from the host against inside the launch: every 100 sweeps (the solver's default) float64
+// 283 against 442 at 600 x 801 and 284 against 420 at 800 x 900, float32 307 / 304 and 297 / 300;
+// every 10 sweeps the launch wins in both types (66 / 56 and 69 / 45 at 600 x 801).
 bool resident_until_fits(int64_t H, int64_t W) {
   const int rpt = resident_rows(H, W);
   return rpt == 2 || rpt == 4;

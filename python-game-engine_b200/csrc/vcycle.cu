@@ -15,8 +15,8 @@
 // one barrier chain per half sweep, store), so the number of dependent launches is the time:
 // 512^2, 7 levels, V(2,2) with red-black smoothing took 260 launches of 2.7 us per pair of
 // cycles as separate kernels (742 us of kernels, 1.5 ms with their issue from the host) and
-// takes 14 launches and 130 us now; 2048^2 float32, 9 levels, 370 us. Cell codes made once per
-// mask instead of four mask bytes a cell and launch: 512^2 down / up 7.0 / 8.3 -> 5.0 / 5.3 us
+// takes 15 launches and 135 us now; 2048^2 float32, 9 levels, 370 us. Cell codes made once per
+// hierarchy (level 0's once a call, 4 us at 512^2) instead of four mask bytes a cell and launch: 512^2 down / up 7.0 / 8.3 -> 5.0 / 5.3 us
 // (4.3 / 4.7 on average over the levels above 64^2, tail 25),
 // 1024^2 19.2 / 20.1 -> 12.1 / 12.1.
 #include <algorithm>

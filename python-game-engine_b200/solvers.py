@@ -58,8 +58,13 @@ def materialize_mask(m, H, W, which, device):
 
 
 # ---------------------------------------------------------------- reference methods
-# Sweep counts up to which the launches of the plain kernels cost less than one resident
-# launch with its cleared exchange buffer.
+# Sweep counts up to which a call keeps the plain kernels: there the resident launch with its
+# cleared exchange buffer gains little or loses. GPU us a call, resident against plain, float32 /
+# float64: one SOR sweep 5.9 / 6.7 against 4.9 / 4.6 at 128^2 and 17.6 / 18.8 against 7.9 / 8.3 at
+# 800 x 900, three 6.6 / 7.4 against 14.5 / 13.6 and 19.9 / 21.1 against 23.6 / 24.9 (two: even, all
+# told); eight Jacobi sweeps, one launch of tiles, 5.6 / 6.9 against 5.2 / 5.6 at 16^2 but 12.6 / 14.7
+# against 20.5 / 21.9 at 512^2, sixteen 8.3 / 9.7 against 8.0 / 8.1 and 17.1 / 19.9 against 36.9 / 37.8.
+# Below 128^2 both take less than the host needs to issue a call (19 us).
 RESIDENT_MIN_JACOBI = 8
 RESIDENT_MIN_SOR = 2
 
@@ -80,7 +85,8 @@ def _resident_sweeps(sor, dtc, H, W, p, ldp, d, ldd, mode, pu, lu, pv, lv, alpha
 
 def jacobi_pressure_solver(pressure, divergence, face_mask_u, face_mask_v, fluid_density, cell_size, dt,
                            iterations, scratch=None, zero_initial_guess=False, **_ignored):
-    """jacobi.py:27-52: ``iterations`` ping-pong sweeps; the result ends in ``pressure``.
+    """jacobi.py:27-52: ``iterations`` ping-pong sweeps; the result ends in ``pressure``. With a
+    caller's ``scratch`` (H x W) nothing is allocated and the sweeps take the plain kernels.
     ``zero_initial_guess``: start from p = 0 whatever ``pressure`` holds."""
     H, W = pressure.shape
     dtc = L.dtype_code(pressure)
@@ -487,6 +493,9 @@ class GeometricMultigridSolver:
     on the correction from zero between two FP64 passes (p += e, residual), instead of the
     fused fine level that corrects p and updates the FP64 residual every cycle; the cycle
     counts then grow in steps of k.
+    ``last_relres`` is the residual of the returned pressure, except on open boxes of at least
+    100 blocks of 64 x 32 cells: their fused fine level carries the residual on from cycle to
+    cycle, which is the true one down to the pressure's own rounding and may go on falling below.
     """
 
     def __init__(self):
